@@ -292,7 +292,7 @@ def forms_section(alg, eng, bi, prec, stream, flush, scn):
                       3, flush)
     prof = eng.read_profile()
     eng.set_profiling(False)
-    out["adjoint"] = {"form": "persistent kernels, adjoint gradients (checkpoints every 256 steps)",
+    out["adjoint"] = {"form": "persistent kernels, adjoint gradients",
                       "scenario_epochs_per_s": 1000.0 / statistics.mean(ms), "ms_per_epoch": statistics.mean(ms),
                       "voxel_steps_per_s": V * T * B * 1000.0 / statistics.mean(ms),
                       "phase_ms": {k: v[0] / 3 for k, v in prof.items() if v[0] > 0}}

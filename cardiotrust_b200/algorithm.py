@@ -39,7 +39,7 @@ class APDerivative(enum.IntEnum):
 
 class GradMode(enum.IntEnum):
     Reference = 0  # the reference's per-step derivation (derivation.rs:173-229)
-    Adjoint = 1  # exact gradient of the stated loss, back-propagation through time with checkpoints
+    Adjoint = 1  # exact gradient of the stated loss, back-propagation through time
 
 
 class Precision(enum.IntEnum):

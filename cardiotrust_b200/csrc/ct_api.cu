@@ -52,9 +52,11 @@ struct ct_scn {
   std::vector<void*> allocations;
   std::vector<int32_t> nbr_host;  // neighbour table in reference order, for validating delay writes
   std::vector<int32_t> nbr_dev;   // neighbour table in device order (adjoint reverse table)
+  std::vector<uint8_t> bank;      // (2 y + z) mod 8 of each device voxel's grid coordinates
+  bool symmetric = true;          // a voxel's neighbours all have it as a neighbour
   // Upper bound of the largest delay of a connected pair: exact after creation and delay writes,
   // +1 per update that rolls delays (roll_delays moves a delay by at most one). Sizes the
-  // adjoint ring without reading the device.
+  // exchange ring without reading the device.
   int64_t dmax_bound = 1;
   // Asynchronous read-back of the device's largest delay after an update (pinned word + event):
   // once it has landed, the bound becomes that value plus the updates enqueued since.
@@ -294,69 +296,156 @@ int prepare_sliced(ct_scn* s) {
   return CT_OK;
 }
 
-// Adjoint-mode buffers, allocated on first use (or when the checkpoint interval k changes); the
-// inbox ring grows with the delay bound.
-int prepare_adjoint(ct_scn* s, int k = ct::kCkptSteps) {
+// The exchange ring of the recursion kernels. A tile overwrites the entry of step t - xrows when it
+// finishes step t; by then every tile that it reads has finished step t - dmax and so has staged all
+// rows up to t - dmin - dmax, provided that the tiles that read it are among those that it reads. Without
+// that symmetry the ring holds every step of the beat.
+int prepare_exchange(ct_scn* s) {
   DeviceScenario& d = s->d;
-  cudaStream_t st = s->ctx->stream;
-  const int64_t V = d.V, plane = d.V * kGainCols;
-  if (d.rev && d.ckpt_k != k) {  // re-made below with the new interval
-    CT_CUDA(cudaStreamSynchronize(st), "adjoint re-layout");
-    for (void* p : {(void*)d.rev, (void*)d.ckpt, (void*)d.seg_q}) release(s, p);
-    d.rev = nullptr;
-    d.ckpt = d.seg_q = nullptr;
-  }
-  if (!d.rev) {
-    std::vector<int32_t> rev((size_t)(V * kOffsets), -1);
-    for (int64_t v = 0; v < V; ++v)
-      for (int n = 0; n < kOffsets; ++n) {
-        const int32_t j = s->nbr_dev[(size_t)(v * kOffsets + n)];
-        if (j < 0) continue;
-        int32_t& slot = rev[(size_t)j * kOffsets + n];
-        if (slot >= 0)
-          return fail(CT_ERR_NOT_SUPPORTED,
-                      "adjoint mode: two voxels reach the same neighbour along one offset (not a lattice)");
-        slot = (int32_t)v;
-      }
-    const int64_t nseg = (d.T + k - 1) / k;
-    const int64_t seg_steps = std::min<int64_t>(d.T, k);
-    d.adj_pitch = (int)(((plane + 3) / 4) * 4);
-    d.ckpt_k = k;
-    int rc = alloc(s, &d.rev, V * kOffsets);
-    if (!rc) rc = alloc(s, &d.ckpt, nseg * plane);
-    if (!rc) rc = alloc(s, &d.seg_q, seg_steps * d.adj_pitch);
-    if (!rc && !d.dCk) rc = alloc(s, &d.dCk, plane);
-    if (rc) {
-      for (void* p : {(void*)d.rev, (void*)d.ckpt, (void*)d.seg_q}) release(s, p);
-      d.rev = nullptr;
-      d.ckpt = d.seg_q = nullptr;
-      return rc;
-    }
-    CT_CUDA(cudaMemcpyAsync(d.rev, rev.data(), sizeof(int32_t) * rev.size(), cudaMemcpyHostToDevice, st),
-            "upload reverse table");
-    CT_CUDA(cudaMemsetAsync(d.ckpt, 0, sizeof(float) * nseg * plane, st), "memset");
-    CT_CUDA(cudaMemsetAsync(d.dCk, 0, sizeof(float) * plane, st), "memset");
-    CT_CUDA(cudaStreamSynchronize(st), "adjoint set-up");
-    d.adj_grid = (int)std::min<int64_t>((V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels,
-                                        ct::adjoint_capacity(s->ctx->device));
-  }
-  if (!d.lam_state) {
-    int rc = alloc(s, &d.lam_state, plane + 4);  // +4: the adjoint's bulk copies round sizes up to 16 bytes
-    if (rc) return rc;
-  }
   refresh_delay_bound(s);
-  int need = 1;
-  while (need < s->dmax_bound + ct::kMaxStepBlock + 2) need <<= 1;
-  if (!d.inbox || d.adj_ring < need) {
-    CT_CUDA(cudaStreamSynchronize(st), "adjoint inbox");
-    release(s, d.inbox);
-    d.inbox = nullptr;
-    d.adj_ring = 0;
-    int rc = alloc(s, &d.inbox, (int64_t)need * d.adj_pitch);
-    if (rc) return rc;
-    d.adj_ring = need;
-  }
+  int64_t want = 8, all = 8;
+  while (want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30)) want <<= 1;
+  while (all < d.T) all <<= 1;
+  if (!s->symmetric || want > all) want = all;
+  if (d.xch && d.xrows >= want) return CT_OK;
+  CT_CUDA(cudaStreamSynchronize(s->ctx->stream), "exchange ring");
+  release(s, d.xch);
+  d.xch = nullptr;
+  d.xrows = 0;
+  int rc = alloc(s, &d.xch, want * d.V);
+  if (rc) return rc;
+  d.xrows = (int)want;
   return CT_OK;
+}
+
+// Halo tables of blocks of TV consecutive device voxels, for the source table `src` [V, 26]: the
+// block's source voxels in device order (the list ends with repetitions of the last one), their slots, and
+// each item's slot. A voxel takes a slot with (slot mod 8) = bank while one is free, so that
+// neighbouring voxels' entries fall into different shared-memory banks. count = -1
+// where a block has more than HM - 1 source voxels; slot HM - 1 stands for an absent source.
+struct HaloTables {
+  std::vector<int32_t> halo, count;
+  std::vector<int16_t> pos, slot;
+};
+HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_t>& bank, int64_t V, int TV, int HM) {
+  HaloTables t;
+  const int64_t blocks = (V + TV - 1) / TV;
+  t.halo.assign((size_t)(blocks * HM), 0);
+  t.pos.assign((size_t)(blocks * HM), 0);
+  t.count.assign((size_t)blocks, 0);
+  t.slot.assign((size_t)(blocks * TV * kOffsets), (int16_t)(HM - 1));
+  std::vector<int32_t> seen((size_t)V, -1), list;
+  std::vector<int16_t> place((size_t)V, 0);
+  std::vector<char> taken((size_t)HM);
+  for (int64_t b = 0; b < blocks; ++b) {
+    const int64_t u0 = b * TV, u1 = std::min<int64_t>(V, u0 + TV);
+    list.clear();
+    for (int64_t i = u0 * kOffsets; i < u1 * kOffsets; ++i) {
+      const int32_t w = src[(size_t)i];
+      if (w < 0 || seen[(size_t)w] == (int32_t)b) continue;
+      seen[(size_t)w] = (int32_t)b;
+      list.push_back(w);
+    }
+    if ((int)list.size() > HM - 1) {
+      t.count[(size_t)b] = -1;
+      continue;
+    }
+    t.count[(size_t)b] = (int32_t)list.size();
+    if (list.empty()) continue;
+    std::sort(list.begin(), list.end());
+    std::fill(taken.begin(), taken.end(), 0);
+    int next[8];
+    for (int r = 0; r < 8; ++r) next[r] = r;
+    for (int pass = 0; pass < 2; ++pass) {  // the second pass places what found its bank full
+      int spare = 0;
+      for (int32_t w : list) {
+        int& at = next[bank[(size_t)w]];
+        if (pass == 0) {
+          place[(size_t)w] = -1;
+          if (at >= HM - 1) continue;
+          place[(size_t)w] = (int16_t)at;
+          taken[(size_t)at] = 1;
+          at += 8;
+        } else if (place[(size_t)w] < 0) {
+          while (taken[(size_t)spare]) ++spare;
+          place[(size_t)w] = (int16_t)spare;
+          taken[(size_t)spare] = 1;
+        }
+      }
+    }
+    for (int i = 0; i < HM; ++i) {
+      const int32_t w = list[std::min<size_t>((size_t)i, list.size() - 1)];
+      t.halo[(size_t)(b * HM + i)] = w;
+      t.pos[(size_t)(b * HM + i)] = place[(size_t)w];
+    }
+    for (int64_t i = u0 * kOffsets; i < u1 * kOffsets; ++i)
+      if (src[(size_t)i] >= 0) t.slot[(size_t)i] = place[(size_t)src[(size_t)i]];
+  }
+  return t;
+}
+
+// Adjoint-mode tables and buffers, allocated on first use.
+int prepare_adjoint(ct_scn* s) {
+  DeviceScenario& d = s->d;
+  if (d.rev) return CT_OK;
+  cudaStream_t st = s->ctx->stream;
+  const int64_t V = d.V;
+  std::vector<int32_t> rev((size_t)(V * kOffsets), -1);
+  for (int64_t v = 0; v < V; ++v)
+    for (int n = 0; n < kOffsets; ++n) {
+      const int32_t j = s->nbr_dev[(size_t)(v * kOffsets + n)];
+      if (j < 0) continue;
+      int32_t& slot = rev[(size_t)j * kOffsets + n];
+      if (slot >= 0)
+        return fail(CT_ERR_NOT_SUPPORTED,
+                    "adjoint mode: two voxels reach the same neighbour along one offset (not a lattice)");
+      slot = (int32_t)v;
+    }
+  const HaloTables t = build_halos(rev, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
+  int rc = alloc(s, &d.rhalo, (int64_t)t.halo.size());
+  if (!rc) rc = alloc(s, &d.rhpos, (int64_t)t.pos.size());
+  if (!rc) rc = alloc(s, &d.rhslot, (int64_t)t.slot.size());
+  if (!rc) rc = alloc(s, &d.rnhalo, (int64_t)t.count.size());
+  if (!rc && !d.LX) rc = alloc(s, &d.LX, d.T * d.S);
+  if (!rc) rc = alloc(s, &d.rev, V * kOffsets);
+  if (!rc) rc = upload(s, d.rev, rev.data(), sizeof(int32_t) * rev.size());
+  if (!rc) rc = upload(s, d.rhalo, t.halo.data(), sizeof(int32_t) * t.halo.size());
+  if (!rc) rc = upload(s, d.rhpos, t.pos.data(), sizeof(int16_t) * t.pos.size());
+  if (!rc) rc = upload(s, d.rhslot, t.slot.data(), sizeof(int16_t) * t.slot.size());
+  if (!rc) rc = upload(s, d.rnhalo, t.count.data(), sizeof(int32_t) * t.count.size());
+  if (!rc) {
+    cudaError_t e = cudaStreamSynchronize(st);  // the host tables go out of scope
+    if (e != cudaSuccess) rc = cuda_fail(e, "adjoint set-up");
+  }
+  if (rc) {
+    for (void* p : {(void*)d.rev, (void*)d.rhalo, (void*)d.rhpos, (void*)d.rhslot, (void*)d.rnhalo, (void*)d.LX}) release(s, p);
+    d.rev = d.rhalo = d.rnhalo = nullptr;
+    d.rhslot = d.rhpos = nullptr;
+    d.LX = nullptr;
+  }
+  return rc;
+}
+
+ct::DeriveScalars derive_scalars(const ct_scn* s) {
+  const ct_algorithm& a = s->algo;
+  ct::DeriveScalars ds;
+  ds.mse_scaling = 1.0f / (float)s->d.M * a.mse_strength;
+  ds.reg_scaling = a.maximum_regularization_strength;
+  ds.threshold = a.maximum_regularization_threshold;
+  ds.diffreg = a.difference_regularization_strength;
+  ds.freeze_gains = a.freeze_gains;
+  ds.freeze_delays = a.freeze_delays;
+  ds.ap_derivative = a.ap_derivative;
+  return ds;
+}
+
+ct::WaveScalars wave_scalars(const ct_scn* s) {
+  const ct::DeriveScalars ds = derive_scalars(s);
+  ct::WaveScalars w;
+  w.threshold = ds.threshold;
+  w.mse_scaling = ds.mse_scaling;
+  w.reg_scaling = ds.reg_scaling;
+  return w;
 }
 
 int run_beat(ct_scn* s, int64_t beat, int precision, int grad_mode) {
@@ -364,11 +453,10 @@ int run_beat(ct_scn* s, int64_t beat, int precision, int grad_mode) {
   const ct_algorithm& a = s->algo;
   cudaStream_t st = s->ctx->stream;
   const bool adjoint = grad_mode == CT_GRAD_ADJOINT;
+  int rc = prepare_exchange(s);  // an update of an earlier beat may have rolled delays
+  if (rc) return rc;
   CT_CUDA(run_phase(s, CT_PHASE_FORWARD, 1,
-                    [&] {
-                      return ct::launch_forward(d, a.maximum_regularization_threshold, adjoint ? d.ckpt : nullptr,
-                                                st);
-                    }),
+                    [&] { return ct::launch_forward(d, a.maximum_regularization_threshold, st); }),
           "forward kernel");
   if (precision == CT_PREC_FP32) {
     CT_CUDA(run_phase(s, CT_PHASE_MEASURE, 3, [&] { return ct::launch_measure(d, beat, true, st); }),
@@ -388,26 +476,18 @@ int run_beat(ct_scn* s, int64_t beat, int precision, int grad_mode) {
                       [&] { return ct::launch_map_residuals_umma(d, beat, precision, st); }),
             "tensor-core mapped-residual kernel");
   }
-  if (adjoint && (!a.freeze_gains || !a.freeze_delays)) {
-    ct::AdjointScalars as;
-    as.mse_scaling = 1.0f / (float)d.M * a.mse_strength;
-    as.reg_scaling = a.maximum_regularization_strength;
-    as.threshold = a.maximum_regularization_threshold;
-    as.diffreg = a.difference_regularization_strength;
-    as.freeze_gains = a.freeze_gains;
-    as.freeze_delays = a.freeze_delays;
-    as.ap_derivative = a.ap_derivative;
-    CT_CUDA(run_phase(s, CT_PHASE_DERIVE, 1, [&] { return ct::launch_adjoint(d, as, st); }), "adjoint kernel");
-  } else if (!a.freeze_gains || !a.freeze_delays) {
-    ct::DeriveScalars ds;
-    ds.mse_scaling = 1.0f / (float)d.M * a.mse_strength;
-    ds.reg_scaling = a.maximum_regularization_strength;
-    ds.threshold = a.maximum_regularization_threshold;
-    ds.diffreg = a.difference_regularization_strength;
-    ds.freeze_gains = a.freeze_gains;
-    ds.freeze_delays = a.freeze_delays;
-    ds.ap_derivative = a.ap_derivative;
-    CT_CUDA(run_phase(s, CT_PHASE_DERIVE, 1, [&] { return ct::launch_derive(d, ds, st); }), "derivation kernel");
+  if (!a.freeze_gains || !a.freeze_delays) {
+    const ct::DeriveScalars ds = derive_scalars(s);
+    if (adjoint) {
+      CT_CUDA(run_phase(s, CT_PHASE_DERIVE, 2,
+                        [&] {
+                          cudaError_t e = ct::launch_adjoint_states(d, wave_scalars(s), st);
+                          return e != cudaSuccess ? e : ct::launch_adjoint_gradients(d, ds, st);
+                        }),
+              "adjoint kernels");
+    } else {
+      CT_CUDA(run_phase(s, CT_PHASE_DERIVE, 1, [&] { return ct::launch_derive(d, ds, st); }), "derivation kernel");
+    }
   }
   CT_CUDA(run_phase(s, CT_PHASE_STEP_METRICS, 2,
                     [&] { return ct::launch_step_metrics(d, a.maximum_regularization_strength, st); }),
@@ -485,7 +565,7 @@ const int kOffsetXYZ[kOffsets][3] = {
     {1, 0, 0},    {1, 0, 1},   {1, 1, -1},  {1, 1, 0},   {1, 1, 1}};
 
 void brick_layout(const std::vector<int32_t>& nbr, int64_t V, std::vector<int32_t>& perm,
-                  std::vector<int32_t>& inv) {
+                  std::vector<int32_t>& inv, std::vector<uint8_t>& bank) {
   std::vector<int64_t> cx((size_t)V), cy((size_t)V), cz((size_t)V), comp((size_t)V, -1);
   std::vector<int32_t> queue;
   queue.reserve((size_t)V);
@@ -530,7 +610,12 @@ void brick_layout(const std::vector<int32_t>& nbr, int64_t V, std::vector<int32_
   };
   std::sort(perm.begin(), perm.end(), [&](int32_t a, int32_t b) { return key(a) < key(b); });
   inv.resize((size_t)V);
-  for (int64_t u = 0; u < V; ++u) inv[(size_t)perm[(size_t)u]] = (int32_t)u;
+  bank.resize((size_t)V);
+  for (int64_t u = 0; u < V; ++u) {
+    const size_t v = (size_t)perm[(size_t)u];
+    inv[v] = (int32_t)u;
+    bank[(size_t)u] = (uint8_t)((2 * cy[v] + cz[v]) & 7);
+  }
 }
 
 // Row blocks of `rows_per_voxel` rows of `row_len` elements: device block u <- reference block perm[u].
@@ -571,47 +656,6 @@ void scatter_state_columns(float* dst, const float* src, const std::vector<int32
       dr[3 * v + 2] = sr[3 * u + 2];
     }
   }
-}
-
-// Per forward tile (kFwdTileVoxels consecutive device voxels): the sorted device voxels its
-// (voxel, offset) items read, and each item's slot in that list. False if a neighbourhood
-// exceeds kFwdHaloMax (the resident forward form is then not used).
-bool build_halos(const ct_scn* s, const std::vector<int32_t>& nbr_ref, int64_t tiles, std::vector<int32_t>& halo,
-                 std::vector<int32_t>& nhalo, std::vector<int16_t>& hslot) {
-  const int TV = ct::kFwdTileVoxels, HM = ct::kFwdHaloMax;
-  const int64_t V = (int64_t)s->perm.size();
-  halo.assign((size_t)(tiles * HM), -1);
-  nhalo.assign((size_t)tiles, 0);
-  hslot.assign((size_t)(tiles * TV * kOffsets), -1);
-  std::vector<int32_t> list;
-  for (int64_t t = 0; t < tiles; ++t) {
-    list.clear();
-    for (int vl = 0; vl < TV; ++vl) {
-      const int64_t u = t * TV + vl;
-      if (u >= V) break;
-      for (int n = 0; n < kOffsets; ++n) {
-        const int32_t w = nbr_ref[(size_t)s->perm[(size_t)u] * kOffsets + n];
-        if (w >= 0) list.push_back(s->inv[(size_t)w]);
-      }
-    }
-    std::sort(list.begin(), list.end());
-    list.erase(std::unique(list.begin(), list.end()), list.end());
-    if ((int)list.size() > HM) return false;
-    nhalo[(size_t)t] = (int32_t)list.size();
-    std::copy(list.begin(), list.end(), halo.begin() + (size_t)(t * HM));
-    for (int vl = 0; vl < TV; ++vl) {
-      const int64_t u = t * TV + vl;
-      if (u >= V) break;
-      for (int n = 0; n < kOffsets; ++n) {
-        const int32_t w = nbr_ref[(size_t)s->perm[(size_t)u] * kOffsets + n];
-        if (w < 0) continue;
-        const int32_t dw = s->inv[(size_t)w];
-        hslot[(size_t)((t * TV + vl) * kOffsets + n)] =
-            (int16_t)(std::lower_bound(list.begin(), list.end(), dw) - list.begin());
-      }
-    }
-  }
-  return true;
 }
 
 int validate_and_build_nbr(const ct_scenario_desc* desc, std::vector<int32_t>& nbr) {
@@ -878,7 +922,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   s->algo = *algo;
   s->nbr_host = nbr;
   s->dmax_bound = max_connected_delay(nbr, desc->delays);
-  brick_layout(nbr, S / 3, s->perm, s->inv);
+  brick_layout(nbr, S / 3, s->perm, s->inv, s->bank);
   DeviceScenario& d = s->d;
   d.S = S;
   d.V = S / 3;
@@ -886,14 +930,9 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   d.T = T;
   d.B = B;
   d.NB = desc->num_batch_slots;
-  // forward form: resident (one tile per CTA, halo ring) when every tile fits a co-resident CTA
-  // and every tile's neighbourhood fits the ring; streaming otherwise
-  const int64_t tiles = (d.V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels;
-  std::vector<int32_t> h_halo, h_nhalo;
-  std::vector<int16_t> h_hslot;
-  d.fwd_ring = tiles <= ct::forward_ring_capacity(ctx->device) &&
-               build_halos(s, nbr, tiles, h_halo, h_nhalo, h_hslot);
-  d.fwd_grid = d.fwd_ring ? (int)tiles : ct::forward_grid_size(d.V, ctx->device);
+  d.tiles = (int)((d.V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels);
+  d.wave_grid = std::min(d.tiles, ct::wave_capacity(ctx->device));
+  const int64_t tiles = d.tiles, sweep_blocks = (d.V + ct::kSweepVoxels - 1) / ct::kSweepVoxels;
   {
     const int64_t tiles = ((M + 63) / 64) * ((T + 63) / 64);
     int64_t ks = (2 * ctx->num_sms + tiles - 1) / tiles;
@@ -921,11 +960,10 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
       return r__;                        \
     }                                    \
   } while (0)
-  // +4 elements: the adjoint kernel bulk-copies per-tile ranges rounded up to 16 bytes
-  ALLOC(d.gains, S * kGainCols + 4);
-  ALLOC(d.nbr, V * kOffsets + 4);
-  ALLOC(d.coefs, V * kOffsets + 4);
-  ALLOC(d.delays, V * kOffsets + 4);
+  ALLOC(d.gains, S * kGainCols);
+  ALLOC(d.nbr, V * kOffsets);
+  ALLOC(d.coefs, V * kOffsets);
+  ALLOC(d.delays, V * kOffsets);
   ALLOC(d.init_delays, V * kOffsets);
   ALLOC(d.H, B * M * S);
   ALLOC(d.ctrl, S);
@@ -953,7 +991,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   ALLOC(d.loss_b, d.NB);
   ALLOC(d.loss_mse_b, d.NB);
   ALLOC(d.loss_mr_b, d.NB);
-  ALLOC(d.stepsum_part, T * d.fwd_grid);
+  ALLOC(d.stepsum_part, T * tiles);
   ALLOC(d.gemm_part, part_floats);
   if (d.umma) {
     ALLOC(d.H_hi, B * M * d.spad);
@@ -965,13 +1003,21 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
     ALLOC(d.R_lo, T * d.kpad);
   }
   ALLOC(d.dmin, 2);
-  if (d.fwd_ring) {
-    ALLOC(d.halo, tiles * ct::kFwdHaloMax);
-    ALLOC(d.hslot, tiles * ct::kFwdTileVoxels * kOffsets);
-    ALLOC(d.nhalo, tiles);
+  ALLOC(d.halo, tiles * ct::kFwdHaloMax);
+  ALLOC(d.hpos, tiles * ct::kFwdHaloMax);
+  ALLOC(d.hslot, tiles * ct::kFwdTileVoxels * kOffsets);
+  ALLOC(d.nhalo, tiles);
+  ALLOC(d.shalo, sweep_blocks * ct::kSweepHaloMax);
+  ALLOC(d.shpos, sweep_blocks * ct::kSweepHaloMax);
+  ALLOC(d.shslot, sweep_blocks * ct::kSweepVoxels * kOffsets);
+  ALLOC(d.snhalo, sweep_blocks);
+  if (d.tiles > d.wave_grid) {
+    unsigned char* rec = nullptr;
+    ALLOC(rec, tiles * (int64_t)ct::wave_record_bytes());
+    d.record = reinterpret_cast<float4*>(rec);
   }
   ALLOC(d.status, 1);
-  ALLOC(d.barrier, 1);
+  ALLOC(d.heartbeat, 1);
 #undef ALLOC
   cudaStream_t st = ctx->stream;
   int r = CT_OK;
@@ -992,6 +1038,15 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
       h_nbr[(size_t)(u * kOffsets + n)] = w < 0 ? -1 : s->inv[(size_t)w];
     }
   s->nbr_dev = h_nbr;
+  for (int64_t u = 0; u < V && s->symmetric; ++u)
+    for (int n = 0; n < kOffsets; ++n) {
+      const int32_t w = h_nbr[(size_t)(u * kOffsets + n)];
+      if (w < 0 || h_nbr[(size_t)w * kOffsets + (kOffsets - 1 - n)] == u) continue;
+      const int32_t* row = h_nbr.data() + (size_t)w * kOffsets;
+      if (std::find(row, row + kOffsets, (int32_t)u) == row + kOffsets) s->symmetric = false;
+    }
+  const HaloTables wave_halo = build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
+  const HaloTables sweep_halo = build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax);
   r = r ? r : upload(s, d.gains, h_gains.data(), sizeof(float) * S * kGainCols);
   r = r ? r : upload(s, d.nbr, h_nbr.data(), sizeof(int32_t) * V * kOffsets);
   r = r ? r : upload(s, d.coefs, h_coefs.data(), sizeof(float) * V * kOffsets);
@@ -999,11 +1054,15 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   r = r ? r : upload(s, d.init_delays, h_init.data(), sizeof(float) * V * kOffsets);
   if (desc->measurement_matrix) r = r ? r : upload(s, d.H, h_H.data(), sizeof(float) * B * M * S);
   r = r ? r : upload(s, d.ctrl, h_ctrl.data(), sizeof(float) * S);
-  if (d.fwd_ring) {
-    r = r ? r : upload(s, d.halo, h_halo.data(), sizeof(int32_t) * h_halo.size());
-    r = r ? r : upload(s, d.hslot, h_hslot.data(), sizeof(int16_t) * h_hslot.size());
-    r = r ? r : upload(s, d.nhalo, h_nhalo.data(), sizeof(int32_t) * h_nhalo.size());
-  }
+  r = r ? r : upload(s, d.halo, wave_halo.halo.data(), sizeof(int32_t) * wave_halo.halo.size());
+  r = r ? r : upload(s, d.hpos, wave_halo.pos.data(), sizeof(int16_t) * wave_halo.pos.size());
+  r = r ? r : upload(s, d.hslot, wave_halo.slot.data(), sizeof(int16_t) * wave_halo.slot.size());
+  r = r ? r : upload(s, d.nhalo, wave_halo.count.data(), sizeof(int32_t) * wave_halo.count.size());
+  r = r ? r : upload(s, d.shalo, sweep_halo.halo.data(), sizeof(int32_t) * sweep_halo.halo.size());
+  r = r ? r : upload(s, d.shpos, sweep_halo.pos.data(), sizeof(int16_t) * sweep_halo.pos.size());
+  r = r ? r : upload(s, d.shslot, sweep_halo.slot.data(), sizeof(int16_t) * sweep_halo.slot.size());
+  r = r ? r : upload(s, d.snhalo, sweep_halo.count.data(), sizeof(int32_t) * sweep_halo.count.size());
+  r = r ? r : prepare_exchange(s);
   r = r ? r : upload(s, d.u, desc->control_function, sizeof(float) * T);
   if (!r && desc->measurements) r = upload(s, d.meas, desc->measurements, sizeof(float) * B * T * M);
   if (!r && !desc->measurements) {
@@ -1038,7 +1097,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   zero(d.loss_mse_b, sizeof(float) * d.NB);
   zero(d.loss_mr_b, sizeof(float) * d.NB);
   zero(d.status, sizeof(int32_t));
-  zero(d.barrier, sizeof(ct::GridBarrier));
+  zero(d.heartbeat, sizeof(ct::Heartbeat));
   std::vector<float> nan_v((size_t)V, std::nanf(""));
   r = r ? r : upload(s, d.avg_delays, nan_v.data(), sizeof(float) * V);
   if (!r) {
@@ -1194,7 +1253,7 @@ static int run_epoch_impl(ct_scn* scn, int64_t* batch_index, const int32_t* beat
   int rc = derivatives_reset(scn);
   if (rc) return rc;
   if (grad_mode == CT_GRAD_ADJOINT && (!a.freeze_gains || !a.freeze_delays)) {
-    rc = prepare_adjoint(scn, scn->d.rev ? scn->d.ckpt_k : ct::kCkptSteps);
+    rc = prepare_adjoint(scn);
     if (rc) return rc;
   }
   int64_t batch = 0;
@@ -1235,7 +1294,7 @@ int ct_run_epoch_host(ct_scn* scn, int64_t* batch_index, const int32_t* beat_ord
   DeviceScenario& d = scn->d;
   cudaStream_t st = scn->ctx->stream;
   // the delays of connected pairs must be >= 1, as ct_write_field checks; their largest sizes the
-  // adjoint's inbox ring
+  // exchange ring
   const std::vector<int32_t>& nbr = scn->nbr_host;
   int64_t dmax = 1;
   for (size_t i = 0; i < nbr.size(); ++i) {
@@ -1291,14 +1350,16 @@ int ct_simulate(ct_scn* scn, float* measurements_out, float* states_out) {
   CT_DEVICE_SCOPE(scn->ctx->device);
   DeviceScenario& d = scn->d;
   cudaStream_t st = scn->ctx->stream;
+  int rc = prepare_exchange(scn);
+  if (rc) return rc;
   for (int64_t beat = 0; beat < d.B; ++beat) {
     CT_CUDA(run_phase(scn, CT_PHASE_FORWARD, 1,
-                      [&] { return ct::launch_forward(d, scn->algo.maximum_regularization_threshold, nullptr, st); }),
+                      [&] { return ct::launch_forward(d, scn->algo.maximum_regularization_threshold, st); }),
             "forward kernel");
     CT_CUDA(run_phase(scn, CT_PHASE_MEASURE, 2, [&] { return ct::launch_measure(d, beat, false, st); }),
             "measurement kernel");
   }
-  int rc = ct_sync(scn);
+  rc = ct_sync(scn);
   if (rc) return rc;
   rc = copy_down(scn, measurements_out, d.Y, sizeof(float) * d.B * d.T * d.M);
   if (rc) return rc;
@@ -1544,15 +1605,15 @@ int ct_read_profile(ct_scn* scn, double* ms, int64_t* launches) {
 // A batch runs one epoch of every member scenario as one schedule: per beat
 // index b, one cooperative forward launch over the tiles of every scenario
 // that has a beat b, the measurement products of each scenario on parallel
-// streams, then one cooperative adjoint launch (or the per-scenario reference
-// derivations), the step metrics, and finally every scenario's update. The
+// streams, then (adjoint mode) one cooperative launch of the adjoint recursion, the gradient
+// sweeps, the step metrics, and finally every scenario's update. The
 // whole epoch is captured once as a CUDA graph and replayed; the values that
 // change from epoch to epoch (Adam bias corrections, batch-metric slots) are
 // read by the kernels from a small device array written before each replay.
 
-// Checkpoint interval of batch members in adjoint mode: segment buffers (2K planes) plus
-// checkpoints (T/K planes) are smallest near K = sqrt(T/2), 22..45 for 1,000..4,000 steps.
-constexpr int kBatchCkptSteps = 64;
+// What ct_batch_autotune reports as the checkpoint interval: the recursions store no checkpoints, and
+// the value is kept for callers that log it.
+constexpr int kReportedCkptSteps = 64;
 
 struct EpochDev {
   float bias[2];        // 1 - beta1^step, 1 - beta2^step (host powf, as in update.rs:140-141)
@@ -1565,14 +1626,17 @@ struct ct_batch {
   int grad_mode = CT_GRAD_REFERENCE;
   int precision = CT_PREC_FP32;
   int nbeats_max = 0;
-  int fwd_grid = 0, adj_grid = 0;
-  std::vector<std::vector<int2>> beat_tiles;  // per beat index: tiles of the scenarios with that beat
-  std::vector<int> beat_tmax;
+  int grid = 0;                               // co-resident CTAs of the recursion kernels
+  std::vector<std::vector<int2>> beat_tiles;  // per beat index: tiles of the scenarios with that beat, by phase
+  std::vector<std::vector<int>> beat_phases;  // first tile of each phase, and the end
   std::vector<int2*> beat_tiles_dev;
+  std::vector<int*> beat_phases_dev;          // [tiles + 1]
+  float4* record = nullptr;                   // packed registers of the tiles that share a CTA
+  size_t record_tiles = 0;
   std::vector<float*> parts;                  // per scenario [T, tiles] step partials
   std::vector<int> ntiles;
-  ct::FwdArgs* fwd_dev = nullptr;
-  ct::AdjScn* adj_dev = nullptr;
+  ct::WaveScn* fwd_dev = nullptr;
+  ct::WaveScn* adj_dev = nullptr;
   EpochDev* epoch_dev = nullptr;
   std::vector<void*> allocations;
   std::vector<cudaStream_t> side;
@@ -1580,13 +1644,10 @@ struct ct_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool use_graph = true;
-  std::vector<int> captured_ring;
+  std::vector<int> captured_rows;
   std::vector<uint64_t> captured_gen;
   int64_t graph_kernels = 0;
-  // tuned choices (ct_batch_autotune): adjoint checkpoint interval, tile order
-  int ckpt_k = kBatchCkptSteps;
-  int tile_order = 0;
-  int captured_k = 0;
+  int tile_order = 0;  // tuned choice (ct_batch_autotune): how the tiles are arranged in phases
   // optional per-phase timing (eager launches, CUDA events on the context stream)
   bool profiling = false;
   cudaEvent_t open_event = nullptr;
@@ -1698,24 +1759,22 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     for (size_t i = 0; i < n; ++i) {
       DeviceScenario& d = b->scns[i]->d;
       if (beat >= d.B) continue;
-      B_CUDA(cudaMemsetAsync(d.ap, 0, sizeof(float) * d.V * kGainCols, side_of(i)));
-      B_CUDA(cudaMemsetAsync(d.ap_last, 0, sizeof(float) * d.V * kGainCols, side_of(i)));
-      if (adjoint) {
-        B_CUDA(cudaMemsetAsync(d.inbox, 0, sizeof(float) * d.adj_ring * (size_t)d.adj_pitch, side_of(i)));
-        B_CUDA(cudaMemsetAsync(d.lam_state, 0, sizeof(float) * d.V * kGainCols, side_of(i)));
-      }
+      B_CUDA(ct::clear_exchange(d, side_of(i)));
     }
     B_CUDA(join_side(b));
     DeviceScenario& d0 = b->scns[0]->d;
-    ct::FwdBatch fb;
-    fb.scns = b->fwd_dev;
-    fb.nscn = (int)n;
-    fb.tiles = b->beat_tiles_dev[(size_t)beat];
-    fb.ntiles = (int)b->beat_tiles[(size_t)beat].size();
-    fb.Tmax = b->beat_tmax[(size_t)beat];
-    fb.status = d0.status;
-    fb.barrier = d0.barrier;
-    B_CUDA(ct::launch_forward_batch(fb, std::min(b->fwd_grid, fb.ntiles), st));
+    ct::WaveLaunch wl;
+    wl.scns = b->fwd_dev;
+    wl.nscn = (int)n;
+    wl.tiles = b->beat_tiles_dev[(size_t)beat];
+    wl.phase_begin = b->beat_phases_dev[(size_t)beat];
+    wl.nphases = (int)b->beat_phases[(size_t)beat].size() - 1;
+    wl.ntiles = (int)b->beat_tiles[(size_t)beat].size();
+    wl.record = b->record;
+    wl.status = d0.status;
+    wl.heartbeat = d0.heartbeat;
+    const int wave_grid = std::min(b->grid, wl.ntiles);
+    B_CUDA(ct::launch_wave(wl, false, wave_grid, st));
     B_CUDA(batch_mark(b, CT_PHASE_FORWARD));
     // measurement products, residuals, (reference) derivations and step metrics per scenario
     B_CUDA(fork_side(b));
@@ -1736,32 +1795,24 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
         B_CUDA(ct::launch_measure_umma(d, beat, true, b->precision, ss));
         B_CUDA(ct::launch_map_residuals_umma(d, beat, b->precision, ss));
       }
-      if (!adjoint && (!a.freeze_gains || !a.freeze_delays)) {
-        ct::DeriveScalars ds;
-        ds.mse_scaling = 1.0f / (float)d.M * a.mse_strength;
-        ds.reg_scaling = a.maximum_regularization_strength;
-        ds.threshold = a.maximum_regularization_threshold;
-        ds.diffreg = a.difference_regularization_strength;
-        ds.freeze_gains = a.freeze_gains;
-        ds.freeze_delays = a.freeze_delays;
-        ds.ap_derivative = a.ap_derivative;
-        B_CUDA(ct::launch_derive(d, ds, ss));
-      }
+      if (adjoint)
+        B_CUDA(ct::clear_exchange(d, ss));
+      else if (!a.freeze_gains || !a.freeze_delays)
+        B_CUDA(ct::launch_derive(d, derive_scalars(s), ss));
       B_CUDA(ct::launch_step_metrics_parts(d, b->parts[i], b->ntiles[i], a.maximum_regularization_strength, ss));
     }
     B_CUDA(join_side(b));
     if (adjoint) {
-      ct::AdjLaunch al;
-      al.scns = b->adj_dev;
-      al.nscn = (int)n;
-      al.tiles = fb.tiles;
-      al.ntiles = fb.ntiles;
-      al.Tmax = fb.Tmax;
-      al.ckpt_steps = b->ckpt_k;
-      al.status = d0.status;
-      al.barrier = d0.barrier;
       B_CUDA(batch_mark(b, CT_PHASE_MEASURE));
-      B_CUDA(ct::launch_adjoint_tiles(al, std::min(b->adj_grid, fb.ntiles), st));
+      wl.scns = b->adj_dev;
+      B_CUDA(ct::launch_wave(wl, true, wave_grid, st));
+      B_CUDA(fork_side(b));
+      for (size_t i = 0; i < n; ++i) {
+        ct_scn* s = b->scns[i];
+        if (beat >= s->d.B || (s->algo.freeze_gains && s->algo.freeze_delays)) continue;
+        B_CUDA(ct::launch_adjoint_gradients(s->d, derive_scalars(s), side_of(i)));
+      }
+      B_CUDA(join_side(b));
       B_CUDA(batch_mark(b, CT_PHASE_DERIVE));
     } else {
       B_CUDA(batch_mark(b, CT_PHASE_MEASURE));
@@ -1801,39 +1852,26 @@ int batch_prepare(ct_batch* b) {
   for (size_t i = 0; i < n; ++i) {
     ct_scn* s = b->scns[i];
     if (b->grad_mode == CT_GRAD_ADJOINT) {
-      const int before = s->d.adj_ring;
-      int rc = prepare_adjoint(s, b->ckpt_k);
+      int rc = prepare_adjoint(s);
       if (rc) return rc;
-      if (s->d.adj_ring != before) stale = true;
     }
-    if (b->captured_ring.size() == n && b->captured_ring[i] != s->d.adj_ring) stale = true;
+    int rc = prepare_exchange(s);
+    if (rc) return rc;
+    if (b->captured_rows.size() == n && b->captured_rows[i] != s->d.xrows) stale = true;
     if (b->captured_gen.size() == n && b->captured_gen[i] != s->config_gen) stale = true;
   }
-  if (b->captured_k != b->ckpt_k) stale = true;
-  if (!stale && b->captured_ring.size() == n) return CT_OK;
+  if (!stale && b->captured_rows.size() == n) return CT_OK;
   // descriptors
-  std::vector<ct::FwdArgs> fa(n);
-  std::vector<ct::AdjScn> aa(n);
+  std::vector<ct::WaveScn> fa(n), aa(n);
+  const bool adjoint = b->grad_mode == CT_GRAD_ADJOINT;
   for (size_t i = 0; i < n; ++i) {
     ct_scn* s = b->scns[i];
-    const ct_algorithm& a = s->algo;
-    DeviceScenario& d = s->d;
-    const bool adjoint = b->grad_mode == CT_GRAD_ADJOINT && (!a.freeze_gains || !a.freeze_delays);
-    fa[i] = ct::forward_scenario(d, a.maximum_regularization_threshold, adjoint ? d.ckpt : nullptr, b->parts[i],
-                                 b->ntiles[i]);
-    ct::AdjointScalars as;
-    as.mse_scaling = 1.0f / (float)d.M * a.mse_strength;
-    as.reg_scaling = a.maximum_regularization_strength;
-    as.threshold = a.maximum_regularization_threshold;
-    as.diffreg = a.difference_regularization_strength;
-    as.freeze_gains = a.freeze_gains || !adjoint;
-    as.freeze_delays = a.freeze_delays || !adjoint;
-    as.ap_derivative = a.ap_derivative;
-    aa[i] = b->grad_mode == CT_GRAD_ADJOINT ? ct::adjoint_scenario(d, as) : ct::AdjScn{};
+    fa[i] = ct::wave_scenario(s->d, false, wave_scalars(s), b->parts[i]);
+    if (adjoint) aa[i] = ct::wave_scenario(s->d, true, wave_scalars(s), nullptr);
   }
-  CT_CUDA(cudaMemcpyAsync(b->fwd_dev, fa.data(), sizeof(ct::FwdArgs) * n, cudaMemcpyHostToDevice, st), "batch upload");
-  if (b->grad_mode == CT_GRAD_ADJOINT)
-    CT_CUDA(cudaMemcpyAsync(b->adj_dev, aa.data(), sizeof(ct::AdjScn) * n, cudaMemcpyHostToDevice, st),
+  CT_CUDA(cudaMemcpyAsync(b->fwd_dev, fa.data(), sizeof(ct::WaveScn) * n, cudaMemcpyHostToDevice, st), "batch upload");
+  if (adjoint)
+    CT_CUDA(cudaMemcpyAsync(b->adj_dev, aa.data(), sizeof(ct::WaveScn) * n, cudaMemcpyHostToDevice, st),
             "batch upload");
   CT_CUDA(cudaStreamSynchronize(st), "batch upload");
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -1877,63 +1915,99 @@ int batch_prepare(ct_batch* b) {
       b->use_graph = false;
     }
   }
-  b->captured_k = b->ckpt_k;
-  b->captured_ring.assign(n, 0);
+  b->captured_rows.assign(n, 0);
   b->captured_gen.assign(n, 0);
   for (size_t i = 0; i < n; ++i) {
-    b->captured_ring[i] = b->scns[i]->d.adj_ring;
+    b->captured_rows[i] = b->scns[i]->d.xrows;
     b->captured_gen[i] = b->scns[i]->config_gen;
   }
   return CT_OK;
 }
 
-// Tile lists per beat index. Order 0: scenarios by decreasing beat length, each scenario's tiles
-// together, so that at any step the live tiles form a prefix of the list, which the round-robin
-// tile -> CTA assignment (CTA c takes tiles c, c + G, ...) spreads evenly. Order 1: the same list
-// folded back and forth over the adjoint grid (chunk k of G tiles reversed when k is odd), so that
-// no CTA always gets the first tile of a chunk. Order 2: scenarios by decreasing beat length, their
-// tiles interleaved one at a time.
+// Tile lists and phases per beat index. A scenario whose tiles fit the grid runs with one tile per
+// CTA, which then keeps the tile's parameters and chains in registers for the whole beat; scenarios are
+// packed into phases of at most `grid` tiles, longest beats first. A scenario with more tiles makes a phase of
+// its own in which every CTA visits k tiles in turn. Order 0: shorter scenarios fill the places that
+// such a phase leaves free. Order 1: they don't. Order 2: one phase with every tile.
 int batch_build_tiles(ct_batch* b, bool upload) {
   const size_t n = b->scns.size();
   std::vector<size_t> order(n);
   for (size_t i = 0; i < n; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return b->scns[x]->d.T > b->scns[y]->d.T; });
   b->beat_tiles.assign((size_t)b->nbeats_max, {});
-  b->beat_tmax.assign((size_t)b->nbeats_max, 0);
+  b->beat_phases.assign((size_t)b->nbeats_max, {});
+  size_t shared_tiles = 0;  // tiles of phases with several tiles per CTA; these phases come first
   for (int beat = 0; beat < b->nbeats_max; ++beat) {
-    std::vector<int2>& tl = b->beat_tiles[(size_t)beat];
-    if (b->tile_order == 2) {
-      for (int t = 0;; ++t) {
-        bool any = false;
-        for (size_t i : order) {
-          DeviceScenario& d = b->scns[i]->d;
-          if (beat >= d.B || t >= b->ntiles[i]) continue;
-          tl.push_back(make_int2((int)i, t * ct::kFwdTileVoxels));
-          any = true;
-        }
-        if (!any) break;
-      }
-    } else {
-      for (size_t i : order) {
-        DeviceScenario& d = b->scns[i]->d;
-        if (beat >= d.B) continue;
-        for (int t = 0; t < b->ntiles[i]; ++t) tl.push_back(make_int2((int)i, t * ct::kFwdTileVoxels));
-      }
-      if (b->tile_order == 1 && b->adj_grid > 0) {
-        const size_t G = (size_t)b->adj_grid;
-        for (size_t k = 1; k * G < tl.size(); k += 2)
-          std::reverse(tl.begin() + (ptrdiff_t)(k * G), tl.begin() + (ptrdiff_t)std::min(tl.size(), (k + 1) * G));
+    struct Phase {
+      int64_t room;
+      std::vector<size_t> members;
+    };
+    std::vector<Phase> large, small;
+    const int64_t G = b->grid;
+    std::vector<size_t> rest;
+    for (size_t i : order) {
+      if (beat >= b->scns[i]->d.B) continue;
+      const int64_t nt = b->ntiles[i];
+      if (b->tile_order == 2) {
+        if (large.empty()) large.push_back({0, {}});
+        large[0].members.push_back(i);
+      } else if (nt > G) {
+        large.push_back({(nt + G - 1) / G * G - nt, {i}});
+      } else {
+        rest.push_back(i);
       }
     }
-    for (const int2& t : tl)
-      b->beat_tmax[(size_t)beat] = std::max<int>(b->beat_tmax[(size_t)beat], (int)b->scns[(size_t)t.x]->d.T);
+    for (size_t i : rest) {
+      const int64_t nt = b->ntiles[i];
+      Phase* at = nullptr;
+      if (b->tile_order == 0)
+        for (Phase& ph : large)
+          if (!at && ph.room >= nt && b->scns[ph.members[0]]->d.T >= b->scns[i]->d.T) at = &ph;
+      for (Phase& ph : small)
+        if (!at && ph.room >= nt) at = &ph;
+      if (!at) {
+        small.push_back({G, {}});
+        at = &small.back();
+      }
+      at->members.push_back(i);
+      at->room -= nt;
+    }
+    std::vector<int2>& tl = b->beat_tiles[(size_t)beat];
+    std::vector<int>& pb = b->beat_phases[(size_t)beat];
+    for (const std::vector<Phase>* group : {&large, &small})
+      for (const Phase& ph : *group) {
+        pb.push_back((int)tl.size());
+        for (size_t i : ph.members)
+          for (int t = 0; t < b->ntiles[i]; ++t) tl.push_back(make_int2((int)i, t * ct::kFwdTileVoxels));
+        if ((int64_t)tl.size() - pb.back() > G) shared_tiles = std::max(shared_tiles, tl.size());
+      }
+    pb.push_back((int)tl.size());
   }
-  if (upload)
+  if (upload) {
+    CT_CUDA(cudaStreamSynchronize(b->ctx->stream), "batch tiles");
+    if (shared_tiles > b->record_tiles) {
+      if (b->record) {
+        cudaFree(b->record);
+        b->allocations.erase(std::remove(b->allocations.begin(), b->allocations.end(), (void*)b->record),
+                             b->allocations.end());
+      }
+      b->record = nullptr;
+      b->record_tiles = 0;
+      void* p = nullptr;
+      int rc = batch_alloc(b, &p, shared_tiles * ct::wave_record_bytes());
+      if (rc) return rc;
+      b->record = static_cast<float4*>(p);
+      b->record_tiles = shared_tiles;
+    }
     for (int beat = 0; beat < b->nbeats_max; ++beat) {
       const auto& tl = b->beat_tiles[(size_t)beat];
+      const auto& pb = b->beat_phases[(size_t)beat];
       CT_CUDA(cudaMemcpy(b->beat_tiles_dev[(size_t)beat], tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice),
               "batch tiles");
+      CT_CUDA(cudaMemcpy(b->beat_phases_dev[(size_t)beat], pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice),
+              "batch phases");
     }
+  }
   return CT_OK;
 }
 
@@ -1984,15 +2058,14 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
     b->ntiles[i] = (int)((d.V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels);
     b->nbeats_max = std::max<int>(b->nbeats_max, (int)d.B);
   }
-  b->fwd_grid = ct::forward_batch_capacity(ctx->device);
-  b->adj_grid = ct::adjoint_capacity(ctx->device);
+  b->grid = ct::wave_capacity(ctx->device);
   batch_build_tiles(b, false);
   void* p = nullptr;
-  rc = batch_alloc(b, &p, sizeof(ct::FwdArgs) * n);
-  b->fwd_dev = static_cast<ct::FwdArgs*>(p);
+  rc = batch_alloc(b, &p, sizeof(ct::WaveScn) * n);
+  b->fwd_dev = static_cast<ct::WaveScn*>(p);
   if (!rc) {
-    rc = batch_alloc(b, &p, sizeof(ct::AdjScn) * n);
-    b->adj_dev = static_cast<ct::AdjScn*>(p);
+    rc = batch_alloc(b, &p, sizeof(ct::WaveScn) * n);
+    b->adj_dev = static_cast<ct::WaveScn*>(p);
   }
   if (!rc) {
     rc = batch_alloc(b, &p, sizeof(EpochDev) * n);
@@ -2007,11 +2080,10 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
     const auto& tl = b->beat_tiles[(size_t)beat];
     rc = batch_alloc(b, &p, sizeof(int2) * tl.size());
     b->beat_tiles_dev.push_back(static_cast<int2*>(p));
-    if (!rc) {
-      cudaError_t e = cudaMemcpy(p, tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) rc = cuda_fail(e, "batch tiles");
-    }
+    if (!rc) rc = batch_alloc(b, &p, sizeof(int) * (n + 2));  // phases never outnumber the members
+    b->beat_phases_dev.push_back(static_cast<int*>(p));
   }
+  if (!rc) rc = batch_build_tiles(b, true);
   const int nside = (int)std::min<size_t>(n, 8);
   for (int i = 0; i < nside && !rc; ++i) {
     cudaStream_t s = nullptr;
@@ -2093,8 +2165,7 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
   CT_CUDA(cudaEventCreate(&e1), "cudaEventCreate");
   const bool was_profiling = b->profiling;
   b->profiling = false;
-  auto trial = [&](int k, int order, double* ms) -> int {
-    b->ckpt_k = k;
+  auto trial = [&](int order, double* ms) -> int {
     b->tile_order = order;
     int rc = batch_build_tiles(b, true);
     if (rc) return rc;
@@ -2102,8 +2173,8 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
-    b->captured_ring.clear();
-    rc = batch_prepare(b);  // re-layout for k, capture
+    b->captured_rows.clear();
+    rc = batch_prepare(b);  // capture
     if (rc) return rc;
     CT_CUDA(cudaStreamSynchronize(st), "autotune");
     CT_CUDA(cudaEventRecord(e0, st), "cudaEventRecord");
@@ -2117,28 +2188,21 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
     *ms = t;
     return CT_OK;
   };
-  int best_k = b->ckpt_k, best_o = b->tile_order;
+  int best_o = b->tile_order;
   double best = 1e300;
   int rc = CT_OK;
-  const int ks[3] = {32, 64, 128};
-  for (int k : ks) {
+  // adjoint mode trains five trial epochs, reference mode three; the first order is timed again while
+  // members' first passes still warm up
+  for (int trial_no = b->grad_mode == CT_GRAD_ADJOINT ? -2 : 0; trial_no <= 2 && !rc; ++trial_no) {
+    const int o = std::max(0, trial_no);
     double ms = 0.0;
-    if (b->grad_mode != CT_GRAD_ADJOINT && k != kBatchCkptSteps) continue;  // the interval only matters for adjoint
-    rc = trial(k, 0, &ms);
-    if (rc) break;
-    if (ms < best) best = ms, best_k = k, best_o = 0;
-  }
-  for (int o = 1; o <= 2 && !rc; ++o) {
-    double ms = 0.0;
-    rc = trial(best_k, o, &ms);
-    if (rc) break;
-    if (ms < best) best = ms, best_o = o;
+    rc = trial(o, &ms);
+    if (!rc && ms < best) best = ms, best_o = o;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   b->profiling = was_profiling;
   if (rc) return rc;
-  b->ckpt_k = best_k;
   b->tile_order = best_o;
   rc = batch_build_tiles(b, true);
   if (rc) return rc;
@@ -2146,8 +2210,8 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
   if (b->graph) cudaGraphDestroy(b->graph);
   b->exec = nullptr;
   b->graph = nullptr;
-  b->captured_ring.clear();
-  if (ckpt_k) *ckpt_k = best_k;
+  b->captured_rows.clear();
+  if (ckpt_k) *ckpt_k = kReportedCkptSteps;
   if (tile_order) *tile_order = best_o;
   if (best_ms) *best_ms = best;
   return CT_OK;
@@ -2191,8 +2255,8 @@ int ct_batch_info(ct_batch* b, int64_t* graph_kernels, int* uses_graph, int* for
   if (!b) return fail(CT_ERR_INVALID_ARGUMENT, "batch is NULL");
   if (graph_kernels) *graph_kernels = b->graph_kernels;
   if (uses_graph) *uses_graph = b->exec != nullptr ? 1 : 0;
-  if (forward_ctas) *forward_ctas = b->fwd_grid;
-  if (adjoint_ctas) *adjoint_ctas = b->adj_grid;
+  if (forward_ctas) *forward_ctas = b->grid;
+  if (adjoint_ctas) *adjoint_ctas = b->grid;
   return CT_OK;
 }
 
@@ -2410,7 +2474,6 @@ int ct_batch_run_model_based(ct_batch* batch, const ct_run_config* cfg, int64_t*
       ct_batch* nb = nullptr;
       rc = ct_batch_create(batch->ctx, scns.data(), (int64_t)scns.size(), batch->grad_mode, batch->precision, &nb);
       if (!rc) {
-        nb->ckpt_k = batch->ckpt_k;
         nb->tile_order = batch->tile_order;
         rc = batch_build_tiles(nb, true);
       }

@@ -13,13 +13,13 @@ namespace ct {
 
 constexpr int kOffsets = 26;   // neighbour offsets per voxel
 constexpr int kGainCols = 78;  // 26 offsets x 3 neighbour components
-constexpr int kMaxStepBlock = 8;  // steps advanced between grid barriers in the forward kernel
-constexpr int kFwdTileVoxels = 32;  // voxels per forward tile (consecutive in device order)
-constexpr int kFwdHaloMax = 160;    // largest neighbourhood of a tile the resident forward form stages
-constexpr int kCkptSteps = 256;     // adjoint mode: default all-pass checkpoint interval (power of two)
+constexpr int kFwdTileVoxels = 32;  // voxels per tile of the recursions (consecutive in device order)
+constexpr int kFwdHaloMax = 192;    // halo slots of a tile; the last one stands for absent neighbours
+constexpr int kSweepVoxels = 8;     // voxels per block of the gradient sweep
+constexpr int kSweepHaloMax = 96;   // halo slots of such a block
 
-// Device-side grid barrier state: a monotone arrival counter, zeroed before each launch.
-struct GridBarrier {
+// Counts the progress of a launch, so that a bounded wait can tell a long wait from a lost one.
+struct Heartbeat {
   unsigned int count;
   unsigned int unused;
 };
@@ -57,9 +57,10 @@ struct DeviceScenario {
   float* loss, *loss_mse, *loss_mr;          // [T]
   float* loss_b, *loss_mse_b, *loss_mr_b;    // [NB]
   // scratch
-  float* stepsum_part;   // [T, fwd_grid] per-CTA partial max-regularisation sums
+  float* stepsum_part;   // [T, tiles] per-tile max-regularisation sums
   float* gemm_part;      // [ksplit, T, Mpad] split-K partials of H x
-  int fwd_grid;          // CTAs of the forward kernel
+  int tiles;             // tiles of kFwdTileVoxels voxels
+  int wave_grid;         // CTAs of the recursion kernels
   int ksplit;            // split-K factor of the H x product (CUDA-core form)
   // tensor-core form (ct_umma.cu); null when the scenario does not support it
   bool umma;             // S % 4 == 0 and the TMA encoder is available
@@ -82,27 +83,31 @@ struct DeviceScenario {
   __nv_bfloat16* R_sl;       // [3][T][kpm] slices of the beat's residuals
   float* R_sc;               // [T][ceil(kpm/512)]
   int32_t* dmin;         // [2] smallest and largest delay of a connected (voxel, offset) pair
-  // resident forward form (one tile per CTA, halo history in a shared ring)
-  bool fwd_ring;
-  int32_t* halo;         // [tiles, kFwdHaloMax] device voxels of each tile's neighbourhood
-  int16_t* hslot;        // [tiles, 26 * kFwdTileVoxels] halo slot of each item's neighbour, -1 if absent
-  int32_t* nhalo;        // [tiles]
-  // adjoint mode (ct_adjoint.cu), allocated on first use
+  // exchange ring of the recursion kernels: [xrows, V] entries {x0, x1, x2, step + 1}
+  uint4* xch;
+  int xrows;             // power of two; grows with the delays
+  float4* record;        // packed registers of tiles that share a CTA, null when every tile has its own
+  // halo tables: slots of each tile's (and each sweep block's) neighbourhood
+  int32_t* halo;         // [tiles, kFwdHaloMax] device voxels of the halo in order, the last one repeated
+  int16_t* hpos;         // [tiles, kFwdHaloMax] their slots
+  int16_t* hslot;        // [tiles, 26 * kFwdTileVoxels] slot of each item's neighbour
+  int32_t* nhalo;        // [tiles] voxels of the halo, -1 if it is too large for the slots
+  int32_t* shalo;        // [sweep blocks, kSweepHaloMax]
+  int16_t* shpos;
+  int16_t* shslot;       // [sweep blocks, 26 * kSweepVoxels]
+  int32_t* snhalo;       // [sweep blocks]
+  // adjoint mode, allocated on first use
   int32_t* rev;          // [V,26] voxel whose offset n points at this voxel, -1 if none
-  int ckpt_k;            // checkpoint interval K (power of two)
-  float* ckpt;           // [ceil(T/K), V, 78] all-pass state before step s * K
-  float* seg_q;          // [min(T, K), pitch] in_t - ap[t-1] of one segment
-  float* inbox;          // [adj_ring, V, 78] adjoint contributions addressed to (voxel, column) by step
-  float* lam_state;      // [V,78] adjoint all-pass state between blocks of steps
-  float* dCk;            // [V,78] per-column coefficient-gradient partials
-  int adj_ring;          // inbox slots (power of two)
-  int adj_pitch;         // floats per plane of seg_q and inbox: V * 78 rounded up to 4 (16-byte rows)
-  int adj_grid;          // CTAs of the adjoint kernel
+  int32_t* rhalo;        // the tiles' halo tables of that direction
+  int16_t* rhpos;
+  int16_t* rhslot;
+  int32_t* rnhalo;
+  float* LX;             // [T,S] gradient of the loss with respect to the states
   // plain form (ct_plain.cu), allocated on first use
   float* plain_mreg;     // [S] maximum regularisation of the current step
   float* plain_part;     // [ceil(V / 256)] per-block sums of the step's regularisation terms
   int32_t* status;       // [1] device-side error code (0 = ok)
-  GridBarrier* barrier;  // [1]
+  Heartbeat* heartbeat;  // [1]
 };
 
 // Records `message` as the calling thread's last error (read by ct_last_error); returns status.
@@ -110,48 +115,60 @@ int report_error(int status, const char* message);
 
 // ---- launchers (all enqueue on `stream`, return cudaError_t of the launch)
 
-// One scenario as the forward kernels see it.
-struct FwdArgs {
-  int V, S, T;
-  int part_stride;  // batched form: tiles of the scenario (stride of stepsum_part rows)
-  const int32_t* nbr;
+// One scenario as the recursion kernel sees it, in one direction (ct_wave.cu).
+struct WaveScn {
+  int V, T, ntiles;
+  int xrows;
+  const int32_t* src;  // [V,26] voxel whose rows item (v, n) gathers, -1 = none
+  const int32_t* halo;
+  const int16_t* hpos;
+  const int16_t* hslot;
+  const int32_t* nhalo;
   const float* coefs;
   const int32_t* delays;
   const float* gains;
+  const int32_t* dmin;
+  uint4* xch;
+  float* rows;         // [T,S] finished rows: states, or their gradient
+  // forward
   const float* ctrl;
   const float* u;
-  float* X;
   float* ap;
   float* ap_last;
-  float* stepsum_part;
-  float* ckpt;  // adjoint checkpoints [ceil(T / ckpt_k), V, 78] or null
-  int ckpt_k;   // checkpoint interval (power of two)
-  const int32_t* dmin;
-  float threshold;
-  int32_t* status;
-  GridBarrier* barrier;
+  float* part;         // [T, ntiles]
+  // adjoint
+  const float* X;
+  const float* MR;
+  float threshold, mse_scaling, reg_scaling;
 };
-// One cooperative forward launch over the tiles of several scenarios (batched form).
-struct FwdBatch {
-  const FwdArgs* scns;  // device array
+struct WaveScalars {
+  float threshold = 0.0f, mse_scaling = 0.0f, reg_scaling = 0.0f;
+};
+// One cooperative launch over the tiles of one or more scenarios. The tiles come in phases; a CTA
+// owns every gridDim-th tile of a phase and goes on to the next phase by itself.
+struct WaveLaunch {
+  const WaveScn* scns;     // device array of nscn scenarios, or null: `single` is the only one
+  WaveScn single;
   int nscn;
-  const int2* tiles;    // (scenario, first voxel)
+  const int2* tiles;       // (scenario, first voxel) per tile, or null: tiles of 32 voxels of scenario 0
+  const int* phase_begin;  // [nphases + 1] first tile of each phase, or null: one phase
+  int nphases;
   int ntiles;
-  int Tmax;
+  float4* record;          // [ntiles] packed registers, null if no CTA owns two tiles of a phase
   int32_t* status;
-  GridBarrier* barrier;
+  Heartbeat* heartbeat;
 };
-FwdArgs forward_scenario(const DeviceScenario& d, float threshold, float* ckpt, float* part, int part_stride);
-// The caller zeroes every scenario's ap and ap_last first.
-cudaError_t launch_forward_batch(const FwdBatch& b, int grid, cudaStream_t stream);
-int forward_batch_capacity(int device);
-
-// Forward propagation of one beat: X[t,:] for t in [0,T). With ckpt non-null the all-pass
-// state before every step s * d.ckpt_k (s >= 1) is stored in ckpt[s].
-cudaError_t launch_forward(DeviceScenario& d, float threshold, float* ckpt, cudaStream_t stream);
-// CTAs of the streaming form, and how many CTAs of the resident form fit on the device.
-int forward_grid_size(int64_t V, int device);
-int forward_ring_capacity(int device);
+WaveScn wave_scenario(const DeviceScenario& d, bool adjoint, const WaveScalars& s, float* part);
+// How many CTAs of the recursion kernel are co-resident, and the bytes of one tile's record.
+int wave_capacity(int device);
+size_t wave_record_bytes();
+// The caller clears every scenario's exchange ring first.
+cudaError_t launch_wave(const WaveLaunch& launch, bool adjoint, int grid, cudaStream_t stream);
+cudaError_t clear_exchange(DeviceScenario& d, cudaStream_t stream);
+// Forward propagation of one beat: X[t,:] for t in [0,T).
+cudaError_t launch_forward(DeviceScenario& d, float threshold, cudaStream_t stream);
+// Back-propagation through time of one beat (needs X and MR): LX = dL/dX.
+cudaError_t launch_adjoint_states(DeviceScenario& d, const WaveScalars& s, cudaStream_t stream);
 
 // y = H[beat] x for all steps; Y[beat] = y, R = y - meas[beat], loss_mse[t].
 cudaError_t launch_measure(DeviceScenario& d, int64_t beat, bool with_residuals, cudaStream_t stream);
@@ -184,52 +201,8 @@ struct DeriveScalars {
 };
 // Per-(voxel, offset) sweep over the steps of one beat: dG, dC, fir, iir.
 cudaError_t launch_derive(DeviceScenario& d, const DeriveScalars& s, cudaStream_t stream);
-
-struct AdjointScalars {
-  float mse_scaling, reg_scaling, threshold, diffreg;
-  int freeze_gains, freeze_delays, ap_derivative;
-};
-// One scenario as the adjoint kernel sees it (device pointers, sizes, scalars).
-struct AdjScn {
-  int V, S, T, ring;
-  int pitch;  // floats between consecutive planes of seg_q and inbox (V * 78 rounded up to 4)
-  const int32_t* nbr;
-  const float* coefs;
-  const int32_t* delays;
-  const float* init_delays;
-  const float* gains;
-  const float* X;
-  const float* MR;
-  const float* ckpt;
-  float* seg_q;
-  float* inbox;
-  float* lam_state;
-  float* dG;
-  float* dC;
-  float* dCk;
-  const int32_t* dmin;
-  float mse_scaling, reg_scaling, threshold, diffreg;
-  int freeze_gains, freeze_delays, ap_derivative;
-};
-// One cooperative adjoint launch over the tiles of one or more scenarios.
-struct AdjLaunch {
-  const AdjScn* scns;  // device array of nscn scenarios, or null: `single` is the only one
-  AdjScn single;
-  int nscn;
-  const int2* tiles;  // (scenario, first voxel) per tile, or null: tiles of 32 voxels of scenario 0
-  int ntiles;
-  int Tmax;           // longest beat of the launch
-  int ckpt_steps;     // checkpoint interval (power of two)
-  int32_t* status;
-  GridBarrier* barrier;
-};
-AdjScn adjoint_scenario(const DeviceScenario& d, const AdjointScalars& s);
-// Back-propagation through time of one beat (needs X, MR and the forward's checkpoints): dG, dC.
-cudaError_t launch_adjoint(DeviceScenario& d, const AdjointScalars& s, cudaStream_t stream);
-// The same over a tile list; the caller zeroes every scenario's inbox and lam_state first.
-cudaError_t launch_adjoint_tiles(const AdjLaunch& launch, int grid, cudaStream_t stream);
-// How many CTAs of the adjoint kernel fit on the device at once.
-int adjoint_capacity(int device);
+// The same sweep for the gradients of the stated loss, from LX: dG, dC.
+cudaError_t launch_adjoint_gradients(DeviceScenario& d, const DeriveScalars& s, cudaStream_t stream);
 
 struct PlainScalars {
   float mse_scaling, reg_scaling, threshold, diffreg;
@@ -244,7 +217,7 @@ cudaError_t launch_step_metrics(DeviceScenario& d, float reg_strength, cudaStrea
 // Batch metrics into slot `index`; the _dev form reads the slot on the device (graph replay).
 cudaError_t launch_batch_metrics(DeviceScenario& d, int64_t index, cudaStream_t stream);
 cudaError_t launch_batch_metrics_dev(DeviceScenario& d, const int64_t* index_dev, cudaStream_t stream);
-// Step metrics from `parts` per-step partial sums (the batched forward's per-tile partials).
+// Step metrics from `parts` per-step partial sums (the forward's per-tile partials).
 cudaError_t launch_step_metrics_parts(DeviceScenario& d, const float* part, int parts, float reg_strength,
                                       cudaStream_t stream);
 

@@ -139,7 +139,7 @@ __global__ void smoothness_kernel(const float* __restrict__ avg, const int32_t* 
 }
 
 // ---- metrics::calculate_step (metrics.rs:180-196) for all steps of a beat.
-// stepsum[t] = sum over forward CTAs of their partial max-regularisation sums
+// stepsum[t] = sum over the forward tiles of their max-regularisation sums
 // (step_sum_kernel: one warp per step, a fixed order), then a deterministic block
 // scan gives the running sum.
 
@@ -325,7 +325,7 @@ cudaError_t launch_smoothness(DeviceScenario& d, float strength, cudaStream_t st
 // The per-step sums go to loss_mr, which the scan then overwrites with the running sum in place (each
 // step's value is read and written by the same thread).
 cudaError_t launch_step_metrics(DeviceScenario& d, float reg_strength, cudaStream_t stream) {
-  return launch_step_metrics_parts(d, d.stepsum_part, d.fwd_grid, reg_strength, stream);
+  return launch_step_metrics_parts(d, d.stepsum_part, d.tiles, reg_strength, stream);
 }
 
 cudaError_t launch_batch_metrics(DeviceScenario& d, int64_t index, cudaStream_t stream) {

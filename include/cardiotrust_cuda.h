@@ -67,8 +67,8 @@ enum ct_grad_mode {
   CT_GRAD_REFERENCE = 0, /* the reference's per-step derivation, derivation.rs:173-229 */
   /* Exact gradient of the stated loss sum_t (mse/M)/2 |r_t|^2 + reg/2 sum_v relu(|x_v|_1 - thr)^2
    * by back-propagation through time (no counterpart in the reference), plus the reference's
-   * difference-regularisation term. All-pass state is checkpointed every 256 steps and the
-   * segments in between are recomputed. Forward, metrics and update are those of mode 0. */
+   * difference-regularisation term. The gradient of the states is kept for the beat; the all-pass
+   * history is not. Forward, metrics and update are those of mode 0. */
   CT_GRAD_ADJOINT = 1
 };
 /* Arithmetic of the two measurement products (H x and H^T r). */
@@ -200,8 +200,8 @@ int ct_scenario_dims(ct_scn* scn, int64_t* S, int64_t* M, int64_t* T, int64_t* B
 /* One estimation epoch, enqueued on the context stream (asynchronous).
  * beat_order: B beat indices, or NULL for the library's seeded shuffle.
  * batch_index: in/out batch-wise metric cursor (algorithm.rs:126).
- * grad_mode: ct_grad_mode. CT_GRAD_ADJOINT allocates its checkpoint and segment buffers on
- * first use (about (T/256 + 256 * 2 + ring) x V x 78 floats) and needs every voxel pair to be
+ * grad_mode: ct_grad_mode. CT_GRAD_ADJOINT allocates the gradient of the states on
+ * first use (T x num_states floats) and needs every voxel pair to be
  * connected along at most one offset (true of the reference's lattice).
  * Device-side failures are reported by ct_sync. */
 int ct_run_epoch(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order, int grad_mode, int precision);
@@ -245,11 +245,12 @@ int ct_batch_destroy(ct_batch* batch);
  * batch_indices: in/out batch-wise metric cursor per member (as ct_run_epoch's batch_index). */
 int ct_batch_run_epoch(ct_batch* batch, int64_t* batch_indices);
 /* Autotuner: runs real epochs of the batch (each one trains and advances batch_indices like
- * ct_batch_run_epoch) under candidate schedules and keeps the fastest: the adjoint checkpoint
- * interval (32, 64, 128 steps; memory against recompute granularity) and the order of the tile
- * lists (by beat length; folded over the grid; interleaved across members), which sets how the
+ * ct_batch_run_epoch) under candidate schedules and keeps the fastest: the arrangement of the
+ * members' tiles in phases (0: small members fill the places that a large member's phase leaves
+ * free; 1: every large member by itself; 2: one phase), which sets how the
  * tiles of members of different sizes spread over the CTAs. Up to five epochs; synchronous.
- * Writes the choice and its epoch time (ms) to the non-NULL outputs. */
+ * Writes the choice and its epoch time (ms) to the non-NULL outputs; ckpt_k, once the adjoint's
+ * checkpoint interval, receives 64 (no checkpoints are stored). */
 int ct_batch_autotune(ct_batch* batch, int64_t* batch_indices, int* ckpt_k, int* tile_order, double* best_ms);
 /* Waits for the batch and reports any device-side failure of a member. */
 int ct_batch_sync(ct_batch* batch);
