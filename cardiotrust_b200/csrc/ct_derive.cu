@@ -43,7 +43,6 @@ namespace {
 constexpr int kVox = kSweepVoxels;
 constexpr int kThreads = kVox * kOffsets;  // 208
 constexpr int kSlots = kSweepHaloMax;      // per ring row; the last one stays zero
-constexpr int kZero = kSlots - 1;
 constexpr int kRows = 32;   // power of two
 constexpr int kChunk = 8;   // steps staged together
 constexpr int kCols = (3 * (kSlots - 1) + kThreads - 1) / kThreads;  // halo words per thread and row
@@ -74,14 +73,14 @@ struct SweepArgs {
 
 struct SweepSmem {
   float4 ring[kRows][kSlots];
-  float4 x[2][kChunk][kVox];    // the voxels' states (reference mode)
-  float4 row[2][kChunk][kVox];  // mapped residuals or lx
-  float4 q[kChunk][kVox];       // reference mode: fma(mr, mse/M, maxreg * reg)
+  float4 x[3][kChunk][kVox];    // the voxels' states (reference mode)
+  float4 row[3][kChunk][kVox];  // mapped residuals or lx
+  float4 q[2][kChunk][kVox];    // reference mode: fma(mr, mse/M, maxreg * reg)
 };
+static_assert(sizeof(SweepSmem) <= 233472 / 4 - 1024, "four blocks per SM");
 
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -89,12 +88,77 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// What a thread keeps through the sweep.
+struct Item {
+  float g[3][3], dG[3][3], sG[3][3];
+  float ap[3], prev[3], fir[3], iir[3];  // adjoint: fir is the tangent z
+  float c, minus_fir, minus_iir, dr_dd, mse, dC, sC;
+  bool valid;
+};
+
+// One step of an item. in: its delayed input (zero before the beat); r: the voxel's mapped residuals or lx; q:
+// their factor of the gain gradients; on: t >= d.
+template <int MODE, bool GAINS, bool COEFS>
+__device__ __forceinline__ void sweep_step(Item& k, const float (&in)[3], const float (&r)[3], const float (&q)[3], bool on) {
+  constexpr bool kAdj = MODE == kAdjoint;
+  float last[3];
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    last[b] = k.ap[b];
+    k.ap[b] = fmaf(k.c, in[b] - k.ap[b], k.prev[b]);
+    k.prev[b] = in[b];
+  }
+  if (GAINS) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        if (kAdj)
+          k.sG[a][b] = fmaf(q[a], k.ap[b], k.sG[a][b]);
+        else
+          k.dG[a][b] = k.dG[a][b] + k.ap[b] * q[a];
+      }
+  }
+  if (!COEFS) return;
+  if (kAdj) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      k.fir[b] = fmaf(-k.c, k.fir[b], in[b] - last[b]);
+      const float gl = fmaf(k.g[2][b], r[2], fmaf(k.g[1][b], r[1], k.g[0][b] * r[0]));
+      k.sC = fmaf(gl, k.fir[b], k.sC);
+    }
+    return;
+  }
+  float u[3];
+  if (MODE == kTextbook) {
+    if (on) {
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        k.fir[b] = fmaf(k.minus_fir, k.fir[b], in[b]);
+        k.iir[b] = fmaf(k.minus_iir, k.iir[b], last[b]);
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 3; ++b) u[b] = k.fir[b] - k.iir[b];
+  } else {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) u[b] = in[b] - last[b];
+  }
+  if (MODE == kTextbook || (k.valid && on)) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) k.dC = k.dC + fmaf(u[b] * k.g[a][b] * r[a], k.mse, k.dr_dd);
+  }
+}
+
 // MODE, and which of the two gradients are wanted.
 template <int MODE, bool GAINS, bool COEFS>
-__global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const SweepArgs p) {
+__global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constant__ SweepArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
   constexpr bool kAdj = MODE == kAdjoint;
+  constexpr bool kNeedQ = !kAdj && GAINS;
   const int tid = threadIdx.x;
   const int v0 = blockIdx.x * kVox;
   const int vl = tid % kVox, n = tid / kVox;
@@ -103,207 +167,187 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const SweepArgs p) {
   const int T = p.T, S = p.S;
   const int64_t idx = (int64_t)v * kOffsets + n;
   const int32_t nb = p.nbr[idx];
-  const bool valid = live && nb >= 0;
   const int d = p.delays[idx];
   const float c_own = p.coefs[idx];
-  const float c = valid ? c_own : 0.0f;
-  const float minus_fir = valid ? -c_own : 0.0f, minus_iir = -c_own;
+  Item k;
+  k.valid = live && nb >= 0;
+  k.c = k.valid ? c_own : 0.0f;
+  k.minus_fir = k.valid ? -c_own : 0.0f;
+  k.minus_iir = -c_own;
+  k.mse = p.s.mse_scaling;
 
   int dmin = p.dmin[0], dmax = p.dmin[1];
   if (dmin > dmax) dmin = dmax = 1;  // no connected pair
   if (dmin < 1) dmin = 1;
   const int nh = p.nhalo[blockIdx.x];
   const bool ring = nh >= 0 && (int64_t)dmax - dmin + 2 * kChunk <= kRows;
-  const int slot = ring ? p.hslot[(size_t)blockIdx.x * kThreads + vl * kOffsets + n] : 0;
-  const int dr = valid ? d : dmin;  // the delay that the ring row follows
+  const int dr = k.valid ? d : dmin;  // the delay that the ring row follows
 
   // delay_delta^5 (powi(5) = x * ((x*x)*(x*x)))
   const float delay = (float)d + (1.0f - c_own) / (c_own + 1.0f);
   const float dx = p.init_delays[idx] - delay;
   const float dx2 = dx * dx;
   const float dx4 = dx2 * dx2;
-  const float dr_dd = p.s.diffreg * (dx * dx4);
-  const float mse_s = p.s.mse_scaling, reg_s = p.s.reg_scaling, thr = p.s.threshold;
+  k.dr_dd = p.s.diffreg * (dx * dx4);
 
-  float g[3][3], dG[3][3], sG[3][3];
-  float ap[3] = {0.0f, 0.0f, 0.0f}, prev[3] = {0.0f, 0.0f, 0.0f};
-  float fir[3] = {0.0f, 0.0f, 0.0f}, iir[3] = {0.0f, 0.0f, 0.0f};  // adjoint: fir is the tangent z
-  float dC = 0.0f, sC = 0.0f;
+  k.dC = k.sC = 0.0f;
+#pragma unroll
+  for (int b = 0; b < 3; ++b) k.ap[b] = k.prev[b] = k.fir[b] = k.iir[b] = 0.0f;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const size_t o = (size_t)(3 * v + a) * kGainCols + 3 * n + b;
-      if (COEFS) g[a][b] = p.gains[o];
-      if (GAINS) dG[a][b] = kAdj ? 0.0f : p.dG[o];
-      sG[a][b] = 0.0f;
+      if (COEFS) k.g[a][b] = p.gains[o];
+      if (GAINS) k.dG[a][b] = kAdj ? 0.0f : p.dG[o];
+      k.sG[a][b] = 0.0f;
     }
   if (COEFS && !kAdj) {
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      fir[b] = p.fir[(size_t)v * kGainCols + 3 * n + b];
-      iir[b] = p.iir[(size_t)v * kGainCols + 3 * n + b];
+      k.fir[b] = p.fir[(size_t)v * kGainCols + 3 * n + b];
+      k.iir[b] = p.iir[(size_t)v * kGainCols + 3 * n + b];
     }
-    dC = p.dC[idx];
+    k.dC = p.dC[idx];
   }
 
-  // staging: this thread's halo words (column of X, offset in a ring row) and its own-row words
-  int col[kCols], dst[kCols];
+  // staging: this thread's halo words (column of X, byte offset in a ring row) and its word of the own rows
+  int col[kCols];
+  uint32_t dst[kCols];
+  const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(&sm.ring[0][0]);
 #pragma unroll
   for (int i = 0; i < kCols; ++i) {
     const int w = tid + i * kThreads, s = w / 3, b = w - 3 * s;
     const bool ok = ring && s < nh;
     const size_t e = (size_t)blockIdx.x * kSlots + (ok ? s : 0);
     col[i] = ok ? 3 * p.halo[e] + b : -1;
-    dst[i] = 4 * p.hpos[e] + b;
+    dst[i] = ring0 + 4u * (4u * p.hpos[e] + b);
   }
-  const int nv = min(kVox, p.V - v0);
-  auto stage = [&](int t0) {
-    const int buf = (t0 / kChunk) & 1;
-    const int tn = min(kChunk, T - t0);
-    if (ring) {
-      const int lo = t0 == 0 ? -dmax : t0 - dmin, hi = t0 + tn - 1 - dmin;
-      for (int r = lo; r <= hi; ++r) {
-        float* to = reinterpret_cast<float*>(sm.ring[r & (kRows - 1)]);
-        const float* from = p.X + (int64_t)r * S;
+  auto copy_row = [&](int r) {  // row r >= 0
+    const uint32_t at = (uint32_t)(r & (kRows - 1)) * (kSlots * 16);
+    const float* from = p.X + (size_t)r * S;
 #pragma unroll
-        for (int i = 0; i < kCols; ++i) {
-          if (col[i] < 0) continue;
-          if (r < 0)
-            to[dst[i]] = 0.0f;
-          else
-            cp_async4(to + dst[i], from + col[i]);
-        }
-      }
+    for (int i = 0; i < kCols; ++i)
+      if (col[i] >= 0) cp_async4(dst[i] + at, from + col[i]);
+  };
+  auto stage_history = [&](int t0) {  // rows that the chunk at t0 adds
+    if (!ring || t0 >= T) return;
+    const int hi = min(t0 + kChunk, T) - dmin;
+    int lo = t0 == 0 ? -dmax : t0 - dmin;
+    for (; lo < min(0, hi); ++lo)
+#pragma unroll
+      for (int i = 0; i < kCols; ++i)
+        if (col[i] >= 0)
+          *reinterpret_cast<float*>(smem_raw + (dst[i] - ring0) + (size_t)(lo & (kRows - 1)) * (kSlots * 16)) = 0.0f;
+    if (hi - lo == kChunk) {
+#pragma unroll
+      for (int j = 0; j < kChunk; ++j) copy_row(lo + j);
+    } else {
+      for (; lo < hi; ++lo) copy_row(lo);
     }
-    // the voxels' own rows: 3 nv words per step
-    for (int e = tid; e < tn * 3 * kVox; e += kThreads) {
-      const int s = e / (3 * kVox), w = e - s * (3 * kVox);
-      if (w >= 3 * nv) continue;
-      const size_t o = (size_t)(t0 + s) * S + 3 * v0 + w;
-      cp_async4(reinterpret_cast<float*>(&sm.row[buf][s][w / 3]) + w % 3, p.rows + o);
-      if (!kAdj) cp_async4(reinterpret_cast<float*>(&sm.x[buf][s][w / 3]) + w % 3, p.X + o);
+  };
+  const int own_s = tid / (3 * kVox), own_w = tid % (3 * kVox);  // 192 words per chunk, one per thread
+  const bool own = tid < kChunk * 3 * kVox && own_w < 3 * min(kVox, p.V - v0);
+  const uint32_t own_dst = 4u * (uint32_t)(4 * (own_s * kVox + own_w / 3) + own_w % 3);
+  const uint32_t x0 = (uint32_t)__cvta_generic_to_shared(&sm.x[0][0][0]);
+  const uint32_t row0 = (uint32_t)__cvta_generic_to_shared(&sm.row[0][0][0]);
+  constexpr uint32_t kOwnBytes = sizeof(sm.x[0]);
+  auto stage_own = [&](int t0, int buf) {
+    if (own && t0 + own_s < T) {
+      const size_t o = (size_t)(t0 + own_s) * S + 3 * v0 + own_w;
+      cp_async4(row0 + buf * kOwnBytes + own_dst, p.rows + o);
+      if (kNeedQ) cp_async4(x0 + buf * kOwnBytes + own_dst, p.X + o);
     }
-    cp_async_commit();
+  };
+  const float reg_s = p.s.reg_scaling, thr = p.s.threshold;
+  auto factors = [&](int buf, int to) {  // 64 threads: one (step, voxel) each
+    if (!kNeedQ || tid >= kChunk * kVox) return;
+    const int s = tid / kVox, w = tid % kVox;
+    const float4 x4 = sm.x[buf][s][w], m4 = sm.row[buf][s][w];
+    const float x[3] = {x4.x, x4.y, x4.z}, m[3] = {m4.x, m4.y, m4.z};
+    const float sum = fabsf(x[0]) + fabsf(x[1]) + fabsf(x[2]);
+    const bool over = sum > thr;
+    const float f = sum - thr;
+    float q[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float mreg = over ? f * copysignf(1.0f, x[a]) : 0.0f;
+      q[a] = fmaf(m[a], k.mse, mreg * reg_s);
+    }
+    sm.q[to][s][w] = make_float4(q[0], q[1], q[2], 0.0f);
   };
 
   // slots no halo voxel owns (the zero slot among them) stay zero; so do the rows of voxels beyond V
-  for (int e = tid; e < kRows * kSlots; e += kThreads) (&sm.ring[0][0])[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int e = tid; e < 2 * kChunk * kVox; e += kThreads) {
-    (&sm.x[0][0][0])[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    (&sm.row[0][0][0])[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  }
+  for (int e = tid; e < (int)(sizeof(SweepSmem) / 16); e += kThreads)
+    reinterpret_cast<float4*>(smem_raw)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   __syncthreads();
 
-  stage(0);
+  // Pipeline per chunk: the history arrives one chunk ahead, the voxels' own rows two, and their factors are
+  // formed one ahead, so that one barrier per chunk is enough.
+  stage_own(0, 0);
+  stage_history(0);
+  cp_async_commit();
+  stage_own(kChunk, 1);
+  cp_async_commit();
+  cp_async_wait<1>();
+  __syncthreads();
+  factors(0, 0);
+  const uint32_t slot = ring0 + 16u * (ring ? (uint32_t)p.hslot[(size_t)blockIdx.x * kThreads + vl * kOffsets + n] : 0u);
+  int buf = 0;  // t0 / kChunk mod 3
   for (int t0 = 0; t0 < T; t0 += kChunk) {
-    const int tn = min(kChunk, T - t0);
-    const int buf = (t0 / kChunk) & 1;
-    // the next chunk's rows overwrite ring rows older than t0 - dmax (kRows >= spread + 2 chunks) and
-    // the buffer that the previous chunk read (the barrier at its end)
-    if (t0 + kChunk < T) {
-      stage(t0 + kChunk);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    cp_async_wait<0>();
+    // this chunk's history, factors and the next chunk's own rows are there for all; the previous chunk's
+    // buffers and the ring rows older than t0 - dmax are free (kRows >= spread + 2 chunks)
     __syncthreads();
-    if (!kAdj && GAINS) {
-      if (tid < tn * kVox) {
-        const int s = tid / kVox, w = tid % kVox;
-        const float4 x4 = sm.x[buf][s][w], m4 = sm.row[buf][s][w];
-        const float x[3] = {x4.x, x4.y, x4.z}, m[3] = {m4.x, m4.y, m4.z};
-        const float sum = fabsf(x[0]) + fabsf(x[1]) + fabsf(x[2]);
-        const bool over = sum > thr;
-        const float f = sum - thr;
-        float q[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float mreg = over ? f * copysignf(1.0f, x[a]) : 0.0f;
-          q[a] = fmaf(m[a], mse_s, mreg * reg_s);
-        }
-        sm.q[s][w] = make_float4(q[0], q[1], q[2], 0.0f);
-      }
-      __syncthreads();
-    }
-    auto step = [&](int s, bool on) {  // on: t >= d
-      const int t = t0 + s;
-      float in[3];
-      if (ring) {
-        const float4 h = sm.ring[(t - dr) & (kRows - 1)][slot];
-        in[0] = h.x;
-        in[1] = h.y;
-        in[2] = h.z;
-      } else {
-#pragma unroll
-        for (int b = 0; b < 3; ++b) in[b] = (valid && t >= d) ? __ldg(p.X + (int64_t)(t - d) * S + 3 * nb + b) : 0.0f;
-      }
-      float last[3];
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        last[b] = ap[b];
-        ap[b] = fmaf(c, in[b] - ap[b], prev[b]);
-        prev[b] = in[b];
-      }
-      const float4 r4 = sm.row[buf][s][vl];
+    const int next = buf == 2 ? 0 : buf + 1, after = next == 2 ? 0 : next + 1;
+    stage_history(t0 + kChunk);
+    stage_own(t0 + 2 * kChunk, after);
+    cp_async_commit();
+    if (t0 + kChunk < T) factors(next, ((t0 / kChunk) + 1) & 1);
+    const float4* rows = &sm.row[buf][0][vl];
+    const float4* facs = &sm.q[(t0 / kChunk) & 1][0][vl];
+    const int tn = min(kChunk, T - t0);
+    auto one = [&](int s, const float (&in)[3], bool on) {
+      const float4 r4 = rows[s * kVox];
       const float r[3] = {r4.x, r4.y, r4.z};
-      if (GAINS) {
-        float q[3] = {r[0], r[1], r[2]};
-        if (!kAdj) {
-          const float4 q4 = sm.q[s][vl];
-          q[0] = q4.x;
-          q[1] = q4.y;
-          q[2] = q4.z;
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            if (kAdj)
-              sG[a][b] = fmaf(q[a], ap[b], sG[a][b]);
-            else
-              dG[a][b] = dG[a][b] + ap[b] * q[a];
-          }
+      float q[3] = {r[0], r[1], r[2]};
+      if (kNeedQ) {
+        const float4 q4 = facs[s * kVox];
+        q[0] = q4.x;
+        q[1] = q4.y;
+        q[2] = q4.z;
       }
-      if (COEFS) {
-        if (kAdj) {
-#pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            fir[b] = fmaf(-c, fir[b], in[b] - last[b]);
-            const float gl = fmaf(g[2][b], r[2], fmaf(g[1][b], r[1], g[0][b] * r[0]));
-            sC = fmaf(gl, fir[b], sC);
-          }
-        } else {
-          float u[3];
-          if (MODE == kTextbook) {
-            if (on) {
-#pragma unroll
-              for (int b = 0; b < 3; ++b) {
-                fir[b] = fmaf(minus_fir, fir[b], in[b]);
-                iir[b] = fmaf(minus_iir, iir[b], last[b]);
-              }
-            }
-#pragma unroll
-            for (int b = 0; b < 3; ++b) u[b] = fir[b] - iir[b];
-          } else {
-#pragma unroll
-            for (int b = 0; b < 3; ++b) u[b] = in[b] - last[b];
-          }
-          if (MODE == kTextbook || (valid && on)) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-              for (int b = 0; b < 3; ++b) dC = dC + fmaf(u[b] * g[a][b] * r[a], mse_s, dr_dd);
-          }
-        }
-      }
+      sweep_step<MODE, GAINS, COEFS>(k, in, r, q, on);
     };
     // past every delay (of absent items too: their stored delay gates nothing but zeros)
-    if (tn == kChunk && t0 >= dmax && (MODE != kTextbook || valid || d <= t0)) {
-#pragma unroll 4
-      for (int s = 0; s < kChunk; ++s) step(s, true);
+    if (ring && tn == kChunk && t0 >= dmax && (MODE != kTextbook || k.valid || d <= t0)) {
+      // the chunk's ring rows are consecutive but for one wrap: an immediate offset from one of two addresses
+      const int first = (t0 - dr) & (kRows - 1);
+      const uint32_t low = slot + (uint32_t)first * (kSlots * 16), high = low - kRows * (kSlots * 16);
+#pragma unroll
+      for (int s = 0; s < kChunk; ++s) {
+        const uint32_t at = (first + s >= kRows ? high : low) + s * (kSlots * 16);
+        float in[3];
+        float pad;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(in[0]), "=f"(in[1]), "=f"(in[2]), "=f"(pad) : "r"(at));
+        one(s, in, true);
+      }
     } else {
-      for (int s = 0; s < tn; ++s) step(s, t0 + s >= d);
+      for (int s = 0; s < tn; ++s) {
+        const int t = t0 + s;
+        float in[3];
+        if (ring) {
+          const uint32_t at = slot - ring0 + (uint32_t)((t - dr) & (kRows - 1)) * (kSlots * 16);
+          const float4 h = *reinterpret_cast<const float4*>(smem_raw + at);
+          in[0] = h.x;
+          in[1] = h.y;
+          in[2] = h.z;
+        } else {
+#pragma unroll
+          for (int b = 0; b < 3; ++b) in[b] = (k.valid && t >= d) ? __ldg(p.X + (int64_t)(t - d) * S + 3 * nb + b) : 0.0f;
+        }
+        one(s, in, t >= d);
+      }
     }
     if (kAdj) {
       // chunk sums into the totals: the error of a long sum stays that of its T / 8 partial sums
@@ -312,14 +356,14 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const SweepArgs p) {
         for (int a = 0; a < 3; ++a)
 #pragma unroll
           for (int b = 0; b < 3; ++b) {
-            dG[a][b] = dG[a][b] + sG[a][b];
-            sG[a][b] = 0.0f;
+            k.dG[a][b] = k.dG[a][b] + k.sG[a][b];
+            k.sG[a][b] = 0.0f;
           }
       }
-      dC = dC + sC;
-      sC = 0.0f;
+      k.dC = k.dC + k.sC;
+      k.sC = 0.0f;
     }
-    __syncthreads();
+    buf = next;
   }
   if (!live) return;
   if (GAINS) {
@@ -329,24 +373,24 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const SweepArgs p) {
       for (int b = 0; b < 3; ++b) {
         float* o = p.dG + (size_t)(3 * v + a) * kGainCols + 3 * n + b;
         if (!kAdj)
-          *o = dG[a][b];
-        else if (valid)
-          *o = *o + dG[a][b];
+          *o = k.dG[a][b];
+        else if (k.valid)
+          *o = *o + k.dG[a][b];
       }
   }
   if (COEFS) {
     if (kAdj) {
       float count = 9.0f * (float)T;
-      if (p.simple) count = valid ? 9.0f * (float)max(0, T - d) : 0.0f;
-      const float sum = (valid ? dC : 0.0f) + count * dr_dd;
+      if (p.simple) count = k.valid ? 9.0f * (float)max(0, T - d) : 0.0f;
+      const float sum = (k.valid ? k.dC : 0.0f) + count * k.dr_dd;
       p.dC[idx] = p.dC[idx] + sum;
     } else {
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
-        p.fir[(size_t)v * kGainCols + 3 * n + b] = fir[b];
-        p.iir[(size_t)v * kGainCols + 3 * n + b] = iir[b];
+        p.fir[(size_t)v * kGainCols + 3 * n + b] = k.fir[b];
+        p.iir[(size_t)v * kGainCols + 3 * n + b] = k.iir[b];
       }
-      p.dC[idx] = dC;
+      p.dC[idx] = k.dC;
     }
   }
 }
