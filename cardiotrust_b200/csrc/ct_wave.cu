@@ -44,16 +44,16 @@
 //   * A CTA that owns one tile hands over two steps at a time where no delay is shorter (one hand-over's waits
 //     and arrivals for two steps: 1.33 -> 1.25 ms on the 20x20x20 cuboid). One that visits several tiles in
 //     turn, min(dmin, 64) steps each, hands over single steps (its short visits fill and drain the
-//     chain: 5.9 against 7.9 ms for the 64x64x48 shell, T = 1,000) and keeps the tiles'
+//     chain: 6.9 against 7.9 ms for the 64x64x48 shell, T = 1,000) and keeps the tiles'
 //     registers in packed records (60 floats per lane) between visits. Work is ordered by (phase, block of steps)
 //     in every CTA and a row depends on earlier blocks only, so the cooperative launch (all CTAs
 //     resident) cannot deadlock.
 //   * Every wait is bounded: a wait that sees neither its data nor any progress of the launch (a
 //     heartbeat counter) for 2 s records CT_ERR_TIMEOUT and the CTA leaves.
 // What bounds it: the cycle of a row through the chain of warps, the exchange and the halo's staging, once
-// per dmin steps (20x20x20 cuboid, dmin = 8: 4,700 + 6,100 clock cycles; issue slots 45 % used, DRAM 1.5 %).
-// Measured, ms before -> now: forward 2.87 -> 1.25 (20x20x20, T = 2,000), 0.56 -> 0.24 (8x8x8, T = 500), 54.6 ->
-// 27.4 (64x64x48 shell, T = 4,000); adjoint recursion 0.54 and 15 on the first and the last, where the
+// per dmin steps (20x20x20 cuboid, dmin = 8: 4,300 + 6,000 clock cycles; issue slots 45 % used, DRAM 1.5 %).
+// Measured, ms before -> now: forward 2.87 -> 1.18 (20x20x20, T = 2,000), 0.56 -> 0.23 (8x8x8, T = 500), 54.6 ->
+// 27.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 24 on the first and the last, where the
 // inbox form took 11.2 and 145 with the gradients in it.
 #include <cuda_runtime.h>
 
@@ -74,7 +74,7 @@ constexpr int kZeroSlot = kHaloSlots - 1;
 constexpr int kRingRows = 32;            // power of two
 constexpr int kHand = 2;                 // hand-over buffers between consecutive warps, power of two
 constexpr int kGroup = 2;                // steps per hand-over, where no delay is shorter
-constexpr int kBatch = 4;                // rows that the staging warp copies together when they are ready
+constexpr int kBatch = 4;                // rows that the staging warp copies together (two at first)
 constexpr int kOwn = 4;                  // steps of the last warp's global reads in flight, power of two
 constexpr int kMaxVisit = 64;            // steps per visit of a CTA that owns several tiles
 constexpr int kPerLane = kHaloSlots / (32 * kStageWarps);  // halo voxels per lane of a staging warp
@@ -305,7 +305,8 @@ __device__ __forceinline__ int copy_rows(const uint4* const (&from)[kPerLane], c
 // ring. It copies a few rows' entries with cp.async and then looks at their tags: an entry is one
 // aligned 16-byte word, written by one access, and a row whose tags are not all there is copied again. Lanes take
 // the halo in device order (runs of neighbouring entries). Two rows at a time while it waits for rows to
-// be finished, up to kBatch while it finds them ready (a visit's older rows, or a tile that lags). Loads into
+// be finished, a few more while it finds them ready (3 against 4 with one tile per CTA: 1.18 against 1.23 ms on
+// the 20x20x20 cuboid; always 2: 1.20, and 7 % slower on the shell). Loads into
 // registers were slower: their round trips to L2 do not overlap (the loads of two batches share
 // scoreboards), 2,250 cycles per two rows.
 __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L) {
@@ -350,7 +351,9 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
       }
       const int V = p.V, mask = p.xrows - 1;
       const int parts = (nh + 31) / 32;
-      int batch = kBatch, spins = 0;
+      // one tile per CTA: rows come one by one, and copying rows that are not there delays the next look
+      const int most = v.whole ? kBatch - 1 : kBatch;
+      int batch = most, spins = 0;
       unsigned long long since = 0;
       while (r < end) {
         const int n = min(batch, end - r);
@@ -366,7 +369,7 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
         } else if (!go_on(sm, L, spins, since, 63)) {
           return;
         }
-        batch = got == n ? kBatch : kBatch / 2;
+        batch = got == n ? most : 2;
       }
     } else {
       for (; pos < after; ++pos) {  // nothing to read
@@ -510,60 +513,47 @@ __device__ __forceinline__ bool compute_group(WaveSmem& sm, const WaveLaunch& L,
     read_own<ADJ>(sm, k, t + N, kGroup);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
   }
-  // the voxel's sums: from warp w - 1, plus this warp's columns, to warp w + 1. What the seven warps do between
-  // taking and passing them on is the latency of a step; everything else comes before or after.
+  // the voxel's sums: from warp w - 1, plus this warp's columns, to warp w + 1, step by step. What the seven warps
+  // do between taking and passing them on is the latency of a step; everything else comes before or after.
   const int buf = cur.group & (kHand - 1);
   const uint32_t tag = (uint32_t)cur.group + 1u;
   if (POS != kLast && cur.group >= kHand &&
       !mbar_wait(&sm.taken[w][buf], ((uint32_t)(cur.group / kHand) & 1u) ^ 1u, sm, L))
     return false;
-  float acc[N][3];
+  float y[N][3];  // last warp: the finished rows
 #pragma unroll
-  for (int s = 0; s < N; ++s) acc[s][0] = acc[s][1] = acc[s][2] = 0.0f;
-  if (POS != kFirst) {
-    const uint32_t from = smem_u32(&sm.hand[w - 1][buf][0][k.lane]);
-    const volatile uint32_t* flag = &sm.hand[w - 1][buf][N - 1][0].w;
-    int spins = 0;
-    unsigned long long since = 0;
-    for (;;) {
-      while (*flag != tag)  // one word, then the entries
-        if (!go_on(sm, L, spins, since, 1023)) return false;
-      bool ok = true;
-#pragma unroll
-      for (int s = 0; s < N; ++s) {
-        const uint4 h = lds_entry(from + 512 * s);
-        ok = ok && h.w == tag;
-        acc[s][0] = __uint_as_float(h.x);
-        acc[s][1] = __uint_as_float(h.y);
-        acc[s][2] = __uint_as_float(h.z);
+  for (int s = 0; s < N; ++s) {
+    float acc[3] = {0.0f, 0.0f, 0.0f};
+    if (POS != kFirst) {
+      const uint32_t from = smem_u32(&sm.hand[w - 1][buf][s][k.lane]);
+      const volatile uint32_t* flag = &sm.hand[w - 1][buf][s][0].w;
+      int spins = 0;
+      unsigned long long since = 0;
+      for (;;) {
+        while (*flag != tag)  // one word, then the entries
+          if (!go_on(sm, L, spins, since, 1023)) return false;
+        const uint4 h = lds_entry(from);
+        acc[0] = __uint_as_float(h.x);
+        acc[1] = __uint_as_float(h.y);
+        acc[2] = __uint_as_float(h.z);
+        if (__all_sync(0xffffffffu, h.w == tag)) break;
       }
-      if (__all_sync(0xffffffffu, ok)) break;
     }
-  }
-  if (ADJ) {
+    if (ADJ) {
 #pragma unroll
-    for (int s = 0; s < N; ++s)
+      for (int b = 0; b < 3; ++b) acc[b] = acc[b] + sum[s][b];
+    } else {
 #pragma unroll
-      for (int b = 0; b < 3; ++b) acc[s][b] = acc[s][b] + sum[s][b];
-  } else {
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
-    for (int i = 0; i < NI; ++i)
+        for (int b = 0; b < 3; ++b)
 #pragma unroll
-      for (int b = 0; b < 3; ++b)
-#pragma unroll
-        for (int s = 0; s < N; ++s)
-#pragma unroll
-          for (int a = 0; a < 3; ++a) acc[s][a] = acc[s][a] + k.g[i][a][b] * x[s][i][b];
-  }
-  if (POS != kLast) {
-#pragma unroll
-    for (int s = 0; s < N; ++s)
+          for (int a = 0; a < 3; ++a) acc[a] = acc[a] + k.g[i][a][b] * x[s][i][b];
+    }
+    if (POS != kLast) {
       sts_entry(smem_u32(&sm.hand[w][buf][s][k.lane]),
-                make_uint4(__float_as_uint(acc[s][0]), __float_as_uint(acc[s][1]), __float_as_uint(acc[s][2]), tag));
-  } else {
-    float y[N][3];
-#pragma unroll
-    for (int s = 0; s < N; ++s) {
+                make_uint4(__float_as_uint(acc[0]), __float_as_uint(acc[1]), __float_as_uint(acc[2]), tag));
+    } else {
       const float(*q)[32] = sm.own[(t + s) & (kOwn - 1)];
       if (ADJ) {
         const float xr[3] = {q[0][k.lane], q[1][k.lane], q[2][k.lane]};
@@ -572,15 +562,17 @@ __device__ __forceinline__ bool compute_group(WaveSmem& sm, const WaveLaunch& L,
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
           const float pull = f > 0.0f ? f * copysignf(1.0f, xr[b]) : 0.0f;
-          y[s][b] = k.mse * q[3 + b][k.lane] + k.reg * pull + acc[s][b];
+          y[s][b] = k.mse * q[3 + b][k.lane] + k.reg * pull + acc[b];
         }
       } else {
         const float u = q[0][k.lane];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) y[s][a] = acc[s][a] + u * k.ctrl[a];
+        for (int a = 0; a < 3; ++a) y[s][a] = acc[a] + u * k.ctrl[a];
       }
       if (k.live) st_entry(k.dst + (size_t)((t + s) & k.mask) * k.V, y[s][0], y[s][1], y[s][2], (uint32_t)(t + s) + 1u);
     }
+  }
+  if (POS == kLast) {
     if (k.live) {
 #pragma unroll
       for (int s = 0; s < N; ++s) {
