@@ -312,7 +312,7 @@ int prepare_exchange(ct_scn* s) {
   release(s, d.xch);
   d.xch = nullptr;
   d.xrows = 0;
-  int rc = alloc(s, &d.xch, want * d.V);
+  int rc = alloc(s, &d.xch, want * d.V + 8 * (int64_t)d.tiles);
   if (rc) return rc;
   d.xrows = (int)want;
   return CT_OK;
@@ -324,7 +324,7 @@ int prepare_exchange(ct_scn* s) {
 // neighbouring voxels' entries fall into different shared-memory banks. count = -1
 // where a block has more than HM - 1 source voxels; slot HM - 1 stands for an absent source.
 struct HaloTables {
-  std::vector<int32_t> halo, count;
+  std::vector<int32_t> halo, count, near;  // near: the blocks (of TV voxels) that the source voxels lie in
   std::vector<int16_t> pos, slot;
 };
 HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_t>& bank, int64_t V, int TV, int HM) {
@@ -333,6 +333,7 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
   t.halo.assign((size_t)(blocks * HM), 0);
   t.pos.assign((size_t)(blocks * HM), 0);
   t.count.assign((size_t)blocks, 0);
+  t.near.assign((size_t)(blocks * ct::kNearTiles), 0);
   t.slot.assign((size_t)(blocks * TV * kOffsets), (int16_t)(HM - 1));
   std::vector<int32_t> seen((size_t)V, -1), list;
   std::vector<int16_t> place((size_t)V, 0);
@@ -353,6 +354,17 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
     t.count[(size_t)b] = (int32_t)list.size();
     if (list.empty()) continue;
     std::sort(list.begin(), list.end());
+    int32_t* near = t.near.data() + (size_t)(b * ct::kNearTiles);
+    int nn = 0;
+    for (int32_t w : list) {
+      if (nn > 0 && near[nn - 1] == w / TV) continue;
+      if (nn == ct::kNearTiles) {
+        near[0] = -1;  // too many to follow
+        break;
+      }
+      near[nn++] = w / TV;
+    }
+    std::fill(near + nn, near + ct::kNearTiles, near[nn - 1]);
     std::fill(taken.begin(), taken.end(), 0);
     int next[8];
     for (int r = 0; r < 8; ++r) next[r] = r;
@@ -405,6 +417,7 @@ int prepare_adjoint(ct_scn* s) {
   int rc = alloc(s, &d.rhalo, (int64_t)t.halo.size());
   if (!rc) rc = alloc(s, &d.rhpos, (int64_t)t.pos.size());
   if (!rc) rc = alloc(s, &d.rhslot, (int64_t)t.slot.size());
+  if (!rc) rc = alloc(s, &d.rnear, (int64_t)t.near.size());
   if (!rc) rc = alloc(s, &d.rnhalo, (int64_t)t.count.size());
   if (!rc && !d.LX) rc = alloc(s, &d.LX, d.T * d.S);
   if (!rc) rc = alloc(s, &d.rev, V * kOffsets);
@@ -412,14 +425,15 @@ int prepare_adjoint(ct_scn* s) {
   if (!rc) rc = upload(s, d.rhalo, t.halo.data(), sizeof(int32_t) * t.halo.size());
   if (!rc) rc = upload(s, d.rhpos, t.pos.data(), sizeof(int16_t) * t.pos.size());
   if (!rc) rc = upload(s, d.rhslot, t.slot.data(), sizeof(int16_t) * t.slot.size());
+  if (!rc) rc = upload(s, d.rnear, t.near.data(), sizeof(int32_t) * t.near.size());
   if (!rc) rc = upload(s, d.rnhalo, t.count.data(), sizeof(int32_t) * t.count.size());
   if (!rc) {
     cudaError_t e = cudaStreamSynchronize(st);  // the host tables go out of scope
     if (e != cudaSuccess) rc = cuda_fail(e, "adjoint set-up");
   }
   if (rc) {
-    for (void* p : {(void*)d.rev, (void*)d.rhalo, (void*)d.rhpos, (void*)d.rhslot, (void*)d.rnhalo, (void*)d.LX}) release(s, p);
-    d.rev = d.rhalo = d.rnhalo = nullptr;
+    for (void* p : {(void*)d.rev, (void*)d.rhalo, (void*)d.rhpos, (void*)d.rhslot, (void*)d.rnear, (void*)d.rnhalo, (void*)d.LX}) release(s, p);
+    d.rev = d.rhalo = d.rnhalo = d.rnear = nullptr;
     d.rhslot = d.rhpos = nullptr;
     d.LX = nullptr;
   }
@@ -1006,6 +1020,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   ALLOC(d.halo, tiles * ct::kFwdHaloMax);
   ALLOC(d.hpos, tiles * ct::kFwdHaloMax);
   ALLOC(d.hslot, tiles * ct::kFwdTileVoxels * kOffsets);
+  ALLOC(d.near, tiles * ct::kNearTiles);
   ALLOC(d.nhalo, tiles);
   ALLOC(d.shalo, sweep_blocks * ct::kSweepHaloMax);
   ALLOC(d.shpos, sweep_blocks * ct::kSweepHaloMax);
@@ -1057,6 +1072,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   r = r ? r : upload(s, d.halo, wave_halo.halo.data(), sizeof(int32_t) * wave_halo.halo.size());
   r = r ? r : upload(s, d.hpos, wave_halo.pos.data(), sizeof(int16_t) * wave_halo.pos.size());
   r = r ? r : upload(s, d.hslot, wave_halo.slot.data(), sizeof(int16_t) * wave_halo.slot.size());
+  r = r ? r : upload(s, d.near, wave_halo.near.data(), sizeof(int32_t) * wave_halo.near.size());
   r = r ? r : upload(s, d.nhalo, wave_halo.count.data(), sizeof(int32_t) * wave_halo.count.size());
   r = r ? r : upload(s, d.shalo, sweep_halo.halo.data(), sizeof(int32_t) * sweep_halo.halo.size());
   r = r ? r : upload(s, d.shpos, sweep_halo.pos.data(), sizeof(int16_t) * sweep_halo.pos.size());

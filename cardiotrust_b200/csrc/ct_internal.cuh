@@ -15,6 +15,7 @@ constexpr int kOffsets = 26;   // neighbour offsets per voxel
 constexpr int kGainCols = 78;  // 26 offsets x 3 neighbour components
 constexpr int kFwdTileVoxels = 32;  // voxels per tile of the recursions (consecutive in device order)
 constexpr int kFwdHaloMax = 192;    // halo slots of a tile; the last one stands for absent neighbours
+constexpr int kNearTiles = 64;      // tiles of a halo that its staging warp can follow
 constexpr int kSweepVoxels = 8;     // voxels per block of the gradient sweep
 constexpr int kSweepHaloMax = 96;   // halo slots of such a block
 
@@ -83,7 +84,8 @@ struct DeviceScenario {
   __nv_bfloat16* R_sl;       // [3][T][kpm] slices of the beat's residuals
   float* R_sc;               // [T][ceil(kpm/512)]
   int32_t* dmin;         // [2] smallest and largest delay of a connected (voxel, offset) pair
-  // exchange ring of the recursion kernels: [xrows, V] entries {x0, x1, x2, step + 1}
+  // exchange ring of the recursion kernels: [xrows, V] entries {x0, x1, x2, step + 1}, then the number of
+  // steps that each tile has finished, 128 bytes apart
   uint4* xch;
   int xrows;             // power of two; grows with the delays
   float4* record;        // packed registers of tiles that share a CTA, null when every tile has its own
@@ -91,6 +93,7 @@ struct DeviceScenario {
   int32_t* halo;         // [tiles, kFwdHaloMax] device voxels of the halo in order, the last one repeated
   int16_t* hpos;         // [tiles, kFwdHaloMax] their slots
   int16_t* hslot;        // [tiles, 26 * kFwdTileVoxels] slot of each item's neighbour
+  int32_t* near;         // [tiles, kNearTiles] tiles of the halo, the last one repeated
   int32_t* nhalo;        // [tiles] voxels of the halo, -1 if it is too large for the slots
   int32_t* shalo;        // [sweep blocks, kSweepHaloMax]
   int16_t* shpos;
@@ -101,6 +104,7 @@ struct DeviceScenario {
   int32_t* rhalo;        // the tiles' halo tables of that direction
   int16_t* rhpos;
   int16_t* rhslot;
+  int32_t* rnear;
   int32_t* rnhalo;
   float* LX;             // [T,S] gradient of the loss with respect to the states
   // plain form (ct_plain.cu), allocated on first use
@@ -123,6 +127,7 @@ struct WaveScn {
   const int32_t* halo;
   const int16_t* hpos;
   const int16_t* hslot;
+  const int32_t* near;
   const int32_t* nhalo;
   const float* coefs;
   const int32_t* delays;

@@ -165,6 +165,18 @@ __device__ __forceinline__ void st_entry(uint4* p, float a, float b, float c, ui
       : "memory");
 }
 
+// Steps that a tile has finished (one word per 128 bytes, behind the exchange ring).
+__device__ __forceinline__ int* progress_of(const WaveScn& p, int tile) {
+  return reinterpret_cast<int*>(p.xch + (size_t)p.xrows * p.V) + 32 * (size_t)tile;
+}
+__device__ __forceinline__ int ld_progress(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_progress(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // Limit of a wait. `since` is 0 at its first call and then what the last call returned; 0 ends the wait.
 // It lasts while the launch makes progress: the heartbeat's lowest bits are part of the value.
 __device__ __noinline__ unsigned long long may_wait(unsigned long long since, int* abort, int32_t* status,
@@ -224,6 +236,7 @@ __device__ __forceinline__ Geometry geometry(const WaveScn& p) {
 struct Visit {
   int tile, scn, v0, t0, t1;
   bool whole;  // the CTA stays with this tile for the whole beat
+  bool shared; // some CTA of the phase visits several tiles
 };
 struct Walk {
   int phase = -1, begin = 0, end = 0, tile = 0, block = 0;
@@ -247,6 +260,7 @@ __device__ __forceinline__ bool next_visit(const WaveSmem& sm, const WaveLaunch&
       }
       const WaveScn& p = scenario_of(sm, L, v.scn);
       v.whole = !w.several;
+      v.shared = w.end - w.begin > (int)gridDim.x;
       v.t0 = 0;
       v.t1 = p.T;
       if (v.whole) return true;
@@ -318,10 +332,9 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
   auto room = [&](int at) -> bool {
     return at < kRingRows || mbar_wait(&sm.empty[at & (kRingRows - 1)], row_parity(at) ^ 1u, sm, L);
   };
-  // every lane's entries of rows [from, to) are stored
+  // this lane's entries of rows [from, to) are stored
   auto publish = [&](int from, int to) {
-    __syncwarp();
-    if (lane < to - from) mbar_arrive(&sm.full[(from + lane) & (kRingRows - 1)]);
+    for (; from < to; ++from) mbar_arrive(&sm.full[from & (kRingRows - 1)]);
   };
   const uint32_t ring = smem_u32(&sm.ring[0][0]);
   while (next_visit(sm, L, walk, v)) {
@@ -351,6 +364,28 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
       }
       const int V = p.V, mask = p.xrows - 1;
       const int parts = (nh + 31) / 32;
+      const int* near = p.near + (size_t)tile * kNearTiles;
+      if (!v.whole && near[0] >= 0) {
+        // All rows of the visit belong to earlier blocks: once the tiles around have published these, the copies
+        // need no look at their tags, and each row's arrival is counted by the copies themselves.
+        const int *a = progress_of(p, near[lane]), *b = progress_of(p, near[lane + 32]);
+        int spins = 0;
+        unsigned long long since = 0;
+        while (!__all_sync(0xffffffffu, ld_progress(a) >= end && ld_progress(b) >= end))
+          if (!go_on(sm, L, spins, since, 63)) return;
+        __syncwarp();  // every lane's acquires before any lane's copies
+        for (; r < end; ++r, ++pos) {
+          if (!room(pos)) return;
+          const size_t row = (size_t)(r & mask) * V;
+          const uint32_t at = ring + (uint32_t)(pos & (kRingRows - 1)) * (kHaloSlots * 16);
+#pragma unroll
+          for (int i = 0; i < kPerLane; ++i)
+            if (i < parts) cp_async16(at + to[i], from[i] + row);
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                           smem_u32(&sm.full[pos & (kRingRows - 1)]))
+                       : "memory");
+        }
+      }
       // one tile per CTA: rows come one by one, and copying rows that are not there delays the next look
       const int most = v.whole ? kBatch - 1 : kBatch;
       int batch = most, spins = 0;
@@ -379,6 +414,7 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
     }
     pos = after;
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Counters that run through all of a warp's visits.
@@ -730,12 +766,26 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
       for (int b = 0; b < 3; ++b) k.prev[i][b] = x[0][i][b];
   }
 
-  int t = v.t0;
+  int t = v.t0, said = v.t0;
+  // last warp: the rows before t are finished, for the staging warps that ask for the progress of tiles
+  auto say = [&](bool now) {
+    if (POS != kLast || !v.shared || (!now && t - said < geo.visit)) return;
+    said = t;
+    __syncwarp();
+    if (lane == 0) st_progress(progress_of(p, tile), t);
+  };
   if (v.whole && geo.pairs)
-    for (; t + kGroup <= v.t1; t += kGroup)
+    for (; t + kGroup <= v.t1;) {
       if (!compute_group<kGroup, NI, POS, ADJ, RING>(sm, L, k, cur, w, t)) return false;
-  for (; t < v.t1; ++t)
+      t += kGroup;
+      say(false);
+    }
+  for (; t < v.t1;) {
     if (!compute_group<1, NI, POS, ADJ, RING>(sm, L, k, cur, w, t)) return false;
+    ++t;
+    say(false);
+  }
+  say(true);
   if (POS == kLast) {
     asm volatile("cp.async.wait_all;" ::: "memory");  // the next visit reuses the buffers
     if (RING && lane == 0)  // the visit's remaining rows
@@ -788,7 +838,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant
     (&sm.hand[0][0][0][0])[i] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x == 0) {
     for (int i = 0; i < kRingRows; ++i) {
-      mbar_init(&sm.full[i], kStageWarps);
+      mbar_init(&sm.full[i], 32 * kStageWarps);
       mbar_init(&sm.empty[i], 1);
     }
     for (int w = 0; w < kComputeWarps - 1; ++w)
@@ -856,6 +906,7 @@ WaveScn wave_scenario(const DeviceScenario& d, bool adjoint, const WaveScalars& 
   a.halo = adjoint ? d.rhalo : d.halo;
   a.hpos = adjoint ? d.rhpos : d.hpos;
   a.hslot = adjoint ? d.rhslot : d.hslot;
+  a.near = adjoint ? d.rnear : d.near;
   a.nhalo = adjoint ? d.rnhalo : d.nhalo;
   a.coefs = d.coefs;
   a.delays = d.delays;
@@ -887,9 +938,9 @@ cudaError_t launch_wave(const WaveLaunch& launch, bool adjoint, int grid, cudaSt
                             args, sizeof(WaveSmem), stream);
 }
 
-// Empty the exchange ring (tag 0: no step).
+// Empty the exchange ring (tag 0: no step) and the tiles' progress.
 cudaError_t clear_exchange(DeviceScenario& d, cudaStream_t stream) {
-  return cudaMemsetAsync(d.xch, 0, sizeof(uint4) * (size_t)d.xrows * d.V, stream);
+  return cudaMemsetAsync(d.xch, 0, sizeof(uint4) * ((size_t)d.xrows * d.V + 8 * (size_t)d.tiles), stream);
 }
 
 namespace {
