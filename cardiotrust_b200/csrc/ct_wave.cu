@@ -41,19 +41,21 @@
 //     (2 y + z) mod 8: the eight lanes of a quarter warp are 4 x 2 neighbouring (y, z), so their 16-byte
 //     reads fall into eight different bank groups whatever the offset. Where the spread of delays does
 //     not fit the ring, or a halo is too large, the compute warps poll the exchange ring themselves.
-//   * A CTA that owns one tile hands over two steps at a time where no delay is shorter (one hand-over's waits
-//     and arrivals for two steps: 1.33 -> 1.25 ms on the 20x20x20 cuboid). One that visits several tiles in
-//     turn, min(dmin, 64) steps each, hands over single steps (its short visits fill and drain the
-//     chain: 6.9 against 7.9 ms for the 64x64x48 shell, T = 1,000) and keeps the tiles'
-//     registers in packed records (60 floats per lane) between visits. Work is ordered by (phase, block of steps)
-//     in every CTA and a row depends on earlier blocks only, so the cooperative launch (all CTAs
+//   * Two steps are handed over together where no delay is shorter (one set of waits and arrivals for both: 1.33 ->
+//     1.25 ms on the 20x20x20 cuboid), each step's sums as soon as they are there (1.25 -> 1.18 ms with the
+//     smaller staging batches).
+//   * A CTA that visits several tiles in turn, min(dmin, 64) steps each, keeps their
+//     registers in packed records (60 floats per lane) between visits. All rows that a visit reads belong to
+//     earlier blocks of steps, so its staging warp waits once for the progress that the tiles around have
+//     published and starts all copies (64x64x48 shell, T = 4,000: 27.4 -> 24.3 ms). Work is ordered by (phase, block
+//     of steps) in every CTA and a row depends on earlier blocks only, so the cooperative launch (all CTAs
 //     resident) cannot deadlock.
 //   * Every wait is bounded: a wait that sees neither its data nor any progress of the launch (a
 //     heartbeat counter) for 2 s records CT_ERR_TIMEOUT and the CTA leaves.
 // What bounds it: the cycle of a row through the chain of warps, the exchange and the halo's staging, once
 // per dmin steps (20x20x20 cuboid, dmin = 8: 4,300 + 6,000 clock cycles; issue slots 45 % used, DRAM 1.5 %).
 // Measured, ms before -> now: forward 2.87 -> 1.18 (20x20x20, T = 2,000), 0.56 -> 0.23 (8x8x8, T = 500), 54.6 ->
-// 27.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 24 on the first and the last, where the
+// 24.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 23 on the first and the last, where the
 // inbox form took 11.2 and 145 with the gradients in it.
 #include <cuda_runtime.h>
 
@@ -774,7 +776,7 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
     __syncwarp();
     if (lane == 0) st_progress(progress_of(p, tile), t);
   };
-  if (v.whole && geo.pairs)
+  if (geo.pairs)
     for (; t + kGroup <= v.t1;) {
       if (!compute_group<kGroup, NI, POS, ADJ, RING>(sm, L, k, cur, w, t)) return false;
       t += kGroup;
@@ -824,7 +826,7 @@ __device__ __forceinline__ void compute(WaveSmem& sm, const WaveLaunch& L, int w
       if (!compute_visit<NI, POS, ADJ, true>(sm, L, p, geo, v, cur, w)) return;
     } else {
       if (!direct_visit<NI, POS, ADJ>(sm, L, p, geo, v, cur, w)) return;  // by value: nothing escapes to memory
-      cur.group += v.whole && geo.pairs ? (v.t1 - v.t0) / kGroup + (v.t1 - v.t0) % kGroup : v.t1 - v.t0;
+      cur.group += geo.pairs ? (v.t1 - v.t0) / kGroup + (v.t1 - v.t0) % kGroup : v.t1 - v.t0;
     }
   }
 }
