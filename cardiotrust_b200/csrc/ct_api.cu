@@ -947,12 +947,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   d.tiles = (int)((d.V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels);
   d.wave_grid = std::min(d.tiles, ct::wave_capacity(ctx->device));
   const int64_t tiles = d.tiles, sweep_blocks = (d.V + ct::kSweepVoxels - 1) / ct::kSweepVoxels;
-  {
-    const int64_t tiles = ((M + 63) / 64) * ((T + 63) / 64);
-    int64_t ks = (2 * ctx->num_sms + tiles - 1) / tiles;
-    ks = std::min<int64_t>(ks, std::max<int64_t>(1, S / 256));
-    d.ksplit = (int)std::max<int64_t>(1, std::min<int64_t>(ks, 64));
-  }
+  d.ksplit = ct::measure_ksplit(T, S, M, ctx->num_sms);
   d.umma = ct::umma_supported(M);
   d.spad = (S + 3) / 4 * 4;
   d.kpad = ((M + 31) / 32) * 32;

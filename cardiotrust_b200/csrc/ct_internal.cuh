@@ -175,6 +175,8 @@ cudaError_t launch_forward(DeviceScenario& d, float threshold, cudaStream_t stre
 // Back-propagation through time of one beat (needs X and MR): LX = dL/dX.
 cudaError_t launch_adjoint_states(DeviceScenario& d, const WaveScalars& s, cudaStream_t stream);
 
+// Split-K factor of the FP32 H x product.
+int measure_ksplit(int64_t T, int64_t S, int64_t M, int sms);
 // y = H[beat] x for all steps; Y[beat] = y, R = y - meas[beat], loss_mse[t].
 cudaError_t launch_measure(DeviceScenario& d, int64_t beat, bool with_residuals, cudaStream_t stream);
 // MR[t,:] = H[beat]^T R[t,:] for all steps.
