@@ -327,9 +327,11 @@ struct HaloTables {
   std::vector<int32_t> halo, count, near;  // near: the blocks (of TV voxels) that the source voxels lie in
   std::vector<int16_t> pos, slot;
 };
-HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_t>& bank, int64_t V, int TV, int HM) {
+// start: each block's first voxel and, at the end, V; empty for blocks of TV voxels.
+HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_t>& bank, int64_t V, int TV, int HM,
+                       const std::vector<int32_t>& start = {}) {
   HaloTables t;
-  const int64_t blocks = (V + TV - 1) / TV;
+  const int64_t blocks = start.empty() ? (V + TV - 1) / TV : (int64_t)start.size() - 1;
   t.halo.assign((size_t)(blocks * HM), 0);
   t.pos.assign((size_t)(blocks * HM), 0);
   t.count.assign((size_t)blocks, 0);
@@ -339,7 +341,8 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
   std::vector<int16_t> place((size_t)V, 0);
   std::vector<char> taken((size_t)HM);
   for (int64_t b = 0; b < blocks; ++b) {
-    const int64_t u0 = b * TV, u1 = std::min<int64_t>(V, u0 + TV);
+    const int64_t u0 = start.empty() ? b * TV : start[(size_t)b];
+    const int64_t u1 = start.empty() ? std::min<int64_t>(V, u0 + TV) : start[(size_t)b + 1];
     list.clear();
     for (int64_t i = u0 * kOffsets; i < u1 * kOffsets; ++i) {
       const int32_t w = src[(size_t)i];
@@ -391,9 +394,41 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
       t.pos[(size_t)(b * HM + i)] = place[(size_t)w];
     }
     for (int64_t i = u0 * kOffsets; i < u1 * kOffsets; ++i)
-      if (src[(size_t)i] >= 0) t.slot[(size_t)i] = place[(size_t)src[(size_t)i]];
+      if (src[(size_t)i] >= 0) t.slot[(size_t)(b * TV * kOffsets + i - u0 * kOffsets)] = place[(size_t)src[(size_t)i]];
   }
   return t;
+}
+
+// Consecutive voxels in blocks of at most TV, a block ending early where its halo would pass HM - 1 voxels. (Uncut, one block
+// of 809 with 96 halo voxels, which gathered its history from global memory, took as long as all the others: 1.42 ms
+// instead of 0.95 per beat on 6,468 voxels, T = 1,500.)
+std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int TV, int HM) {
+  std::vector<int32_t> start{0}, seen((size_t)V, -1);
+  int halo = 0;
+  for (int64_t u = 0; u < V; ++u) {
+    const int32_t b = (int32_t)start.size() - 1;
+    int more = 0;
+    for (int n = 0; n < kOffsets; ++n) {
+      const int32_t w = src[(size_t)(u * kOffsets + n)];
+      if (w >= 0 && seen[(size_t)w] != b) {
+        seen[(size_t)w] = b;
+        ++more;
+      }
+    }
+    halo += more;
+    if (u == start.back() || (u - start.back() < TV && halo <= HM - 1)) continue;
+    start.push_back((int32_t)u);  // u opens the next block
+    halo = 0;
+    for (int n = 0; n < kOffsets; ++n) {
+      const int32_t w = src[(size_t)(u * kOffsets + n)];
+      if (w >= 0 && seen[(size_t)w] != b + 1) {
+        seen[(size_t)w] = b + 1;
+        ++halo;
+      }
+    }
+  }
+  start.push_back((int32_t)V);
+  return start;
 }
 
 // Adjoint-mode tables and buffers, allocated on first use.
@@ -946,7 +981,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   d.NB = desc->num_batch_slots;
   d.tiles = (int)((d.V + ct::kFwdTileVoxels - 1) / ct::kFwdTileVoxels);
   d.wave_grid = std::min(d.tiles, ct::wave_capacity(ctx->device));
-  const int64_t tiles = d.tiles, sweep_blocks = (d.V + ct::kSweepVoxels - 1) / ct::kSweepVoxels;
+  const int64_t tiles = d.tiles;
   d.ksplit = ct::measure_ksplit(T, S, M, ctx->num_sms);
   d.umma = ct::umma_supported(M);
   d.spad = (S + 3) / 4 * 4;
@@ -1017,10 +1052,6 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   ALLOC(d.hslot, tiles * ct::kFwdTileVoxels * kOffsets);
   ALLOC(d.near, tiles * ct::kNearTiles);
   ALLOC(d.nhalo, tiles);
-  ALLOC(d.shalo, sweep_blocks * ct::kSweepHaloMax);
-  ALLOC(d.shpos, sweep_blocks * ct::kSweepHaloMax);
-  ALLOC(d.shslot, sweep_blocks * ct::kSweepVoxels * kOffsets);
-  ALLOC(d.snhalo, sweep_blocks);
   if (d.tiles > d.wave_grid) {
     unsigned char* rec = nullptr;
     ALLOC(rec, tiles * (int64_t)ct::wave_record_bytes());
@@ -1056,7 +1087,14 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
       if (std::find(row, row + kOffsets, (int32_t)u) == row + kOffsets) s->symmetric = false;
     }
   const HaloTables wave_halo = build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
-  const HaloTables sweep_halo = build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax);
+  const std::vector<int32_t> sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax);
+  const HaloTables sweep_halo = build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax, sweep_start);
+  d.sweep_blocks = (int)sweep_start.size() - 1;
+  r = r ? r : alloc(s, &d.sstart, (int64_t)sweep_start.size());
+  r = r ? r : alloc(s, &d.shalo, (int64_t)sweep_halo.halo.size());
+  r = r ? r : alloc(s, &d.shpos, (int64_t)sweep_halo.pos.size());
+  r = r ? r : alloc(s, &d.shslot, (int64_t)sweep_halo.slot.size());
+  r = r ? r : alloc(s, &d.snhalo, (int64_t)sweep_halo.count.size());
   r = r ? r : upload(s, d.gains, h_gains.data(), sizeof(float) * S * kGainCols);
   r = r ? r : upload(s, d.nbr, h_nbr.data(), sizeof(int32_t) * V * kOffsets);
   r = r ? r : upload(s, d.coefs, h_coefs.data(), sizeof(float) * V * kOffsets);
@@ -1069,6 +1107,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   r = r ? r : upload(s, d.hslot, wave_halo.slot.data(), sizeof(int16_t) * wave_halo.slot.size());
   r = r ? r : upload(s, d.near, wave_halo.near.data(), sizeof(int32_t) * wave_halo.near.size());
   r = r ? r : upload(s, d.nhalo, wave_halo.count.data(), sizeof(int32_t) * wave_halo.count.size());
+  r = r ? r : upload(s, d.sstart, sweep_start.data(), sizeof(int32_t) * sweep_start.size());
   r = r ? r : upload(s, d.shalo, sweep_halo.halo.data(), sizeof(int32_t) * sweep_halo.halo.size());
   r = r ? r : upload(s, d.shpos, sweep_halo.pos.data(), sizeof(int16_t) * sweep_halo.pos.size());
   r = r ? r : upload(s, d.shslot, sweep_halo.slot.data(), sizeof(int16_t) * sweep_halo.slot.size());

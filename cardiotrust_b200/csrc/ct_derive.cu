@@ -24,15 +24,21 @@
 // The tangent z runs forward in time like ap itself, so neither the adjoint chain nor the
 // all-pass history has to be stored or recomputed for the coefficients.
 //
-// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 30 in adjoint mode).
-// Layout: a CTA owns 8 voxels (4 x 2 neighbours in y and z), 208 items, four CTAs per SM. The history that
+// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of about 100 and
+// 70 instructions), and the waits of a block's warps for each other at each chunk.
+// Layout: a CTA owns up to 8 consecutive voxels (4 x 2 neighbours in y and z inside a grid), 208 items. The history that
 // the items gather comes from a ring of rows in shared memory, one 16-byte entry {x0, x1, x2, -}
 // per halo voxel, staged by cp.async one chunk of 8 steps ahead; thread e works on voxel e mod 8, offset
 // e / 8, and a voxel's slot has (slot mod 8) = (2 y + z) mod 8, so a quarter warp's eight entries lie in
 // eight different bank groups. The factor fma(mr, mse/M, maxreg * reg) is the same for a voxel's 26
-// offsets and is formed once per (voxel, step). (One thread per item gathering single floats through L1
-// issued 161 instructions per item-step: 2.28 ms on the 20x20x20 cuboid, T = 2,000.) Items whose delays spread
-// too far for the ring, or whose halo is too large, read the rows from global memory.
+// offsets and is formed once per (voxel, step). Blocks end early where their halo would not fit. Where the delays spread
+// too far for the ring the items read the rows from global memory.
+// Three CTAs per SM with 80 registers and 112 slots beat four with 72 and 96, which keep some values in local
+// memory and cut more blocks. 20x20x20 cuboid, T = 2,000, textbook: 2.28 ms with one thread per item gathering single
+// floats through L1, 1.83 with four CTAs and blocks of exactly 8 voxels, 1.66 with addresses that do not
+// wrap inside a chunk, 1.56 so. Ellipsoidal shell of 47,264 voxels, T = 4,000, adjoint sweep: 15, then 7.3. (Two items
+// per thread in paired multiply-adds, 16 voxels per block: 1.77 and 7.6; a pair of FP32 operations with three
+// operands takes 2.4 cycles.)
 #include <cuda_runtime.h>
 
 #include "ct_internal.cuh"
@@ -44,6 +50,7 @@ constexpr int kVox = kSweepVoxels;
 constexpr int kThreads = kVox * kOffsets;  // 208
 constexpr int kSlots = kSweepHaloMax;      // per ring row; the last one stays zero
 constexpr int kRows = 32;   // power of two
+constexpr int kRowBytes = kSlots * 16;
 constexpr int kChunk = 8;   // steps staged together
 constexpr int kCols = (3 * (kSlots - 1) + kThreads - 1) / kThreads;  // halo words per thread and row
 
@@ -62,10 +69,12 @@ struct SweepArgs {
   float* dC;
   float* fir;
   float* iir;
+  int blocks;
+  const int32_t* start;  // [blocks + 1] first voxel of each block
   const int32_t* halo;   // [blocks, kSlots] voxels of the halo
   const int16_t* hpos;   // [blocks, kSlots] their slots
   const int16_t* hslot;  // [blocks, kVox * 26], slot of the item's neighbour, kZero if absent
-  const int32_t* nhalo;  // [blocks], -1 if the halo is too large
+  const int32_t* nhalo;  // [blocks] voxels of the halo
   const int32_t* dmin;   // [2]
   DeriveScalars s;
   int simple;
@@ -77,7 +86,8 @@ struct SweepSmem {
   float4 row[3][kChunk][kVox];  // mapped residuals or lx
   float4 q[2][kChunk][kVox];    // reference mode: fma(mr, mse/M, maxreg * reg)
 };
-static_assert(sizeof(SweepSmem) <= 233472 / 4 - 1024, "four blocks per SM");
+constexpr int kPerSm = 3;
+static_assert(sizeof(SweepSmem) <= 233472 / kPerSm - 1024, "blocks per SM");
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -154,15 +164,15 @@ __device__ __forceinline__ void sweep_step(Item& k, const float (&in)[3], const 
 
 // MODE, and which of the two gradients are wanted.
 template <int MODE, bool GAINS, bool COEFS>
-__global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constant__ SweepArgs p) {
+__global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_constant__ SweepArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
   constexpr bool kAdj = MODE == kAdjoint;
   constexpr bool kNeedQ = !kAdj && GAINS;
   const int tid = threadIdx.x;
-  const int v0 = blockIdx.x * kVox;
+  const int v0 = p.start[blockIdx.x], nv = p.start[blockIdx.x + 1] - v0;
   const int vl = tid % kVox, n = tid / kVox;
-  const bool live = v0 + vl < p.V;
+  const bool live = vl < nv;
   const int v = live ? v0 + vl : v0;
   const int T = p.T, S = p.S;
   const int64_t idx = (int64_t)v * kOffsets + n;
@@ -180,8 +190,10 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
   if (dmin > dmax) dmin = dmax = 1;  // no connected pair
   if (dmin < 1) dmin = 1;
   const int nh = p.nhalo[blockIdx.x];
-  const bool ring = nh >= 0 && (int64_t)dmax - dmin + 2 * kChunk <= kRows;
-  const int dr = k.valid ? d : dmin;  // the delay that the ring row follows
+  const bool ring = (int64_t)dmax - dmin + 2 * kChunk <= kRows;
+  const int late = k.valid ? d - dmin : 0;  // how far behind the newest row the item reads
+  // from here on t >= d holds (for absent items too: their stored delay gates nothing but zeros)
+  const int settled = MODE == kTextbook ? max(dmax, d) : dmax;
 
   // delay_delta^5 (powi(5) = x * ((x*x)*(x*x)))
   const float delay = (float)d + (1.0f - c_own) / (c_own + 1.0f);
@@ -211,7 +223,8 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
     k.dC = p.dC[idx];
   }
 
-  // staging: this thread's halo words (column of X, byte offset in a ring row) and its word of the own rows
+  // Staging: this thread's halo words (column of X, address in ring row 0) and its word of the own rows. Row r
+  // lies at ring position (r + dmin) mod kRows, so that a chunk's rows do not wrap.
   int col[kCols];
   uint32_t dst[kCols];
   const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(&sm.ring[0][0]);
@@ -223,46 +236,42 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
     col[i] = ok ? 3 * p.halo[e] + b : -1;
     dst[i] = ring0 + 4u * (4u * p.hpos[e] + b);
   }
-  auto copy_row = [&](int r) {  // row r >= 0
-    const uint32_t at = (uint32_t)(r & (kRows - 1)) * (kSlots * 16);
-    const float* from = p.X + (size_t)r * S;
+  auto stage_history = [&](int t0) {  // the rows that the chunk at t0 adds; rows before the beat stay zero
+    if (t0 >= T) return;
+    const int lo = t0 - dmin;
+    const uint32_t at = (uint32_t)(t0 & (kRows - 1)) * kRowBytes;
 #pragma unroll
-    for (int i = 0; i < kCols; ++i)
-      if (col[i] >= 0) cp_async4(dst[i] + at, from + col[i]);
-  };
-  auto stage_history = [&](int t0) {  // rows that the chunk at t0 adds
-    if (!ring || t0 >= T) return;
-    const int hi = min(t0 + kChunk, T) - dmin;
-    int lo = t0 == 0 ? -dmax : t0 - dmin;
-    for (; lo < min(0, hi); ++lo)
+    for (int i = 0; i < kCols; ++i) {
+      if (col[i] < 0) continue;
+      const float* from = p.X + (int64_t)lo * S + col[i];
+      if (lo >= 0 && t0 + kChunk <= T) {
 #pragma unroll
-      for (int i = 0; i < kCols; ++i)
-        if (col[i] >= 0)
-          *reinterpret_cast<float*>(smem_raw + (dst[i] - ring0) + (size_t)(lo & (kRows - 1)) * (kSlots * 16)) = 0.0f;
-    if (hi - lo == kChunk) {
-#pragma unroll
-      for (int j = 0; j < kChunk; ++j) copy_row(lo + j);
-    } else {
-      for (; lo < hi; ++lo) copy_row(lo);
+        for (int j = 0; j < kChunk; ++j, from += S) cp_async4(dst[i] + at + j * kRowBytes, from);
+      } else {
+        for (int j = 0; j < min(kChunk, T - t0); ++j, from += S)
+          if (lo + j >= 0) cp_async4(dst[i] + at + j * kRowBytes, from);
+      }
     }
   };
   const int own_s = tid / (3 * kVox), own_w = tid % (3 * kVox);  // 192 words per chunk, one per thread
-  const bool own = tid < kChunk * 3 * kVox && own_w < 3 * min(kVox, p.V - v0);
+  const bool own = tid < kChunk * 3 * kVox && own_w < 3 * nv;
   const uint32_t own_dst = 4u * (uint32_t)(4 * (own_s * kVox + own_w / 3) + own_w % 3);
   const uint32_t x0 = (uint32_t)__cvta_generic_to_shared(&sm.x[0][0][0]);
   const uint32_t row0 = (uint32_t)__cvta_generic_to_shared(&sm.row[0][0][0]);
   constexpr uint32_t kOwnBytes = sizeof(sm.x[0]);
+  int64_t own_at = (int64_t)own_s * S + 3 * v0 + own_w;  // moves on a chunk with every call
   auto stage_own = [&](int t0, int buf) {
-    if (own && t0 + own_s < T) {
-      const size_t o = (size_t)(t0 + own_s) * S + 3 * v0 + own_w;
-      cp_async4(row0 + buf * kOwnBytes + own_dst, p.rows + o);
-      if (kNeedQ) cp_async4(x0 + buf * kOwnBytes + own_dst, p.X + o);
-    }
+    const int64_t at = own_at;
+    own_at += (int64_t)kChunk * S;
+    if (!own || t0 + own_s >= T) return;
+    cp_async4(row0 + buf * kOwnBytes + own_dst, p.rows + at);
+    if (kNeedQ) cp_async4(x0 + buf * kOwnBytes + own_dst, p.X + at);
   };
   const float reg_s = p.s.reg_scaling, thr = p.s.threshold;
-  auto factors = [&](int buf, int to) {  // 64 threads: one (step, voxel) each
-    if (!kNeedQ || tid >= kChunk * kVox) return;
-    const int s = tid / kVox, w = tid % kVox;
+  auto factors = [&](int buf, int to) {  // one (step, voxel) each, on two warps that stage less
+    constexpr int kFirst = 128;
+    if (!kNeedQ || tid < kFirst || tid >= kFirst + kChunk * kVox) return;
+    const int s = (tid - kFirst) / kVox, w = tid % kVox;
     const float4 x4 = sm.x[buf][s][w], m4 = sm.row[buf][s][w];
     const float x[3] = {x4.x, x4.y, x4.z}, m[3] = {m4.x, m4.y, m4.z};
     const float sum = fabsf(x[0]) + fabsf(x[1]) + fabsf(x[2]);
@@ -292,7 +301,8 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
   cp_async_wait<1>();
   __syncthreads();
   factors(0, 0);
-  const uint32_t slot = ring0 + 16u * (ring ? (uint32_t)p.hslot[(size_t)blockIdx.x * kThreads + vl * kOffsets + n] : 0u);
+  // address of the neighbour in ring row 0; without a ring its column of X
+  const uint32_t slot = ring ? ring0 + 16u * (uint32_t)p.hslot[(size_t)blockIdx.x * kThreads + vl * kOffsets + n] : 3u * (uint32_t)max(nb, 0);
   int buf = 0;  // t0 / kChunk mod 3
   for (int t0 = 0; t0 < T; t0 += kChunk) {
     cp_async_wait<0>();
@@ -319,14 +329,13 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
       }
       sweep_step<MODE, GAINS, COEFS>(k, in, r, q, on);
     };
-    // past every delay (of absent items too: their stored delay gates nothing but zeros)
-    if (ring && tn == kChunk && t0 >= dmax && (MODE != kTextbook || k.valid || d <= t0)) {
-      // the chunk's ring rows are consecutive but for one wrap: an immediate offset from one of two addresses
-      const int first = (t0 - dr) & (kRows - 1);
-      const uint32_t low = slot + (uint32_t)first * (kSlots * 16), high = low - kRows * (kSlots * 16);
+    if (ring && tn == kChunk && t0 >= settled) {
+      // the chunk's rows are consecutive but for one wrap: an immediate offset from one of two addresses
+      const int first = (t0 - late) & (kRows - 1);
+      const uint32_t low = slot + (uint32_t)first * kRowBytes, high = low - kRows * kRowBytes;
 #pragma unroll
       for (int s = 0; s < kChunk; ++s) {
-        const uint32_t at = (first + s >= kRows ? high : low) + s * (kSlots * 16);
+        const uint32_t at = (first + s >= kRows ? high : low) + s * kRowBytes;
         float in[3];
         float pad;
         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(in[0]), "=f"(in[1]), "=f"(in[2]), "=f"(pad) : "r"(at));
@@ -337,14 +346,14 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
         const int t = t0 + s;
         float in[3];
         if (ring) {
-          const uint32_t at = slot - ring0 + (uint32_t)((t - dr) & (kRows - 1)) * (kSlots * 16);
+          const uint32_t at = slot - ring0 + (uint32_t)((t - late) & (kRows - 1)) * kRowBytes;
           const float4 h = *reinterpret_cast<const float4*>(smem_raw + at);
           in[0] = h.x;
           in[1] = h.y;
           in[2] = h.z;
         } else {
 #pragma unroll
-          for (int b = 0; b < 3; ++b) in[b] = (k.valid && t >= d) ? __ldg(p.X + (int64_t)(t - d) * S + 3 * nb + b) : 0.0f;
+          for (int b = 0; b < 3; ++b) in[b] = (k.valid && t >= d) ? __ldg(p.X + (int64_t)(t - d) * S + slot + b) : 0.0f;
         }
         one(s, in, t >= d);
       }
@@ -365,13 +374,14 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
     }
     buf = next;
   }
-  if (!live) return;
+  const int w = p.start[blockIdx.x] + vl;  // the voxel, read again rather than kept in a register
+  if (w >= p.start[blockIdx.x + 1]) return;
   if (GAINS) {
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
-        float* o = p.dG + (size_t)(3 * v + a) * kGainCols + 3 * n + b;
+        float* o = p.dG + (size_t)(3 * w + a) * kGainCols + 3 * n + b;
         if (!kAdj)
           *o = k.dG[a][b];
         else if (k.valid)
@@ -383,14 +393,14 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_kernel(const __grid_constan
       float count = 9.0f * (float)T;
       if (p.simple) count = k.valid ? 9.0f * (float)max(0, T - d) : 0.0f;
       const float sum = (k.valid ? k.dC : 0.0f) + count * k.dr_dd;
-      p.dC[idx] = p.dC[idx] + sum;
+      p.dC[(int64_t)w * kOffsets + n] = p.dC[(int64_t)w * kOffsets + n] + sum;
     } else {
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
-        p.fir[(size_t)v * kGainCols + 3 * n + b] = k.fir[b];
-        p.iir[(size_t)v * kGainCols + 3 * n + b] = k.iir[b];
+        p.fir[(size_t)w * kGainCols + 3 * n + b] = k.fir[b];
+        p.iir[(size_t)w * kGainCols + 3 * n + b] = k.iir[b];
       }
-      p.dC[idx] = k.dC;
+      p.dC[(int64_t)w * kOffsets + n] = k.dC;
     }
   }
 }
@@ -408,8 +418,7 @@ cudaError_t launch(const SweepArgs& a, cudaStream_t stream) {
     if (err != cudaSuccess) return err;
     done[device] = true;
   }
-  const unsigned blocks = (unsigned)((a.V + kVox - 1) / kVox);
-  sweep_kernel<MODE, GAINS, COEFS><<<blocks, kThreads, sizeof(SweepSmem), stream>>>(a);
+  sweep_kernel<MODE, GAINS, COEFS><<<(unsigned)a.blocks, kThreads, sizeof(SweepSmem), stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -436,6 +445,8 @@ SweepArgs sweep_args(DeviceScenario& d, const DeriveScalars& s) {
   a.dC = d.dC;
   a.fir = d.fir;
   a.iir = d.iir;
+  a.blocks = d.sweep_blocks;
+  a.start = d.sstart;
   a.halo = d.shalo;
   a.hpos = d.shpos;
   a.hslot = d.shslot;

@@ -16,8 +16,8 @@ constexpr int kGainCols = 78;  // 26 offsets x 3 neighbour components
 constexpr int kFwdTileVoxels = 32;  // voxels per tile of the recursions (consecutive in device order)
 constexpr int kFwdHaloMax = 192;    // halo slots of a tile; the last one stands for absent neighbours
 constexpr int kNearTiles = 64;      // tiles of a halo that its staging warp can follow
-constexpr int kSweepVoxels = 8;     // voxels per block of the gradient sweep
-constexpr int kSweepHaloMax = 96;   // halo slots of such a block
+constexpr int kSweepVoxels = 8;     // most voxels per block of the gradient sweep
+constexpr int kSweepHaloMax = 112;  // halo slots of such a block
 
 // Counts the progress of a launch, so that a bounded wait can tell a long wait from a lost one.
 struct Heartbeat {
@@ -95,6 +95,8 @@ struct DeviceScenario {
   int16_t* hslot;        // [tiles, 26 * kFwdTileVoxels] slot of each item's neighbour
   int32_t* near;         // [tiles, kNearTiles] tiles of the halo, the last one repeated
   int32_t* nhalo;        // [tiles] voxels of the halo, -1 if it is too large for the slots
+  int sweep_blocks;      // blocks of the gradient sweep: consecutive voxels whose halo fits
+  int32_t* sstart;       // [sweep blocks + 1] their first voxels
   int32_t* shalo;        // [sweep blocks, kSweepHaloMax]
   int16_t* shpos;
   int16_t* shslot;       // [sweep blocks, 26 * kSweepVoxels]

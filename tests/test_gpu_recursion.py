@@ -103,6 +103,29 @@ def test_recursions_and_sweep(alg, ctx, oracle_mod, case):
     eng.close()
 
 
+@pytest.mark.parametrize("case", ["delays_3_to_9_odd_end", "several_tiles_per_cta", "several_tiles_ring_overflow"])
+@pytest.mark.parametrize("kw", [{}, {"ap_derivative": 0}, {"freeze_gains": True}, {"freeze_delays": True}],
+                         ids=["textbook", "simple", "coefs_only", "gains_only"])
+def test_sweep_bits(alg, ctx, oracle_mod, case, kw):
+    """With and without the shared history, whole and cut blocks: bit for bit the CPU loop, given the mapped residuals."""
+    scn = _scenario(oracle_mod, case)
+    shared = dict(learning_rate=0.0, maximum_regularization_threshold=0.5, difference_regularization_strength=1e-3)
+    a = alg.Algorithm(**shared, **{"freeze_delays": False, **kw,
+                                   "ap_derivative": alg.APDerivative(kw.get("ap_derivative", 1))})
+    oa = oracle_mod.algo(**shared, **{"freeze_delays": 0, **{k: int(v) for k, v in kw.items()}})
+    eng = alg.EpochEngine.from_scenario(ctx, scn, algorithm=a)
+    eng.run_epoch(0)
+    o = oracle_mod.from_scenario(scn)
+    o.mapped_residuals_override = np.ascontiguousarray(eng.read("mapped_residuals_history")[None])
+    o.run_epoch(oa)
+    for name, want in (("grad_gains", o.d_gains), ("grad_coefs", o.d_coefs), ("coefs_fir", o.coefs_fir),
+                       ("coefs_iir", o.coefs_iir)):
+        if (name == "grad_gains" and a.freeze_gains) or (name != "grad_gains" and a.freeze_delays):
+            continue
+        np.testing.assert_array_equal(eng.read(name).view(np.uint32), want.view(np.uint32), err_msg=name)
+    eng.close()
+
+
 def test_batch_phases_match_single_runs(alg, ctx, oracle_mod):
     """A batch whose members differ in tiles per CTA, delays and beat lengths, in every arrangement of its tiles."""
     names = ["several_tiles_per_cta", "delays_2_to_5", "ring_overflow", "one_way", "several_tiles_delays_1_to_3"]
