@@ -30,6 +30,7 @@ CASES = {
     "two_steps": ((3, 3, 3), 2, 1, 1, 0.0),
     "one_way": ((6, 6, 5), 90, 4, 9, 0.3),
     "one_way_short_delays": ((5, 5, 5), 70, 1, 3, 0.5),
+    "scattered": ((6, 6, 5), 70, 3, 8, 0.2),
     "several_tiles_per_cta": ((22, 21, 22), 50, 8, 14, 0.0),
     "several_tiles_delays_1_to_3": ((22, 21, 22), 37, 1, 3, 0.0),
     "several_tiles_ring_overflow": ((22, 21, 22), 45, 2, 40, 0.1),
@@ -62,7 +63,10 @@ def _scenario(oracle_mod, case):
     def vary(p):
         connected = p.output_state_indices[::3, ::3] >= 0  # [V, 26]
         keep = connected & (draw >= cut)
-        osi = np.where(np.repeat(np.repeat(keep, 3, axis=0), 3, axis=1), p.output_state_indices, -1).astype(np.int32)
+        to = p.output_state_indices
+        if case == "scattered":  # neighbours anywhere: halos of many voxels, cut blocks
+            to = np.repeat(3 * np.repeat(where, 3, axis=0), 3, axis=1) + np.tile(np.arange(3), 26)
+        osi = np.where(np.repeat(np.repeat(keep, 3, axis=0), 3, axis=1), to, -1).astype(np.int32)
         # gains on every connection, damped so that 26 of them with short delays do not grow
         gains = np.where(osi >= 0, gain, 0.0).astype(np.float32)
         return dataclasses.replace(p, output_state_indices=osi, delays=np.where(keep, delays, p.delays).astype(np.int32),
@@ -70,6 +74,7 @@ def _scenario(oracle_mod, case):
 
     V = scn.model.coefs.shape[0]
     draw = rng.random((V, 26))
+    where = np.argsort(np.random.default_rng(1).random((V, V)), axis=1)[:, :26] if case == "scattered" else None
     delays = rng.integers(lo, hi + 1, size=(V, 26))
     delays[0, :], delays[-1, :] = lo, hi  # both ends occur
     gain = rng.normal(0.0, 0.06, size=(3 * V, 78))
@@ -95,6 +100,9 @@ def test_recursions_and_sweep(alg, ctx, oracle_mod, case):
     assert rel_err(eng.read("grad_coefs"), o32.d_coefs) < TOL_GRAD
     assert rel_err(eng.read("loss_maximum_regularization"), o32.loss_maximum_regularization) < 1e-4
 
+    if case == "scattered":  # the adjoint wants a lattice
+        eng.close()
+        return
     eng.run_epoch(0, grad_mode=alg.GradMode.Adjoint)
     o64 = oracle_mod.from_scenario(scn, dtype=np.float64)
     o64.run_epoch(oa, adjoint=True)
@@ -103,7 +111,7 @@ def test_recursions_and_sweep(alg, ctx, oracle_mod, case):
     eng.close()
 
 
-@pytest.mark.parametrize("case", ["delays_3_to_9_odd_end", "several_tiles_per_cta", "several_tiles_ring_overflow"])
+@pytest.mark.parametrize("case", ["delays_3_to_9_odd_end", "scattered", "several_tiles_per_cta", "several_tiles_ring_overflow"])
 @pytest.mark.parametrize("kw", [{}, {"ap_derivative": 0}, {"freeze_gains": True}, {"freeze_delays": True}],
                          ids=["textbook", "simple", "coefs_only", "gains_only"])
 def test_sweep_bits(alg, ctx, oracle_mod, case, kw):
