@@ -47,6 +47,8 @@ struct DeviceScenario {
   float* ap_last;        // [V,78] all-pass output of step T-2
   float* avg_delays;     // [V]
   // derivatives
+  float* derivatives;    // dG, dC, fir, iir and mreg_sum, each on a multiple of 64 floats
+  int64_t derivatives_len;
   float* dG;             // [S,78]
   float* dC;             // [V,26]
   float* fir;            // [V,78]
