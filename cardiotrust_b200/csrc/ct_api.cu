@@ -15,6 +15,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <string>
 #include <vector>
 
@@ -1071,17 +1072,24 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   std::vector<float> h_gains((size_t)(S * kGainCols)), h_coefs((size_t)(V * kOffsets)),
       h_init((size_t)(V * kOffsets)), h_ctrl((size_t)S), h_H(desc->measurement_matrix ? (size_t)(B * M * S) : 0);
   std::vector<int32_t> h_nbr((size_t)(V * kOffsets)), h_delays((size_t)(V * kOffsets));
+  for (int64_t u = 0; u < V; ++u)
+    for (int n = 0; n < kOffsets; ++n) {
+      const int32_t w = nbr[(size_t)s->perm[(size_t)u] * kOffsets + n];
+      h_nbr[(size_t)(u * kOffsets + n)] = w < 0 ? -1 : s->inv[(size_t)w];
+    }
+  // the halo tables (26 ms on 47,264 voxels) are built beside the gathering of the model (40 ms)
+  std::vector<int32_t> sweep_start;
+  auto wave_job = std::async([&] { return build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax); });
+  auto sweep_job = std::async([&] {
+    sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax);
+    return build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax, sweep_start);
+  });
   gather_rows(h_gains.data(), desc->gains, s->perm, 3, kGainCols);
   gather_rows(h_coefs.data(), desc->coefs, s->perm, 1, kOffsets);
   gather_rows(h_init.data(), desc->initial_delays, s->perm, 1, kOffsets);
   gather_rows(h_delays.data(), desc->delays, s->perm, 1, kOffsets);
   gather_state_columns(h_ctrl.data(), desc->control_matrix, s->perm, 1);
   if (desc->measurement_matrix) gather_state_columns(h_H.data(), desc->measurement_matrix, s->perm, B * M);
-  for (int64_t u = 0; u < V; ++u)
-    for (int n = 0; n < kOffsets; ++n) {
-      const int32_t w = nbr[(size_t)s->perm[(size_t)u] * kOffsets + n];
-      h_nbr[(size_t)(u * kOffsets + n)] = w < 0 ? -1 : s->inv[(size_t)w];
-    }
   s->nbr_dev = h_nbr;
   for (int64_t u = 0; u < V && s->symmetric; ++u)
     for (int n = 0; n < kOffsets; ++n) {
@@ -1090,9 +1098,8 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
       const int32_t* row = h_nbr.data() + (size_t)w * kOffsets;
       if (std::find(row, row + kOffsets, (int32_t)u) == row + kOffsets) s->symmetric = false;
     }
-  const HaloTables wave_halo = build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
-  const std::vector<int32_t> sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax);
-  const HaloTables sweep_halo = build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax, sweep_start);
+  const HaloTables wave_halo = wave_job.get();
+  const HaloTables sweep_halo = sweep_job.get();
   d.sweep_blocks = (int)sweep_start.size() - 1;
   r = r ? r : alloc(s, &d.sstart, (int64_t)sweep_start.size());
   r = r ? r : alloc(s, &d.shalo, (int64_t)sweep_halo.halo.size());
