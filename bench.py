@@ -523,8 +523,8 @@ def batched_section(args, alg, sc, ctx, prec, stream, flush, rank=0, world=1):
         "voxels_total_this_rank": int(sum(sizes)), "voxel_steps_per_epoch": int(vtb),
         "build_s": build_s,
         "chosen": {"form": "batched: one persistent forward and one persistent adjoint launch per beat index over "
-                           "every member's tiles, epoch replayed from a CUDA graph; adjoint gradients, checkpoint interval "
-                           "from the autotuner", "precision": f"{['fp32', 'tf32x3', 'tf32', 'bf16x6'][int(prec)]} products for every member",
+                           "every member's tiles, epoch replayed from a CUDA graph; adjoint gradients, phases of tiles "
+                           "arranged by the autotuner", "precision": f"{['fp32', 'tf32x3', 'tf32', 'bf16x6'][int(prec)]} products for every member",
                    "scenario_epochs_per_s": chosen, "voxel_steps_per_s": vtb * 1000.0 / chosen_ms,
                    "ms_per_epoch": chosen_ms, "graph_kernels": info["graph_kernels"], "uses_graph": info["uses_graph"],
                    "forward_ctas": info["forward_ctas"], "adjoint_ctas": info["adjoint_ctas"], "autotuned": tuned,
@@ -781,11 +781,10 @@ def gpu_arm(args):
     # the dominant kernel of the epoch is the forward propagation (one launch per beat)
     launches_of = max(1, prof["forward"][1] // args.steps)
     per_launch_ms = phase_ms["forward"] / launches_of
-    # the resident form runs when every 32-voxel tile fits a co-resident CTA (two per SM)
-    fwd_kernel = "forward_ring_kernel" if (V + 31) // 32 <= 2 * 148 else "forward_stream_kernel"
+    fwd_kernel = "wave_kernel"
     # bytes a launch must move through HBM in this design: the state history it writes (4 B per
     # state-step), and once per launch the gains [S,78], coefficients, delays and neighbour table
-    # [V,26], the all-pass state [V,78] read and written, control column and function
+    # [V,26], the last two all-pass states [V,78] written, control column and function
     must = 4.0 * S * T + 4.0 * 78 * S + 12.0 * 26 * V + 2 * 4.0 * 78 * V + 4.0 * S + 4.0 * T
     achieved = must / (per_launch_ms / 1000.0) / 1e9
     pc = profiled_counters(fwd_kernel, args.workload) or {}

@@ -24,8 +24,8 @@
 // The tangent z runs forward in time like ap itself, so neither the adjoint chain nor the
 // all-pass history has to be stored or recomputed for the coefficients.
 //
-// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of about 100 and
-// 70 instructions), and the waits of a block's warps for each other at each chunk.
+// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of 91 and
+// 51 instructions), and the waits of a block's warps for each other at each chunk.
 // Layout: a CTA owns up to 8 consecutive voxels (4 x 2 neighbours in y and z inside a grid), 208 items. The history that
 // the items gather comes from a ring of rows in shared memory, one 16-byte entry {x0, x1, x2, -}
 // per halo voxel, staged by cp.async one chunk of 8 steps ahead; thread e works on voxel e mod 8, offset
@@ -38,7 +38,7 @@
 // floats through L1, 1.83 with four CTAs and blocks of exactly 8 voxels, 1.66 with addresses that do not
 // wrap inside a chunk, 1.56 so. Ellipsoidal shell of 47,264 voxels, T = 4,000, adjoint sweep: 15, then 7.3. (Two items
 // per thread in paired multiply-adds, 16 voxels per block: 1.77 and 7.6; a pair of FP32 operations with three
-// operands takes 2.4 cycles.)
+// operands takes 2.4 cycles. Two mbarriers instead of the CTA barrier, so that warps may be steps apart: 1.70.)
 #include <cuda_runtime.h>
 
 #include "ct_internal.cuh"

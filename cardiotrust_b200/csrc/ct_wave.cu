@@ -53,7 +53,7 @@
 //   * Every wait is bounded: a wait that sees neither its data nor any progress of the launch (a
 //     heartbeat counter) for 2 s records CT_ERR_TIMEOUT and the CTA leaves.
 // What bounds it: the cycle of a row through the chain of warps, the exchange and the halo's staging, once
-// per dmin steps (20x20x20 cuboid, dmin = 8: 4,300 + 6,000 clock cycles; issue slots 45 % used, DRAM 1.5 %).
+// per dmin steps (20x20x20 cuboid, dmin = 8: 4,300 + 6,000 clock cycles; issue slots 51 % used, DRAM 1.7 %).
 // Measured, ms before -> now: forward 2.87 -> 1.18 (20x20x20, T = 2,000), 0.56 -> 0.23 (8x8x8, T = 500), 54.6 ->
 // 24.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 23 on the first and the last, where the
 // inbox form took 11.2 and 145 with the gradients in it.
