@@ -1716,7 +1716,10 @@ namespace {
 
 int batch_alloc(ct_batch* b, void** p, size_t bytes) {
   cudaError_t err = cudaMalloc(p, bytes > 0 ? bytes : 1);
-  if (err != cudaSuccess) return cuda_fail(err, "cudaMalloc (batch)");
+  if (err != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next launch
+    return cuda_fail(err, "cudaMalloc (batch)");
+  }
   b->allocations.push_back(*p);
   return CT_OK;
 }
@@ -1977,19 +1980,24 @@ int batch_prepare(ct_batch* b) {
   return CT_OK;
 }
 
-// Tile lists and phases per beat index. A scenario whose tiles fit the grid runs with one tile per
+// Tile lists and phases of an arrangement, per beat index. A scenario whose tiles fit the grid runs with one tile per
 // CTA, which then keeps the tile's parameters and chains in registers for the whole beat; scenarios are
 // packed into phases of at most `grid` tiles, longest beats first. A scenario with more tiles makes a phase of
 // its own in which every CTA visits k tiles in turn. Order 0: shorter scenarios fill the places that
 // such a phase leaves free. Order 1: they don't. Order 2: one phase with every tile.
-int batch_build_tiles(ct_batch* b, bool upload) {
+struct BatchTiles {
+  std::vector<std::vector<int2>> tiles;
+  std::vector<std::vector<int>> phases;
+  size_t shared = 0;  // tiles of phases with several tiles per CTA; these phases come first
+};
+BatchTiles arrange_tiles(const ct_batch* b, int tile_order) {
   const size_t n = b->scns.size();
   std::vector<size_t> order(n);
   for (size_t i = 0; i < n; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return b->scns[x]->d.T > b->scns[y]->d.T; });
-  b->beat_tiles.assign((size_t)b->nbeats_max, {});
-  b->beat_phases.assign((size_t)b->nbeats_max, {});
-  size_t shared_tiles = 0;  // tiles of phases with several tiles per CTA; these phases come first
+  BatchTiles out;
+  out.tiles.resize((size_t)b->nbeats_max);
+  out.phases.resize((size_t)b->nbeats_max);
   for (int beat = 0; beat < b->nbeats_max; ++beat) {
     struct Phase {
       int64_t room;
@@ -2001,7 +2009,7 @@ int batch_build_tiles(ct_batch* b, bool upload) {
     for (size_t i : order) {
       if (beat >= b->scns[i]->d.B) continue;
       const int64_t nt = b->ntiles[i];
-      if (b->tile_order == 2) {
+      if (tile_order == 2) {
         if (large.empty()) large.push_back({0, {}});
         large[0].members.push_back(i);
       } else if (nt > G) {
@@ -2013,7 +2021,7 @@ int batch_build_tiles(ct_batch* b, bool upload) {
     for (size_t i : rest) {
       const int64_t nt = b->ntiles[i];
       Phase* at = nullptr;
-      if (b->tile_order == 0)
+      if (tile_order == 0)
         for (Phase& ph : large)
           if (!at && ph.room >= nt && b->scns[ph.members[0]]->d.T >= b->scns[i]->d.T) at = &ph;
       for (Phase& ph : small)
@@ -2025,41 +2033,62 @@ int batch_build_tiles(ct_batch* b, bool upload) {
       at->members.push_back(i);
       at->room -= nt;
     }
-    std::vector<int2>& tl = b->beat_tiles[(size_t)beat];
-    std::vector<int>& pb = b->beat_phases[(size_t)beat];
+    std::vector<int2>& tl = out.tiles[(size_t)beat];
+    std::vector<int>& pb = out.phases[(size_t)beat];
     for (const std::vector<Phase>* group : {&large, &small})
       for (const Phase& ph : *group) {
         pb.push_back((int)tl.size());
         for (size_t i : ph.members)
           for (int t = 0; t < b->ntiles[i]; ++t) tl.push_back(make_int2((int)i, t * ct::kFwdTileVoxels));
-        if ((int64_t)tl.size() - pb.back() > G) shared_tiles = std::max(shared_tiles, tl.size());
+        if ((int64_t)tl.size() - pb.back() > G) out.shared = std::max(out.shared, tl.size());
       }
     pb.push_back((int)tl.size());
   }
-  if (upload) {
-    CT_CUDA(cudaStreamSynchronize(b->ctx->stream), "batch tiles");
-    if (shared_tiles > b->record_tiles) {
+  return out;
+}
+
+void drop_graph(ct_batch* b) {
+  if (b->exec) cudaGraphExecDestroy(b->exec);
+  if (b->graph) cudaGraphDestroy(b->graph);
+  b->exec = nullptr;
+  b->graph = nullptr;
+  b->captured_rows.clear();
+}
+
+// Makes `tile_order` the batch's arrangement. What the new one needs is allocated before anything of the old one goes, so
+// a refused allocation leaves the batch as it was; the graph, which names the old record and lists, goes before they
+// change. fit: give back what is more than the arrangement needs.
+int batch_set_order(ct_batch* b, int tile_order, bool fit) {
+  BatchTiles t = arrange_tiles(b, tile_order);
+  CT_CUDA(cudaStreamSynchronize(b->ctx->stream), "batch tiles");
+  if (t.shared > b->record_tiles || (fit && t.shared < b->record_tiles)) {
+    void* p = nullptr;
+    if (t.shared > 0) {
+      int rc = batch_alloc(b, &p, t.shared * ct::wave_record_bytes());
+      if (rc && t.shared > b->record_tiles) return rc;
+    }
+    if (p || t.shared == 0) {
+      drop_graph(b);
       if (b->record) {
         cudaFree(b->record);
         b->allocations.erase(std::remove(b->allocations.begin(), b->allocations.end(), (void*)b->record),
                              b->allocations.end());
       }
-      b->record = nullptr;
-      b->record_tiles = 0;
-      void* p = nullptr;
-      int rc = batch_alloc(b, &p, shared_tiles * ct::wave_record_bytes());
-      if (rc) return rc;
       b->record = static_cast<float4*>(p);
-      b->record_tiles = shared_tiles;
+      b->record_tiles = t.shared;
     }
-    for (int beat = 0; beat < b->nbeats_max; ++beat) {
-      const auto& tl = b->beat_tiles[(size_t)beat];
-      const auto& pb = b->beat_phases[(size_t)beat];
-      CT_CUDA(cudaMemcpy(b->beat_tiles_dev[(size_t)beat], tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice),
-              "batch tiles");
-      CT_CUDA(cudaMemcpy(b->beat_phases_dev[(size_t)beat], pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice),
-              "batch phases");
-    }
+  }
+  drop_graph(b);
+  b->tile_order = tile_order;
+  b->beat_tiles.swap(t.tiles);
+  b->beat_phases.swap(t.phases);
+  for (int beat = 0; beat < b->nbeats_max; ++beat) {
+    const auto& tl = b->beat_tiles[(size_t)beat];
+    const auto& pb = b->beat_phases[(size_t)beat];
+    CT_CUDA(cudaMemcpy(b->beat_tiles_dev[(size_t)beat], tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice),
+            "batch tiles");
+    CT_CUDA(cudaMemcpy(b->beat_phases_dev[(size_t)beat], pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice),
+            "batch phases");
   }
   return CT_OK;
 }
@@ -2112,7 +2141,7 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
     b->nbeats_max = std::max<int>(b->nbeats_max, (int)d.B);
   }
   b->grid = ct::wave_capacity(ctx->device);
-  batch_build_tiles(b, false);
+  const BatchTiles first = arrange_tiles(b, b->tile_order);  // every order lists the same tiles
   void* p = nullptr;
   rc = batch_alloc(b, &p, sizeof(ct::WaveScn) * n);
   b->fwd_dev = static_cast<ct::WaveScn*>(p);
@@ -2130,13 +2159,12 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
     b->parts.push_back(static_cast<float*>(p));
   }
   for (int beat = 0; beat < b->nbeats_max && !rc; ++beat) {
-    const auto& tl = b->beat_tiles[(size_t)beat];
-    rc = batch_alloc(b, &p, sizeof(int2) * tl.size());
+    rc = batch_alloc(b, &p, sizeof(int2) * first.tiles[(size_t)beat].size());
     b->beat_tiles_dev.push_back(static_cast<int2*>(p));
     if (!rc) rc = batch_alloc(b, &p, sizeof(int) * (n + 2));  // phases never outnumber the members
     b->beat_phases_dev.push_back(static_cast<int*>(p));
   }
-  if (!rc) rc = batch_build_tiles(b, true);
+  if (!rc) rc = batch_set_order(b, b->tile_order, false);
   const int nside = (int)std::min<size_t>(n, 8);
   for (int i = 0; i < nside && !rc; ++i) {
     cudaStream_t s = nullptr;
@@ -2218,16 +2246,8 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
   CT_CUDA(cudaEventCreate(&e1), "cudaEventCreate");
   const bool was_profiling = b->profiling;
   b->profiling = false;
-  auto trial = [&](int order, double* ms) -> int {
-    b->tile_order = order;
-    int rc = batch_build_tiles(b, true);
-    if (rc) return rc;
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
-    b->captured_rows.clear();
-    rc = batch_prepare(b);  // capture
+  auto trial = [&](double* ms) -> int {
+    int rc = batch_prepare(b);  // capture
     if (rc) return rc;
     CT_CUDA(cudaStreamSynchronize(st), "autotune");
     CT_CUDA(cudaEventRecord(e0, st), "cudaEventRecord");
@@ -2241,7 +2261,8 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
     *ms = t;
     return CT_OK;
   };
-  int best_o = b->tile_order;
+  const int before = b->tile_order;
+  int best_o = before;
   double best = 1e300;
   int rc = CT_OK;
   // adjoint mode trains five trial epochs, reference mode three; the first order is timed again while
@@ -2249,21 +2270,24 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
   for (int trial_no = b->grad_mode == CT_GRAD_ADJOINT ? -2 : 0; trial_no <= 2 && !rc; ++trial_no) {
     const int o = std::max(0, trial_no);
     double ms = 0.0;
-    rc = trial(o, &ms);
+    rc = batch_set_order(b, o, false);
+    if (rc == CT_ERR_OUT_OF_MEMORY) {  // no room for this arrangement's records: the others are timed
+      rc = CT_OK;
+      continue;
+    }
+    if (!rc) rc = trial(&ms);
     if (!rc && ms < best) best = ms, best_o = o;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   b->profiling = was_profiling;
+  if (rc) {
+    const std::string what = g_last_error;
+    batch_set_order(b, before, true);
+    return fail(rc, "%s", what.c_str());
+  }
+  rc = batch_set_order(b, best_o, true);
   if (rc) return rc;
-  b->tile_order = best_o;
-  rc = batch_build_tiles(b, true);
-  if (rc) return rc;
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  b->exec = nullptr;
-  b->graph = nullptr;
-  b->captured_rows.clear();
   if (ckpt_k) *ckpt_k = kReportedCkptSteps;
   if (tile_order) *tile_order = best_o;
   if (best_ms) *best_ms = best;
@@ -2526,10 +2550,7 @@ int ct_batch_run_model_based(ct_batch* batch, const ct_run_config* cfg, int64_t*
       for (size_t i : still) scns.push_back(batch->scns[i]);
       ct_batch* nb = nullptr;
       rc = ct_batch_create(batch->ctx, scns.data(), (int64_t)scns.size(), batch->grad_mode, batch->precision, &nb);
-      if (!rc) {
-        nb->tile_order = batch->tile_order;
-        rc = batch_build_tiles(nb, true);
-      }
+      if (!rc) rc = batch_set_order(nb, batch->tile_order, true);
       if (sub) ct_batch_destroy(sub);
       sub = nb;
       cur = nb;

@@ -1,0 +1,128 @@
+"""The host side of the library without a GPU: ct_api.cu compiled as C++ against tests/native/host_device.cpp, where device
+memory is host memory with known blocks and a launch checks that what it was given is there. Allocations are
+made to fail on the host; what a later launch is then given must still be live and large enough."""
+
+import ctypes
+import pathlib
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = pathlib.Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    from cardiotrust_b200 import _lib
+
+    so = tmp_path_factory.mktemp("host_device") / "libhost_device.so"
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
+                           "-x", "c++", str(ROOT / "cardiotrust_b200/csrc/ct_api.cu"),
+                           str(ROOT / "tests/native/host_device.cpp"), "-o", str(so), "-lpthread"])
+    return _lib.load(so)
+
+
+class _Host:
+    """The compiled library in the place of the real one, and its controls."""
+
+    def __init__(self, lib):
+        self.lib = lib
+        lib.host_device_live.restype = ctypes.c_size_t
+
+    def fail_from(self, nbytes):
+        self.lib.host_device_fail_from(ctypes.c_size_t(nbytes))
+
+    def live(self):
+        return int(self.lib.host_device_live())
+
+    def times(self, *ms):
+        self.lib.host_device_times((ctypes.c_float * len(ms))(*ms), len(ms))
+
+    def report(self):
+        buf = ctypes.create_string_buffer(4096)
+        self.lib.host_device_report(buf, len(buf))
+        return buf.value.decode()
+
+
+NEVER = (1 << 64) - 1
+
+
+@pytest.fixture
+def host(library, monkeypatch):
+    from cardiotrust_b200 import _lib
+
+    monkeypatch.setattr(_lib, "_LIB", library)
+    h = _Host(library)
+    h.fail_from(NEVER)
+    h.times()
+    h.report()
+    yield h
+    h.fail_from(NEVER)
+
+
+def _engine(ctx, shape, steps, **kw):
+    from cardiotrust_b200 import algorithm as alg
+    from cardiotrust_b200 import scenario as sc
+
+    spec = sc.ScenarioSpec(shape=shape, num_steps=steps, num_sensors=3, patho_size=1, patho_origin=(1, 1, 1), seed=2)
+    scn = sc.build(spec)
+    scn.measurements = np.zeros((1, steps, scn.num_sensors), np.float32)
+    return alg.EpochEngine.from_scenario(ctx, scn, num_batch_slots=16, **kw)
+
+
+@pytest.fixture
+def ctx(host):
+    from cardiotrust_b200 import algorithm as alg
+
+    c = alg.Context(0)
+    yield c
+    c.close()
+
+
+def _batch(ctx, members, **kw):
+    from cardiotrust_b200 import algorithm as alg
+
+    engines = [_engine(ctx, *m) for m in members]
+    return engines, alg.EpochBatch(ctx, engines, precision=alg.Precision.Fp32, **kw)
+
+
+#: 9, 2 and 2 tiles on 4 CTAs: only the arrangement in one phase needs records for all 13
+MEMBERS = [((8, 6, 6), 90), ((4, 4, 4), 70), ((4, 4, 4), 60)]
+
+
+def test_autotune_without_room_for_one_arrangement(host, ctx):
+    """The record of the arrangement in one phase cannot be allocated: the tuner times the others, and the epochs
+    that follow use memory that is still there."""
+    engines, batch = _batch(ctx, MEMBERS)
+    batch.run_epoch()  # a graph that names the first record
+    assert host.report() == ""
+    before = host.live()
+    host.fail_from(1)
+    tuned = batch.autotune()
+    host.fail_from(NEVER)
+    assert tuned["tile_order"] in (0, 1)
+    batch.run_epoch()
+    assert host.report() == ""
+    assert host.live() == before
+    batch.close()
+
+
+def test_autotune_gives_back_the_larger_record(host, ctx):
+    engines, batch = _batch(ctx, MEMBERS)
+    before = host.live()
+    host.times(1.0, 2.0, 3.0)  # the first arrangement is the fastest, the last needed the most records
+    assert batch.autotune()["tile_order"] == 0
+    batch.run_epoch()
+    assert host.report() == ""
+    assert host.live() == before
+    batch.close()
+
+
+def test_autotune_keeps_the_record_of_its_choice(host, ctx):
+    engines, batch = _batch(ctx, MEMBERS)
+    host.times(3.0, 2.0, 1.0)
+    assert batch.autotune()["tile_order"] == 2
+    batch.run_epoch()
+    assert host.report() == ""
+    batch.close()
