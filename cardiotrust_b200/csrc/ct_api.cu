@@ -65,7 +65,7 @@ struct ct_scn {
   cudaEvent_t dmax_event = nullptr;
   int64_t updates = 0;          // updates that may roll delays, enqueued so far
   int64_t updates_at_read = -1; // `updates` when the pending read-back was enqueued (-1: none)
-  // bumped whenever the algorithm settings change (batches re-capture their epoch graph)
+  // bumped whenever the algorithm settings or the exchange ring change (batches re-capture their epoch graph)
   uint64_t config_gen = 0;
   // Device voxel order: device voxel u holds reference voxel perm[u]; inv is the inverse.
   std::vector<int32_t> perm, inv;
@@ -182,7 +182,10 @@ int alloc(ct_scn* s, T** p, int64_t count) {
   void* ptr = nullptr;
   const size_t bytes = sizeof(T) * (size_t)(count > 0 ? count : 1);
   cudaError_t err = cudaMalloc(&ptr, bytes);
-  if (err != cudaSuccess) return cuda_fail(err, "cudaMalloc");
+  if (err != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next launch
+    return cuda_fail(err, "cudaMalloc");
+  }
   s->allocations.push_back(ptr);
   *p = static_cast<T*>(ptr);
   return CT_OK;
@@ -313,6 +316,7 @@ int prepare_exchange(ct_scn* s) {
   release(s, d.xch);
   d.xch = nullptr;
   d.xrows = 0;
+  s->config_gen += 1;
   int rc = alloc(s, &d.xch, want * d.V + 8 * (int64_t)d.tiles);
   if (rc) return rc;
   d.xrows = (int)want;
@@ -1701,7 +1705,6 @@ struct ct_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool use_graph = true;
-  std::vector<int> captured_rows;
   std::vector<uint64_t> captured_gen;
   int64_t graph_kernels = 0;
   int tile_order = 0;  // tuned choice (ct_batch_autotune): how the tiles are arranged in phases
@@ -1913,10 +1916,9 @@ int batch_prepare(ct_batch* b) {
     }
     int rc = prepare_exchange(s);
     if (rc) return rc;
-    if (b->captured_rows.size() == n && b->captured_rows[i] != s->d.xrows) stale = true;
     if (b->captured_gen.size() == n && b->captured_gen[i] != s->config_gen) stale = true;
   }
-  if (!stale && b->captured_rows.size() == n) return CT_OK;
+  if (!stale && b->captured_gen.size() == n) return CT_OK;
   // descriptors
   std::vector<ct::WaveScn> fa(n), aa(n);
   const bool adjoint = b->grad_mode == CT_GRAD_ADJOINT;
@@ -1971,12 +1973,8 @@ int batch_prepare(ct_batch* b) {
       b->use_graph = false;
     }
   }
-  b->captured_rows.assign(n, 0);
   b->captured_gen.assign(n, 0);
-  for (size_t i = 0; i < n; ++i) {
-    b->captured_rows[i] = b->scns[i]->d.xrows;
-    b->captured_gen[i] = b->scns[i]->config_gen;
-  }
+  for (size_t i = 0; i < n; ++i) b->captured_gen[i] = b->scns[i]->config_gen;
   return CT_OK;
 }
 
@@ -2052,7 +2050,7 @@ void drop_graph(ct_batch* b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   b->exec = nullptr;
   b->graph = nullptr;
-  b->captured_rows.clear();
+  b->captured_gen.clear();
 }
 
 // Makes `tile_order` the batch's arrangement. What the new one needs is allocated before anything of the old one goes, so

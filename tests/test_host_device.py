@@ -126,3 +126,30 @@ def test_autotune_keeps_the_record_of_its_choice(host, ctx):
     batch.run_epoch()
     assert host.report() == ""
     batch.close()
+
+
+def _with_delays(engine, largest):
+    d = engine.read("delays")
+    d[:] = 8
+    d[0, :] = largest
+    engine.write("delays", d)
+
+
+def test_batch_after_an_exchange_ring_that_could_not_grow(host, ctx):
+    """A ring that was given back for a longer one, which then did not fit, is made again at its former length: the
+    batch's graph must not name the old one, although the lengths agree."""
+    from cardiotrust_b200._lib import CtError
+
+    engines, batch = _batch(ctx, [((4, 4, 4), 300), ((4, 4, 4), 200)])
+    _with_delays(engines[0], 12)
+    batch.run_epoch()
+    _with_delays(engines[0], 60)
+    host.fail_from(1)
+    with pytest.raises(CtError, match="made to fail"):
+        engines[0].run_epoch(0, precision=0)
+    host.fail_from(NEVER)
+    _with_delays(engines[0], 12)
+    engines[0].run_epoch(0, precision=0)
+    batch.run_epoch()
+    assert host.report() == ""
+    batch.close()
