@@ -56,7 +56,7 @@ struct ct_scn {
   std::vector<uint8_t> bank;      // (2 y + z) mod 8 of each device voxel's grid coordinates
   bool symmetric = true;          // a voxel's neighbours all have it as a neighbour
   // Upper bound of the largest delay of a connected pair: exact after creation and delay writes,
-  // +1 per update that rolls delays (roll_delays moves a delay by at most one). Sizes the
+  // +1 per update that rolls delays (roll_delays moves a delay by at most one, and none past 1,000). Sizes the
   // exchange ring without reading the device.
   int64_t dmax_bound = 1;
   // Asynchronous read-back of the device's largest delay after an update (pinned word + event):
@@ -234,7 +234,7 @@ void release(ct_scn* s, void* p) {
 // After an update that may roll delays: count it and enqueue the read-back of the largest delay.
 void note_delay_update(ct_scn* s, cudaStream_t st) {
   s->updates += 1;
-  s->dmax_bound = std::min<int64_t>(s->dmax_bound + 1, 1000);
+  if (s->dmax_bound < 1000) s->dmax_bound += 1;  // a larger delay that was written stays (roll_delays)
   if (!s->dmax_host) {
     void* p = nullptr;
     if (cudaMallocHost(&p, sizeof(int32_t)) != cudaSuccess) return;

@@ -153,3 +153,16 @@ def test_batch_after_an_exchange_ring_that_could_not_grow(host, ctx):
     batch.run_epoch()
     assert host.report() == ""
     batch.close()
+
+
+def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
+    """An update moves no delay past 1,000, but leaves a larger one that was written where it is: the ring that is
+    sized afterwards holds the rows that it reads."""
+    from cardiotrust_b200 import algorithm as alg
+
+    eng = _engine(ctx, (4, 4, 4), 4200, algorithm=alg.Algorithm(freeze_delays=False))
+    _with_delays(eng, 1500)
+    eng.run_epoch_plain(0)  # an update, before any recursion has asked for its ring
+    eng.run_epoch(0, precision=0)
+    assert host.report() == ""
+    eng.close()
