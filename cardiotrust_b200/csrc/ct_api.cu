@@ -16,7 +16,11 @@
 #include <cstdio>
 #include <cstring>
 #include <future>
+#include <memory>
+#include <new>
+#include <stdexcept>
 #include <string>
+#include <system_error>
 #include <vector>
 
 #include "ct_internal.cuh"
@@ -123,6 +127,19 @@ int cuda_fail(cudaError_t err, const char* what) {
     if (err__ != cudaSuccess) return cuda_fail(err__, what); \
   } while (0)
 
+// Entry points return a status: exceptions of the standard library end here (function-try-blocks, CT_CATCH).
+int caught(const std::exception& e) noexcept {
+  const bool memory = dynamic_cast<const std::bad_alloc*>(&e) != nullptr;
+  const int status = memory ? CT_ERR_OUT_OF_MEMORY : CT_ERR_INVALID_ARGUMENT;
+  try {
+    return fail(status, "%s: %s", memory ? "host memory" : "host error", e.what());
+  } catch (...) {
+    return status;  // no memory for the message either
+  }
+}
+#define CT_CATCH \
+  catch (const std::exception& e) { return caught(e); }
+
 // Makes `device` current for the rest of the enclosing scope and restores the caller's current
 // device when the scope ends, so that no entry point changes the calling thread's device.
 struct DeviceScope {
@@ -186,7 +203,12 @@ int alloc(ct_scn* s, T** p, int64_t count) {
     cudaGetLastError();  // reported here, not by the next launch
     return cuda_fail(err, "cudaMalloc");
   }
-  s->allocations.push_back(ptr);
+  try {
+    s->allocations.push_back(ptr);
+  } catch (...) {
+    cudaFree(ptr);
+    throw;
+  }
   *p = static_cast<T*>(ptr);
   return CT_OK;
 }
@@ -434,6 +456,16 @@ std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int 
   }
   start.push_back((int32_t)V);
   return start;
+}
+
+// Runs f on a thread of its own, or, where none can be started, when its result is asked for.
+template <typename F>
+auto beside(F f) {
+  try {
+    return std::async(std::launch::async, f);
+  } catch (const std::system_error&) {
+    return std::async(std::launch::deferred, f);
+  }
 }
 
 // Adjoint-mode tables and buffers, allocated on first use.
@@ -903,7 +935,7 @@ int ct_last_error(char* buf, size_t len) {
   return CT_OK;
 }
 
-int ct_ctx_create(int device, void* stream, ct_ctx** out) {
+int ct_ctx_create(int device, void* stream, ct_ctx** out) try {
   if (!out) return fail(CT_ERR_INVALID_ARGUMENT, "out is NULL");
   *out = nullptr;
   int count = 0;
@@ -925,7 +957,7 @@ int ct_ctx_create(int device, void* stream, ct_ctx** out) {
   }
   *out = c;
   return CT_OK;
-}
+} CT_CATCH
 
 namespace {
 void ctx_release(ct_ctx* ctx) {
@@ -936,19 +968,19 @@ void ctx_release(ct_ctx* ctx) {
 }
 }  // namespace
 
-int ct_ctx_destroy(ct_ctx* ctx) {
+int ct_ctx_destroy(ct_ctx* ctx) try {
   if (!ctx) return CT_OK;
   ctx_release(ctx);
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_ctx_stream(ct_ctx* ctx, void** stream) {
+int ct_ctx_stream(ct_ctx* ctx, void** stream) try {
   if (!ctx || !stream) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   *stream = ctx->stream;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algorithm* algo, ct_scn** out) {
+int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algorithm* algo, ct_scn** out) try {
   if (!ctx || !desc || !out) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   *out = nullptr;
   int rc = check_algo(algo);
@@ -967,7 +999,14 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   if (rc) return rc;
   CT_DEVICE_SCOPE(ctx->device);
 
-  ct_scn* s = new ct_scn;
+  struct Release {
+    void operator()(ct_scn* p) const {
+      free_scenario(p);
+      delete p;
+    }
+  };
+  std::unique_ptr<ct_scn, Release> owner(new ct_scn);  // until the scenario is handed out
+  ct_scn* s = owner.get();
   s->ctx = ctx;
   s->algo = *algo;
   s->nbr_host = nbr;
@@ -999,11 +1038,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
 #define ALLOC(ptr, n)                    \
   do {                                   \
     int r__ = alloc(s, &(ptr), (n));     \
-    if (r__) {                           \
-      free_scenario(s);                  \
-      delete s;                          \
-      return r__;                        \
-    }                                    \
+    if (r__) return r__;                 \
   } while (0)
   ALLOC(d.gains, S * kGainCols);
   ALLOC(d.nbr, V * kOffsets);
@@ -1083,8 +1118,8 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
     }
   // the halo tables (26 ms on 47,264 voxels) are built beside the gathering of the model (40 ms)
   std::vector<int32_t> sweep_start;
-  auto wave_job = std::async([&] { return build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax); });
-  auto sweep_job = std::async([&] {
+  auto wave_job = beside([&] { return build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax); });
+  auto sweep_job = beside([&] {
     sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax);
     return build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax, sweep_start);
   });
@@ -1173,17 +1208,13 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) r = cuda_fail(e, "scenario upload");
   }
-  if (r) {
-    free_scenario(s);
-    delete s;
-    return r;
-  }
+  if (r) return r;
   ctx->refs += 1;
-  *out = s;
+  *out = owner.release();
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_scenario_destroy(ct_scn* scn) {
+int ct_scenario_destroy(ct_scn* scn) try {
   if (!scn) return CT_OK;
   ct_ctx* ctx = scn->ctx;
   DeviceScope device_scope__(ctx->device);
@@ -1192,16 +1223,16 @@ int ct_scenario_destroy(ct_scn* scn) {
   delete scn;
   ctx_release(ctx);
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_scenario_dims(ct_scn* scn, int64_t* S, int64_t* M, int64_t* T, int64_t* B) {
+int ct_scenario_dims(ct_scn* scn, int64_t* S, int64_t* M, int64_t* T, int64_t* B) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   if (S) *S = scn->d.S;
   if (M) *M = scn->d.M;
   if (T) *T = scn->d.T;
   if (B) *B = scn->d.B;
   return CT_OK;
-}
+} CT_CATCH
 
 static int run_beat_plain(ct_scn* s, int64_t beat) {
   DeviceScenario& d = s->d;
@@ -1337,19 +1368,19 @@ static int run_epoch_impl(ct_scn* scn, int64_t* batch_index, const int32_t* beat
   return batch_end(scn, d.B, batch_index);
 }
 
-int ct_run_epoch(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order, int grad_mode, int precision) {
+int ct_run_epoch(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order, int grad_mode, int precision) try {
   return run_epoch_impl(scn, batch_index, beat_order, grad_mode, precision, false);
-}
+} CT_CATCH
 
-int ct_run_epoch_plain(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order) {
+int ct_run_epoch_plain(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order) try {
   return run_epoch_impl(scn, batch_index, beat_order, CT_GRAD_REFERENCE, CT_PREC_FP32, true);
-}
+} CT_CATCH
 
 // One epoch for a caller that keeps the model in host memory, as the reference's run_epoch
 // (src/core/algorithm.rs:124-129) mutates `results.model` in place: every copy, reordering kernel
 // and the epoch go onto the context stream back to back, and the call waits once at the end.
 int ct_run_epoch_host(ct_scn* scn, int64_t* batch_index, const int32_t* beat_order, int grad_mode, int precision,
-                      float* gains, float* coefs, int32_t* delays, const float* measurements, float* loss_batch) {
+                      float* gains, float* coefs, int32_t* delays, const float* measurements, float* loss_batch) try {
   if (!scn || !batch_index || !gains || !coefs || !delays) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(scn->ctx->device);
   DeviceScenario& d = scn->d;
@@ -1404,9 +1435,9 @@ int ct_run_epoch_host(ct_scn* scn, int64_t* batch_index, const int32_t* beat_ord
   if (loss_batch)
     CT_CUDA(cudaMemcpyAsync(loss_batch, d.loss_b, sizeof(float) * d.NB, cudaMemcpyDeviceToHost, st), "copy loss");
   return ct_sync(scn);
-}
+} CT_CATCH
 
-int ct_simulate(ct_scn* scn, float* measurements_out, float* states_out) {
+int ct_simulate(ct_scn* scn, float* measurements_out, float* states_out) try {
   if (!scn || !measurements_out) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(scn->ctx->device);
   DeviceScenario& d = scn->d;
@@ -1426,38 +1457,38 @@ int ct_simulate(ct_scn* scn, float* measurements_out, float* states_out) {
   if (rc) return rc;
   if (states_out) rc = copy_down_state_columns(scn, states_out, d.X, d.T);
   return rc;
-}
+} CT_CATCH
 
-int ct_set_algorithm(ct_scn* scn, const ct_algorithm* algo) {
+int ct_set_algorithm(ct_scn* scn, const ct_algorithm* algo) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   int rc = check_algo(algo);
   if (rc) return rc;
   scn->algo = *algo;
   scn->config_gen += 1;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_set_freeze(ct_scn* scn, int freeze_gains, int freeze_delays) {
+int ct_set_freeze(ct_scn* scn, int freeze_gains, int freeze_delays) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   scn->algo.freeze_gains = freeze_gains != 0;
   scn->algo.freeze_delays = freeze_delays != 0;
   scn->config_gen += 1;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_set_learning_rate(ct_scn* scn, float learning_rate) {
+int ct_set_learning_rate(ct_scn* scn, float learning_rate) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   scn->algo.learning_rate = learning_rate;
   scn->config_gen += 1;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_field_size(ct_scn* scn, int field, size_t* nbytes) {
+int ct_field_size(ct_scn* scn, int field, size_t* nbytes) try {
   if (!scn || !nbytes) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   return field_bytes(scn, field, nbytes);
-}
+} CT_CATCH
 
-int ct_read_field(ct_scn* scn, int field, void* dst, size_t nbytes) {
+int ct_read_field(ct_scn* scn, int field, void* dst, size_t nbytes) try {
   if (!scn || !dst) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   size_t want = 0;
   int rc = field_bytes(scn, field, &want);
@@ -1549,9 +1580,9 @@ int ct_read_field(ct_scn* scn, int field, void* dst, size_t nbytes) {
       return scn->snap_n ? copy_down(scn, dst, scn->snap_Y, nbytes) : CT_OK;
     default: return fail(CT_ERR_INVALID_ARGUMENT, "unknown field %d", field);
   }
-}
+} CT_CATCH
 
-int ct_write_field(ct_scn* scn, int field, const void* src, size_t nbytes) {
+int ct_write_field(ct_scn* scn, int field, const void* src, size_t nbytes) try {
   if (!scn || !src) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   size_t want = 0;
   int rc = field_bytes(scn, field, &want);
@@ -1600,9 +1631,9 @@ int ct_write_field(ct_scn* scn, int field, const void* src, size_t nbytes) {
   if (field == CT_FIELD_DELAYS) CT_CUDA(ct::launch_min_delay(d, scn->ctx->stream), "min delay kernel");
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "write field");
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_sync(ct_scn* scn) {
+int ct_sync(ct_scn* scn) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   CT_DEVICE_SCOPE(scn->ctx->device);
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "cudaStreamSynchronize");
@@ -1613,15 +1644,15 @@ int ct_sync(ct_scn* scn) {
     return fail(status, "device-side failure: %s", ct_status_string(status));
   }
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_kernel_launches(ct_scn* scn, int64_t* launches) {
+int ct_kernel_launches(ct_scn* scn, int64_t* launches) try {
   if (!scn || !launches) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   *launches = scn->launches;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_set_profiling(ct_scn* scn, int enable) {
+int ct_set_profiling(ct_scn* scn, int enable) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   CT_DEVICE_SCOPE(scn->ctx->device);
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "cudaStreamSynchronize");
@@ -1638,9 +1669,9 @@ int ct_set_profiling(ct_scn* scn, int enable) {
     }
   }
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_read_profile(ct_scn* scn, double* ms, int64_t* launches) {
+int ct_read_profile(ct_scn* scn, double* ms, int64_t* launches) try {
   if (!scn || !ms || !launches) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(scn->ctx->device);
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "cudaStreamSynchronize");
@@ -1657,7 +1688,7 @@ int ct_read_profile(ct_scn* scn, double* ms, int64_t* launches) {
     launches[i] = scn->phase_launches[i];
   }
   return CT_OK;
-}
+} CT_CATCH
 
 }  // extern "C"
 
@@ -1723,7 +1754,12 @@ int batch_alloc(ct_batch* b, void** p, size_t bytes) {
     cudaGetLastError();  // reported here, not by the next launch
     return cuda_fail(err, "cudaMalloc (batch)");
   }
-  b->allocations.push_back(*p);
+  try {
+    b->allocations.push_back(*p);
+  } catch (...) {
+    cudaFree(*p);
+    throw;
+  }
   return CT_OK;
 }
 
@@ -2096,7 +2132,7 @@ int batch_set_order(ct_batch* b, int tile_order, bool fit) {
 extern "C" {
 
 int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int grad_mode, int precision,
-                    ct_batch** out) {
+                    ct_batch** out) try {
   if (!ctx || !scenarios || !out || count <= 0) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument or empty batch");
   *out = nullptr;
   if (grad_mode != CT_GRAD_REFERENCE && grad_mode != CT_GRAD_ADJOINT)
@@ -2125,7 +2161,14 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
         int rc0 = check_tf32_gradients(scenarios[i], precision);
         if (rc0) return rc0;
       }
-  ct_batch* b = new ct_batch;
+  struct Release {
+    void operator()(ct_batch* p) const {
+      batch_free(p);
+      delete p;
+    }
+  };
+  std::unique_ptr<ct_batch, Release> owner(new ct_batch);  // until the batch is handed out
+  ct_batch* b = owner.get();
   b->ctx = ctx;
   b->grad_mode = grad_mode;
   b->precision = precision;
@@ -2175,17 +2218,13 @@ int ct_batch_create(ct_ctx* ctx, ct_scn* const* scenarios, int64_t count, int gr
     if (e1) b->fork_ev.push_back(e1);
     if (e2) b->join_ev.push_back(e2);
   }
-  if (rc) {
-    batch_free(b);
-    delete b;
-    return rc;
-  }
+  if (rc) return rc;
   ctx->refs += 1;
-  *out = b;
+  *out = owner.release();
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_destroy(ct_batch* b) {
+int ct_batch_destroy(ct_batch* b) try {
   if (!b) return CT_OK;
   ct_ctx* ctx = b->ctx;
   DeviceScope device_scope__(ctx->device);
@@ -2194,9 +2233,9 @@ int ct_batch_destroy(ct_batch* b) {
   delete b;
   ctx_release(ctx);
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_run_epoch(ct_batch* b, int64_t* batch_indices) {
+int ct_batch_run_epoch(ct_batch* b, int64_t* batch_indices) try {
   if (!b || !batch_indices) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(b->ctx->device);
   const size_t n = b->scns.size();
@@ -2233,9 +2272,9 @@ int ct_batch_run_epoch(ct_batch* b, int64_t* batch_indices) {
     if (!s->algo.freeze_delays) note_delay_update(s, st);
   }
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* tile_order, double* best_ms) {
+int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* tile_order, double* best_ms) try {
   if (!b || !batch_indices) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(b->ctx->device);
   cudaStream_t st = b->ctx->stream;
@@ -2290,25 +2329,25 @@ int ct_batch_autotune(ct_batch* b, int64_t* batch_indices, int* ckpt_k, int* til
   if (tile_order) *tile_order = best_o;
   if (best_ms) *best_ms = best;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_sync(ct_batch* b) {
+int ct_batch_sync(ct_batch* b) try {
   if (!b) return fail(CT_ERR_INVALID_ARGUMENT, "batch is NULL");
   for (ct_scn* s : b->scns) {
     int rc = ct_sync(s);
     if (rc) return rc;
   }
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_set_profiling(ct_batch* b, int enable) {
+int ct_batch_set_profiling(ct_batch* b, int enable) try {
   if (!b) return fail(CT_ERR_INVALID_ARGUMENT, "batch is NULL");
   b->profiling = enable != 0;
   for (double& m : b->phase_ms) m = 0.0;
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_read_profile(ct_batch* b, double* ms) {
+int ct_batch_read_profile(ct_batch* b, double* ms) try {
   if (!b || !ms) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   CT_DEVICE_SCOPE(b->ctx->device);
   CT_CUDA(cudaStreamSynchronize(b->ctx->stream), "cudaStreamSynchronize");
@@ -2324,16 +2363,16 @@ int ct_batch_read_profile(ct_batch* b, double* ms) {
   b->open_event = nullptr;
   for (int i = 0; i < CT_PHASE_COUNT; ++i) ms[i] = b->phase_ms[i];
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_batch_info(ct_batch* b, int64_t* graph_kernels, int* uses_graph, int* forward_ctas, int* adjoint_ctas) {
+int ct_batch_info(ct_batch* b, int64_t* graph_kernels, int* uses_graph, int* forward_ctas, int* adjoint_ctas) try {
   if (!b) return fail(CT_ERR_INVALID_ARGUMENT, "batch is NULL");
   if (graph_kernels) *graph_kernels = b->graph_kernels;
   if (uses_graph) *uses_graph = b->exec != nullptr ? 1 : 0;
   if (forward_ctas) *forward_ctas = b->grid;
   if (adjoint_ctas) *adjoint_ctas = b->grid;
   return CT_OK;
-}
+} CT_CATCH
 
 }  // extern "C"
 
@@ -2459,7 +2498,7 @@ float scheduled_rate(const ct_run_config* c, int64_t e, float running, float ori
 extern "C" {
 
 int ct_run_model_based(ct_scn* scn, const ct_run_config* cfg, const int32_t* beat_orders, int64_t* batch_index,
-                       float* epoch_losses, ct_run_summary* summary) {
+                       float* epoch_losses, ct_run_summary* summary) try {
   if (!scn || !cfg || !batch_index || !summary) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   int rc = check_run_config(cfg);
   if (rc) return rc;
@@ -2496,10 +2535,10 @@ int ct_run_model_based(ct_scn* scn, const ct_run_config* cfg, const int32_t* bea
   CT_CUDA(ct::launch_average_delays(scn->d, scn->ctx->stream), "average delays kernel");
   scn->launches += 1;
   return ct_sync(scn);
-}
+} CT_CATCH
 
 int ct_batch_run_model_based(ct_batch* batch, const ct_run_config* cfg, int64_t* batch_indices, float* epoch_losses,
-                             ct_run_summary* summaries) {
+                             ct_run_summary* summaries) try {
   if (!batch || !cfg || !batch_indices || !summaries) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   int rc = check_run_config(cfg);
   if (rc) return rc;
@@ -2563,9 +2602,9 @@ int ct_batch_run_model_based(ct_batch* batch, const ct_run_config* cfg, int64_t*
     s->launches += 1;
   }
   return ct_batch_sync(batch);
-}
+} CT_CATCH
 
-int ct_calculate_plotting_arrays(ct_scn* scn, float sample_rate_hz) {
+int ct_calculate_plotting_arrays(ct_scn* scn, float sample_rate_hz) try {
   if (!scn) return fail(CT_ERR_INVALID_ARGUMENT, "scenario is NULL");
   CT_DEVICE_SCOPE(scn->ctx->device);
   int rc = ensure_post(scn, true);
@@ -2576,10 +2615,10 @@ int ct_calculate_plotting_arrays(ct_scn* scn, float sample_rate_hz) {
   rc = ct_sync(scn);
   if (rc == CT_OK || rc == CT_ERR_NO_MAXIMUM) scn->post_arrays = true;
   return rc;
-}
+} CT_CATCH
 
 int ct_calculate_final(ct_scn* scn, const int32_t* ground_truth_types, const int32_t* voxel_numbers, int64_t nx,
-                       int64_t ny, int64_t nz, ct_final_metrics* out) {
+                       int64_t ny, int64_t nz, ct_final_metrics* out) try {
   if (!scn || !ground_truth_types || !voxel_numbers || !out) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   if (nx <= 0 || ny <= 0 || nz <= 0) return fail(CT_ERR_INVALID_ARGUMENT, "empty grid");
   const int64_t cells = nx * ny * nz;
@@ -2621,7 +2660,7 @@ int ct_calculate_final(ct_scn* scn, const int32_t* ground_truth_types, const int
   if (e != cudaSuccess) return cuda_fail(e, "final metrics");
   scn->launches += 4;
   return ct_sync(scn);
-}
+} CT_CATCH
 
 
 // ---- model construction on the device
@@ -2715,7 +2754,7 @@ int fill_lead_field(ct_ctx* ctx, const ct_spatial_desc* g, const std::vector<flo
 
 extern "C" {
 
-int ct_measurement_matrix(ct_ctx* ctx, const ct_spatial_desc* desc, float* out, size_t nbytes) {
+int ct_measurement_matrix(ct_ctx* ctx, const ct_spatial_desc* desc, float* out, size_t nbytes) try {
   if (!ctx || !desc || !out) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   std::vector<int64_t> cell_of;
   int rc = check_grid(desc, cell_of);
@@ -2740,9 +2779,9 @@ int ct_measurement_matrix(ct_ctx* ctx, const ct_spatial_desc* desc, float* out, 
   CT_CUDA(cudaMemcpyAsync(out, dH, want, cudaMemcpyDeviceToHost, ctx->stream), "download");
   CT_CUDA(cudaStreamSynchronize(ctx->stream), "download");
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_scenario_set_measurement_matrix(ct_scn* scn, const ct_spatial_desc* desc) {
+int ct_scenario_set_measurement_matrix(ct_scn* scn, const ct_spatial_desc* desc) try {
   if (!scn || !desc) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   std::vector<int64_t> cell_of;
   int rc = check_grid(desc, cell_of);
@@ -2778,10 +2817,10 @@ int ct_scenario_set_measurement_matrix(ct_scn* scn, const ct_spatial_desc* desc)
   }
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "measurement matrix");
   return CT_OK;
-}
+} CT_CATCH
 
 int ct_delay_samples(ct_ctx* ctx, const ct_spatial_desc* desc, float* initial_delays, int32_t* delays, float* coefs,
-                     int64_t count) {
+                     int64_t count) try {
   if (!ctx || !desc || !initial_delays || !delays || !coefs || !desc->propagation_velocities_m_per_s)
     return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   std::vector<int64_t> cell_of;
@@ -2830,10 +2869,10 @@ int ct_delay_samples(ct_ctx* ctx, const ct_spatial_desc* desc, float* initial_de
                 x, y, z, n);
   }
   return CT_OK;
-}
+} CT_CATCH
 
 int ct_connect_voxels(const ct_spatial_desc* desc, float current_factor_in_pathology, float* gains, size_t gains_bytes,
-                      float* activation_time_ms) {
+                      float* activation_time_ms) try {
   if (!desc || !gains || !activation_time_ms || !desc->propagation_velocities_m_per_s)
     return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   std::vector<int64_t> cell_of;
@@ -2847,9 +2886,9 @@ int ct_connect_voxels(const ct_spatial_desc* desc, float current_factor_in_patho
                           desc->nz, desc->propagation_velocities_m_per_s, current_factor_in_pathology, gains,
                           activation_time_ms);
   return CT_OK;
-}
+} CT_CATCH
 
-int ct_output_state_indices(const ct_spatial_desc* desc, int32_t* out, size_t nbytes) {
+int ct_output_state_indices(const ct_spatial_desc* desc, int32_t* out, size_t nbytes) try {
   if (!desc || !out) return fail(CT_ERR_INVALID_ARGUMENT, "NULL argument");
   std::vector<int64_t> cell_of;
   int rc = check_grid(desc, cell_of);
@@ -2859,6 +2898,6 @@ int ct_output_state_indices(const ct_spatial_desc* desc, int32_t* out, size_t nb
   if (nbytes != want) return fail(CT_ERR_INVALID_ARGUMENT, "output_state_indices have %zu bytes, got %zu", want, nbytes);
   ct::output_state_indices_host(desc->voxel_types, desc->voxel_numbers, desc->nx, desc->ny, desc->nz, cell_of, out);
   return CT_OK;
-}
+} CT_CATCH
 
 }  // extern "C"

@@ -6,7 +6,10 @@
 // wrong is kept as text (host_device_report). Allocations can be made to fail by size, elapsed times
 // can be scripted.
 #include <cuda_runtime.h>
+#include <dlfcn.h>
+#include <pthread.h>
 
+#include <cerrno>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -34,7 +37,8 @@ struct Graph {
 std::map<char*, size_t> g_blocks;
 size_t g_live = 0;
 size_t g_fail_from = ~size_t(0);      // device allocations of at least so many bytes fail
-size_t g_host_fail_from = ~size_t(0); // and the library's host allocations
+size_t g_host_fail_from = ~size_t(0) / 2;  // the library's host allocations of this size up to twice as much fail
+bool g_no_threads = false;            // no thread can be started (with this library preloaded)
 cudaError_t g_last = cudaSuccess;     // of this runtime, until it is asked for
 std::string g_report;
 Graph* g_capturing = nullptr;
@@ -90,7 +94,7 @@ void check(const Recorded& r) {
 
 // ---- the library's host allocations
 void* operator new(size_t n) {
-  void* p = n >= g_host_fail_from ? nullptr : std::malloc(n ? n : 1);
+  void* p = n >= g_host_fail_from && n < g_host_fail_from * 2 ? nullptr : std::malloc(n ? n : 1);
   if (!p) throw std::bad_alloc();
   return p;
 }
@@ -102,6 +106,12 @@ extern "C" {
 // ---- control
 void host_device_fail_from(size_t bytes) { g_fail_from = bytes; }
 void host_device_fail_host_from(size_t bytes) { g_host_fail_from = bytes; }
+void host_device_no_threads(int on) { g_no_threads = on != 0; }
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* p) {
+  using Create = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+  static Create next = (Create)dlsym(RTLD_NEXT, "pthread_create");
+  return g_no_threads ? EPERM : next(t, a, f, p);
+}
 size_t host_device_live() { return g_live; }
 void host_device_times(const float* ms, int n) {
   g_times.assign(ms, ms + n);

@@ -3,8 +3,10 @@ memory is host memory with known blocks and a launch checks that what it was giv
 made to fail on the host; what a later launch is then given must still be live and large enough."""
 
 import ctypes
+import os
 import pathlib
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -17,10 +19,14 @@ def library(tmp_path_factory):
     from cardiotrust_b200 import _lib
 
     so = tmp_path_factory.mktemp("host_device") / "libhost_device.so"
+    _build(so)
+    return _lib.load(so)
+
+
+def _build(so):
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
                            "-x", "c++", str(ROOT / "cardiotrust_b200/csrc/ct_api.cu"),
-                           str(ROOT / "tests/native/host_device.cpp"), "-o", str(so), "-lpthread"])
-    return _lib.load(so)
+                           str(ROOT / "tests/native/host_device.cpp"), "-o", str(so), "-lpthread", "-ldl"])
 
 
 class _Host:
@@ -32,6 +38,9 @@ class _Host:
 
     def fail_from(self, nbytes):
         self.lib.host_device_fail_from(ctypes.c_size_t(nbytes))
+
+    def fail_host_from(self, nbytes):
+        self.lib.host_device_fail_host_from(ctypes.c_size_t(nbytes))
 
     def live(self):
         return int(self.lib.host_device_live())
@@ -45,7 +54,14 @@ class _Host:
         return buf.value.decode()
 
 
-NEVER = (1 << 64) - 1
+NEVER = (1 << 63) - 1
+#: batches and engines made by a test, closed with the library that they belong to
+OPEN = []
+
+
+def _close_all():
+    while OPEN:
+        OPEN.pop().close()
 
 
 @pytest.fixture
@@ -59,6 +75,7 @@ def host(library, monkeypatch):
     h.report()
     yield h
     h.fail_from(NEVER)
+    _close_all()
 
 
 def _engine(ctx, shape, steps, **kw):
@@ -68,7 +85,8 @@ def _engine(ctx, shape, steps, **kw):
     spec = sc.ScenarioSpec(shape=shape, num_steps=steps, num_sensors=3, patho_size=1, patho_origin=(1, 1, 1), seed=2)
     scn = sc.build(spec)
     scn.measurements = np.zeros((1, steps, scn.num_sensors), np.float32)
-    return alg.EpochEngine.from_scenario(ctx, scn, num_batch_slots=16, **kw)
+    OPEN.append(alg.EpochEngine.from_scenario(ctx, scn, num_batch_slots=16, **kw))
+    return OPEN[-1]
 
 
 @pytest.fixture
@@ -77,6 +95,7 @@ def ctx(host):
 
     c = alg.Context(0)
     yield c
+    _close_all()
     c.close()
 
 
@@ -84,7 +103,8 @@ def _batch(ctx, members, **kw):
     from cardiotrust_b200 import algorithm as alg
 
     engines = [_engine(ctx, *m) for m in members]
-    return engines, alg.EpochBatch(ctx, engines, precision=alg.Precision.Fp32, **kw)
+    OPEN.append(alg.EpochBatch(ctx, engines, precision=alg.Precision.Fp32, **kw))
+    return engines, OPEN[-1]
 
 
 #: 9, 2 and 2 tiles on 4 CTAs: only the arrangement in one phase needs records for all 13
@@ -105,7 +125,6 @@ def test_autotune_without_room_for_one_arrangement(host, ctx):
     batch.run_epoch()
     assert host.report() == ""
     assert host.live() == before
-    batch.close()
 
 
 def test_autotune_gives_back_the_larger_record(host, ctx):
@@ -116,7 +135,6 @@ def test_autotune_gives_back_the_larger_record(host, ctx):
     batch.run_epoch()
     assert host.report() == ""
     assert host.live() == before
-    batch.close()
 
 
 def test_autotune_keeps_the_record_of_its_choice(host, ctx):
@@ -125,7 +143,6 @@ def test_autotune_keeps_the_record_of_its_choice(host, ctx):
     assert batch.autotune()["tile_order"] == 2
     batch.run_epoch()
     assert host.report() == ""
-    batch.close()
 
 
 def _with_delays(engine, largest):
@@ -152,7 +169,6 @@ def test_batch_after_an_exchange_ring_that_could_not_grow(host, ctx):
     engines[0].run_epoch(0, precision=0)
     batch.run_epoch()
     assert host.report() == ""
-    batch.close()
 
 
 def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
@@ -165,4 +181,46 @@ def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
     eng.run_epoch_plain(0)  # an update, before any recursion has asked for its ring
     eng.run_epoch(0, precision=0)
     assert host.report() == ""
-    eng.close()
+
+
+#: no thread can be started, then each size of host allocation fails: a status each time, never an abort
+CHILD = """
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import pathlib
+import test_host_device as t
+from cardiotrust_b200 import _lib, algorithm as alg
+_lib._LIB = _lib.load(pathlib.Path({so!r}))
+host = t._Host(_lib._LIB)
+ctx = alg.Context(0)
+host.lib.host_device_no_threads(1)
+t._engine(ctx, (4, 4, 4), 50)
+t._close_all()
+print("without threads")
+host.lib.host_device_no_threads(0)
+before, refused = host.live(), 0
+for bits in range(4, 24):
+    host.fail_host_from(1 << bits)
+    try:
+        engines, batch = t._batch(ctx, t.MEMBERS, grad_mode=alg.GradMode.Adjoint)
+        batch.run_epoch()
+        batch.autotune()
+        engines[0].run_epoch(0, precision=0)
+    except _lib.CtError as e:
+        assert e.status == _lib.CT_ERR_OUT_OF_MEMORY, e
+        refused += 1
+    host.fail_host_from(t.NEVER)
+    t._close_all()
+    assert host.live() == before and host.report() == "", (bits, host.live(), before)
+print("refused", refused)
+"""
+
+
+def test_host_failures_are_reported(tmp_path):
+    so = tmp_path / "libhost_device.so"
+    _build(so)
+    code = CHILD.format(root=str(ROOT), tests=str(ROOT / "tests"), so=str(so))
+    done = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=str(so)), capture_output=True,
+                          text=True, timeout=300)
+    assert done.returncode == 0, done.stdout + done.stderr
+    assert "without threads" in done.stdout and int(done.stdout.split("refused")[1]) >= 8
