@@ -197,7 +197,11 @@ __device__ __noinline__ unsigned long long may_wait(unsigned long long since, in
   }
   return since;
 }
-// Every `mask` + 1 spins of a wait: whether it may go on.
+// Every `mask` + 1 spins of a wait: whether it may go on. Lanes decide for themselves, and one whose wait is lost leaves the
+// kernel on the shortest way, without another vote or barrier. The others find sm.abort at their next look; until
+// then their votes, shuffles and reductions count the threads that have not exited, and no mbarrier phase can
+// complete without the arrivals that are missing now, so that they end in waits that look. (One decision per warp, by a
+// vote in every wait, cost 1 % on the 20x20x20 cuboid and 11 % on the shell's forward.)
 __device__ __forceinline__ bool go_on(WaveSmem& sm, const WaveLaunch& L, int& spins, unsigned long long& since, int mask) {
   if ((++spins & mask) != 0) return true;
   since = may_wait(since, &sm.abort, L.status, &L.heartbeat->count);
@@ -416,7 +420,6 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
     }
     pos = after;
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Counters that run through all of a warp's visits.
@@ -868,6 +871,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant
     compute<kItems, kMiddle, ADJ>(sm, L, w);
   else
     compute<kLastItems, kLast, ADJ>(sm, L, w);
+  asm volatile("cp.async.wait_all;" ::: "memory");  // no thread leaves before its copies have landed, after a lost wait either
 }
 
 bool configure(int device) {
