@@ -32,7 +32,8 @@
 //   * No grid barrier: a finished row goes to an exchange ring in global memory (L2) as one
 //     16-byte entry {x0, x1, x2, step + 1} per voxel, and the readers look at the entry itself until its
 //     tag is the step they need: a 128-bit relaxed access is one access, so no fence separates data and
-//     flag. Every read is of a row at least dmin steps back, so tiles run up to dmin steps apart, and the
+//     flag. That is the programming model's word for the polls (ld.relaxed.b128); the staging warp's cp.async of 16
+//     aligned bytes relies on the hardware, which moves such a piece of one 32-byte sector as a whole. Every read is of a row at least dmin steps back, so tiles run up to dmin steps apart, and the
 //     latency of the exchange overlaps the work on the steps between. (The former kernels met at a
 //     grid barrier every 8 steps, staged a block's rows after it and ran their producer and consumer
 //     phases one after the other.)
@@ -361,6 +362,7 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
         from[i] = p.xch + p.halo[e];
         to[i] = 16u * p.hpos[e];
       }
+      const bool zeros = r < 0;
       for (; r < min(0, end); ++r, ++pos) {  // rows before the beat
         if (!room(pos)) return;
 #pragma unroll
@@ -371,9 +373,11 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
       const int V = p.V, mask = p.xrows - 1;
       const int parts = (nh + 31) / 32;
       const int* near = p.near + (size_t)tile * kNearTiles;
-      if (!v.whole && near[0] >= 0) {
+      if (!v.whole && near[0] >= 0 && !zeros) {
         // All rows of the visit belong to earlier blocks: once the tiles around have published these, the copies
-        // need no look at their tags, and each row's arrival is counted by the copies themselves.
+        // need no look at their tags, and each row's arrival is counted by the copies themselves. Such an arrival stands for
+        // the copies alone: zero rows stored before it, which readers do not wait for one by one, would not be ordered by
+        // it, so the few visits that begin before the beat take the other way.
         const int *a = progress_of(p, near[lane]), *b = progress_of(p, near[lane + 32]);
         int spins = 0;
         unsigned long long since = 0;
