@@ -323,8 +323,8 @@ int prepare_sliced(ct_scn* s) {
 }
 
 // The exchange ring of the recursion kernels. A tile overwrites the entry of step t - xrows when it
-// finishes step t; by then every tile that it reads has finished step t - dmax and so has staged all
-// rows up to t - dmin - dmax, provided that the tiles that read it are among those that it reads. Without
+// finishes step t; by then every tile that it reads has finished step t - dmax and so reads no row before
+// t - 2 dmax any more, provided that the tiles that read it are among those that it reads. Without
 // that symmetry the ring holds every step of the beat.
 int prepare_exchange(ct_scn* s) {
   DeviceScenario& d = s->d;

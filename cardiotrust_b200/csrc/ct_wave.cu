@@ -857,11 +857,12 @@ __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant
     if (!L.scns) sm.single = L.single;
   }
   __syncthreads();
-  // every exchange ring must hold the rows that a reader may still want (or all of them)
+  // Every exchange ring must hold the rows that a reader may still want, or all of them: when a tile writes step t, its
+  // neighbours have finished step t - dmax at least, and from there on they read back to t - 2 dmax.
   for (int s = 0; s < L.nscn; ++s) {
     const WaveScn& p = scenario_of(sm, L, s);
     const Geometry geo = geometry(p);
-    if (p.xrows < p.T && (long long)geo.dmin + geo.dmax + 2 > p.xrows) {  // every CTA leaves here
+    if (p.xrows < p.T && 2ll * geo.dmax + 2 > p.xrows) {  // every CTA leaves here
       if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(L.status, 0, (int32_t)CT_ERR_NOT_SUPPORTED);
       return;
     }

@@ -1,5 +1,5 @@
 // Launches of the recursion kernel whose rows never all come: tiles of a small scenario wait for a tile that the launch
-// leaves out. Every wait is bounded, so the launch ends by itself with a status.
+// leaves out, or the exchange ring is too short. Every wait is bounded, so the launch ends by itself with a status.
 // wave_waits(form, status, ms): 0, or the line of the call that failed.
 #include <cuda_runtime.h>
 
@@ -28,6 +28,7 @@ enum Form {
   kStaged,     // one tile of two, its history staged
   kDirect,     // the same with delays too far apart for the staging ring
   kShared,     // two tiles of three in one CTA, which asks for the progress of the third
+  kShortRing,  // every tile runs, in a ring that could lose rows before they are read
 };
 
 extern "C" int wave_waits(int form, int* status, float* ms) {
@@ -36,7 +37,7 @@ extern "C" int wave_waits(int form, int* status, float* ms) {
   const int tiles = form == kShared ? 3 : 2, V = tiles * kTile, S = 3 * V, T = 200;
   // voxel u reads its counterpart in the next tile (the last tile: in the first) along offset 0, and in the tile before along 1
   std::vector<int32_t> src(V * ct::kOffsets, -1), delays(V * ct::kOffsets, 1), halo(tiles * kHalo), nhalo(tiles),
-      near(tiles * ct::kNearTiles), dmin = {wide ? 2 : 6, wide ? 60 : 9};
+      near(tiles * ct::kNearTiles), dmin = {wide || form == kShortRing ? 2 : 6, wide ? 60 : 9};
   std::vector<int16_t> hpos(tiles * kHalo), hslot(tiles * kTile * ct::kOffsets, kHalo - 1);
   for (int t = 0; t < tiles; ++t) {
     const int next = (t + 1) % tiles, last = (t + tiles - 1) % tiles;
@@ -61,7 +62,7 @@ extern "C" int wave_waits(int form, int* status, float* ms) {
   p.V = V;
   p.T = T;
   p.ntiles = tiles;
-  p.xrows = 128;
+  p.xrows = form == kShortRing ? 16 : 128;
   p.src = device(src);
   p.halo = device(halo);
   p.hpos = device(hpos);
@@ -83,7 +84,7 @@ extern "C" int wave_waits(int form, int* status, float* ms) {
   p.threshold = 1.0f;
   std::vector<int2> list;
   for (int t = 0; t < tiles; ++t)
-    if (form == kAll || t + 1 < tiles) list.push_back(make_int2(0, t * kTile));
+    if (form == kAll || form == kShortRing || t + 1 < tiles) list.push_back(make_int2(0, t * kTile));
   ct::WaveLaunch l{};
   l.scns = device(std::vector<ct::WaveScn>(1, p));
   l.nscn = 1;

@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 ROOT = pathlib.Path(__file__).resolve().parents[1]
-ALL, STAGED, DIRECT, SHARED = range(4)
+ALL, STAGED, DIRECT, SHARED, SHORT_RING = range(5)
 
 
 @pytest.fixture(scope="module")
@@ -39,4 +39,14 @@ def test_rows_that_never_come(waits, form):
     status, ms = waits(form)
     assert status == _lib.CT_ERR_TIMEOUT
     assert 1900 < ms < 10000
+    assert waits(ALL)[0] == _lib.CT_OK
+
+
+def test_a_ring_that_could_lose_rows_is_refused(waits):
+    """16 rows with delays of 2 to 9, where readers may go back 18 steps: a status at once, nothing runs."""
+    from cardiotrust_b200 import _lib
+
+    status, ms = waits(SHORT_RING)
+    assert status == _lib.CT_ERR_NOT_SUPPORTED
+    assert ms < 100
     assert waits(ALL)[0] == _lib.CT_OK
