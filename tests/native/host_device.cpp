@@ -45,6 +45,7 @@ Graph* g_capturing = nullptr;
 std::vector<float> g_times;
 size_t g_time = 0;
 std::vector<int> g_orders;  // phases of every batched forward that ran
+int g_routes[2][3];         // tiles of the last forward and adjoint: followed by progress, by tags, polled directly
 
 void wrong(const std::string& what) {
   if (g_report.size() < 4000) g_report += what + "\n";
@@ -90,6 +91,11 @@ void check(const Recorded& r) {
   for (int i = 0; i < l.nscn; ++i) check_ring(l.scns[i], r.adjoint ? "batched adjoint" : "batched forward");
 }
 
+void count_routes(int (&n)[3], const ct::DeviceScenario& d, const int32_t* nhalo, const int32_t* near) {
+  n[0] = n[1] = n[2] = 0;
+  for (int t = 0; t < d.tiles; ++t) ++n[nhalo[t] < 0 ? 2 : nhalo[t] > 0 && near[t * ct::kNearTiles] < 0 ? 1 : 0];
+}
+
 }  // namespace
 
 // ---- the library's host allocations
@@ -124,6 +130,7 @@ int host_device_report(char* out, int len) {  // and forget it
   g_report.clear();
   return n;
 }
+void host_device_routes(int* out) { std::memcpy(out, g_routes, sizeof(g_routes)); }
 int host_device_phases(int* out, int len) {  // phases of the batched forwards since the last call
   const int n = (int)g_orders.size();
   for (int i = 0; i < n && i < len; ++i) out[i] = g_orders[(size_t)i];
@@ -254,11 +261,13 @@ cudaError_t launch_wave(const WaveLaunch& l, bool adjoint, int grid, cudaStream_
 }
 cudaError_t launch_forward(DeviceScenario& d, float, cudaStream_t) {
   check_ring(wave_scenario(d, false, WaveScalars{}, nullptr), "forward");
+  count_routes(g_routes[0], d, d.nhalo, d.near);
   if (d.tiles > d.wave_grid) need(d.record, (size_t)d.tiles * kRecordBytes, "forward record");
   return cudaSuccess;
 }
 cudaError_t launch_adjoint_states(DeviceScenario& d, const WaveScalars&, cudaStream_t) {
   check_ring(wave_scenario(d, true, WaveScalars{}, nullptr), "adjoint");
+  count_routes(g_routes[1], d, d.rnhalo, d.rnear);
   return cudaSuccess;
 }
 cudaError_t clear_exchange(DeviceScenario& d, cudaStream_t) {

@@ -78,6 +78,25 @@ def host(library, monkeypatch):
     _close_all()
 
 
+@pytest.mark.parametrize("case", ["exchanged", "exchanged_short", "far", "far_short"])
+def test_rewired_cases_meet_every_route(host, ctx, case):
+    """The scenarios that test_gpu_routes.py runs: tiles followed by progress, by tags and polled directly."""
+    import test_gpu_routes as routes
+
+    from cardiotrust_b200 import algorithm as alg
+
+    scn = routes.scenario(*routes.CASES[case])
+    scn.measurements = np.zeros((1, scn.control_function.shape[0], scn.num_sensors), np.float32)
+    OPEN.append(alg.EpochEngine.from_scenario(ctx, scn, algorithm=alg.Algorithm(freeze_delays=False)))
+    far = "far" in routes.CASES[case]
+    OPEN[-1].run_epoch(0, grad_mode=alg.GradMode.Reference if far else alg.GradMode.Adjoint, precision=0)
+    n = (ctypes.c_int * 6)()
+    host.lib.host_device_routes(n)
+    progress, tags, polled = n[:3] if far else (min(n[0], n[3]), 3, min(n[2], n[5]))
+    assert min(progress, tags, polled) >= 3, list(n)
+    assert sum(n[:3]) == 318 and host.report() == ""
+
+
 def _engine(ctx, shape, steps, **kw):
     from cardiotrust_b200 import algorithm as alg
     from cardiotrust_b200 import scenario as sc
