@@ -59,12 +59,13 @@ struct ct_scn {
   std::vector<int32_t> nbr_dev;   // neighbour table in device order (adjoint reverse table)
   std::vector<uint8_t> bank;      // (2 y + z) mod 8 of each device voxel's grid coordinates
   bool symmetric = true;          // a voxel's neighbours all have it as a neighbour
-  // Upper bound of the largest delay of a connected pair: exact after creation and delay writes,
-  // +1 per update that rolls delays (roll_delays moves a delay by at most one, and none past 1,000). Sizes the
-  // exchange ring without reading the device.
-  int64_t dmax_bound = 1;
-  // Asynchronous read-back of the device's largest delay after an update (pinned word + event):
-  // once it has landed, the bound becomes that value plus the updates enqueued since.
+  // Bounds of the delays of connected pairs: exact after creation and delay writes, one wider
+  // per update that rolls delays (roll_delays moves a delay by at most one, and none past 1,000). They size the
+  // exchange ring and choose the recursions' kernel without reading the device.
+  int64_t dmin_bound = 1, dmax_bound = 1;
+  bool halo_fits = true, rhalo_fits = true;  // every tile's halo (in the adjoint's direction) fits the staging slots
+  // Asynchronous read-back of the device's delay range after an update (pinned words + event):
+  // once it has landed, the bounds become that range, wider by the updates enqueued since.
   int32_t* dmax_host = nullptr;
   cudaEvent_t dmax_event = nullptr;
   int64_t updates = 0;          // updates that may roll delays, enqueued so far
@@ -240,11 +241,18 @@ void seeded_shuffle(ct_scn* s, std::vector<int32_t>& order) {
   }
 }
 
-int64_t max_connected_delay(const std::vector<int32_t>& nbr, const int32_t* delays) {
-  int64_t m = 1;
+// Takes the bounds of the delays from the delays themselves (of connected pairs, in reference order).
+void bound_delays(ct_scn* s, const int32_t* delays) {
+  const std::vector<int32_t>& nbr = s->nbr_host;
+  int32_t lo = INT32_MAX, hi = 1;
   for (size_t i = 0; i < nbr.size(); ++i)
-    if (nbr[i] >= 0 && delays[i] > m) m = delays[i];
-  return m;
+    if (nbr[i] >= 0) {
+      lo = std::min(lo, delays[i]);
+      hi = std::max(hi, delays[i]);
+    }
+  s->dmin_bound = std::min(lo, hi);
+  s->dmax_bound = hi;
+  s->updates_at_read = -1;
 }
 
 void release(ct_scn* s, void* p) {
@@ -253,13 +261,14 @@ void release(ct_scn* s, void* p) {
   s->allocations.erase(std::remove(s->allocations.begin(), s->allocations.end(), p), s->allocations.end());
 }
 
-// After an update that may roll delays: count it and enqueue the read-back of the largest delay.
+// After an update that may roll delays: count it and enqueue the read-back of the delay range.
 void note_delay_update(ct_scn* s, cudaStream_t st) {
   s->updates += 1;
   if (s->dmax_bound < 1000) s->dmax_bound += 1;  // a larger delay that was written stays (roll_delays)
+  if (s->dmin_bound > 1) s->dmin_bound -= 1;
   if (!s->dmax_host) {
     void* p = nullptr;
-    if (cudaMallocHost(&p, sizeof(int32_t)) != cudaSuccess) return;
+    if (cudaMallocHost(&p, 2 * sizeof(int32_t)) != cudaSuccess) return;
     if (cudaEventCreateWithFlags(&s->dmax_event, cudaEventDisableTiming) != cudaSuccess) {
       cudaFreeHost(p);
       return;
@@ -267,7 +276,7 @@ void note_delay_update(ct_scn* s, cudaStream_t st) {
     s->dmax_host = static_cast<int32_t*>(p);
   }
   if (s->updates_at_read >= 0 && cudaEventQuery(s->dmax_event) != cudaSuccess) return;  // one in flight
-  if (cudaMemcpyAsync(s->dmax_host, s->d.dmin + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+  if (cudaMemcpyAsync(s->dmax_host, s->d.dmin, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaEventRecord(s->dmax_event, st) != cudaSuccess) {
     cudaGetLastError();
     return;
@@ -275,11 +284,12 @@ void note_delay_update(ct_scn* s, cudaStream_t st) {
   s->updates_at_read = s->updates;
 }
 
-// Tightens dmax_bound with a read-back that has landed.
-void refresh_delay_bound(ct_scn* s) {
+// Tightens the bounds with a read-back that has landed.
+void refresh_delay_bounds(ct_scn* s) {
   if (s->updates_at_read < 0 || cudaEventQuery(s->dmax_event) != cudaSuccess) return;
-  const int64_t bound = std::max<int64_t>(1, *s->dmax_host) + (s->updates - s->updates_at_read);
-  s->dmax_bound = std::min<int64_t>(s->dmax_bound, bound);
+  const int64_t since = s->updates - s->updates_at_read, lo = s->dmax_host[0], hi = std::max<int64_t>(1, s->dmax_host[1]);
+  s->dmax_bound = std::min<int64_t>(s->dmax_bound, hi + since);
+  if (lo <= hi) s->dmin_bound = std::max<int64_t>(s->dmin_bound, lo - since);
   s->updates_at_read = -1;
 }
 
@@ -328,7 +338,13 @@ int prepare_sliced(ct_scn* s) {
 // that symmetry the ring holds every step of the beat.
 int prepare_exchange(ct_scn* s) {
   DeviceScenario& d = s->d;
-  refresh_delay_bound(s);
+  refresh_delay_bounds(s);
+  const bool wide = s->dmax_bound - s->dmin_bound > ct::kFwdRingSpread;
+  const int routes = !s->halo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
+  const int rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
+  if (d.routes != routes || d.rroutes != rroutes) s->config_gen += 1;
+  d.routes = routes;
+  d.rroutes = rroutes;
   int64_t want = 8, all = 8;
   while (want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30)) want <<= 1;
   while (all < d.T) all <<= 1;
@@ -486,11 +502,13 @@ int prepare_adjoint(ct_scn* s) {
       slot = (int32_t)v;
     }
   const HaloTables t = build_halos(rev, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
+  s->rhalo_fits = *std::min_element(t.count.begin(), t.count.end()) >= 0;
   int rc = alloc(s, &d.rhalo, (int64_t)t.halo.size());
   if (!rc) rc = alloc(s, &d.rhpos, (int64_t)t.pos.size());
   if (!rc) rc = alloc(s, &d.rhslot, (int64_t)t.slot.size());
   if (!rc) rc = alloc(s, &d.rnear, (int64_t)t.near.size());
   if (!rc) rc = alloc(s, &d.rnhalo, (int64_t)t.count.size());
+  if (!rc) rc = alloc(s, &d.rrange, 2 * (int64_t)t.count.size());
   if (!rc && !d.LX) rc = alloc(s, &d.LX, d.T * d.S);
   if (!rc) rc = alloc(s, &d.rev, V * kOffsets);
   if (!rc) rc = upload(s, d.rev, rev.data(), sizeof(int32_t) * rev.size());
@@ -500,12 +518,14 @@ int prepare_adjoint(ct_scn* s) {
   if (!rc) rc = upload(s, d.rnear, t.near.data(), sizeof(int32_t) * t.near.size());
   if (!rc) rc = upload(s, d.rnhalo, t.count.data(), sizeof(int32_t) * t.count.size());
   if (!rc) {
-    cudaError_t e = cudaStreamSynchronize(st);  // the host tables go out of scope
+    cudaError_t e = ct::launch_delay_ranges(d, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host tables go out of scope
     if (e != cudaSuccess) rc = cuda_fail(e, "adjoint set-up");
   }
+  s->config_gen += 1;  // an update that a batch captured before knows nothing of these ranges
   if (rc) {
-    for (void* p : {(void*)d.rev, (void*)d.rhalo, (void*)d.rhpos, (void*)d.rhslot, (void*)d.rnear, (void*)d.rnhalo, (void*)d.LX}) release(s, p);
-    d.rev = d.rhalo = d.rnhalo = d.rnear = nullptr;
+    for (void* p : {(void*)d.rev, (void*)d.rhalo, (void*)d.rhpos, (void*)d.rhslot, (void*)d.rnear, (void*)d.rnhalo, (void*)d.rrange, (void*)d.LX}) release(s, p);
+    d.rev = d.rhalo = d.rnhalo = d.rnear = d.rrange = nullptr;
     d.rhslot = d.rhpos = nullptr;
     d.LX = nullptr;
   }
@@ -541,7 +561,7 @@ int run_beat(ct_scn* s, int64_t beat, int precision, int grad_mode) {
   const bool adjoint = grad_mode == CT_GRAD_ADJOINT;
   int rc = prepare_exchange(s);  // an update of an earlier beat may have rolled delays
   if (rc) return rc;
-  CT_CUDA(run_phase(s, CT_PHASE_FORWARD, 1,
+  CT_CUDA(run_phase(s, CT_PHASE_FORWARD, d.routes == ct::kDecide ? 2 : 1,
                     [&] { return ct::launch_forward(d, a.maximum_regularization_threshold, st); }),
           "forward kernel");
   if (precision == CT_PREC_FP32) {
@@ -565,7 +585,7 @@ int run_beat(ct_scn* s, int64_t beat, int precision, int grad_mode) {
   if (!a.freeze_gains || !a.freeze_delays) {
     const ct::DeriveScalars ds = derive_scalars(s);
     if (adjoint) {
-      CT_CUDA(run_phase(s, CT_PHASE_DERIVE, 2,
+      CT_CUDA(run_phase(s, CT_PHASE_DERIVE, d.rroutes == ct::kDecide ? 3 : 2,
                         [&] {
                           cudaError_t e = ct::launch_adjoint_states(d, wave_scalars(s), st);
                           return e != cudaSuccess ? e : ct::launch_adjoint_gradients(d, ds, st);
@@ -617,7 +637,7 @@ int batch_end(ct_scn* s, int64_t n_beats, int64_t* batch_index) {
   e = ct::launch_update(d, u, st);
   if (e != cudaSuccess) return e;
   if (!a.freeze_delays) {
-    e = ct::launch_min_delay(d, st);
+    e = ct::launch_delay_ranges(d, st);
     if (e != cudaSuccess) return e;
   }
   return ct::launch_batch_metrics(d, *batch_index, st);
@@ -1010,7 +1030,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   s->ctx = ctx;
   s->algo = *algo;
   s->nbr_host = nbr;
-  s->dmax_bound = max_connected_delay(nbr, desc->delays);
+  bound_delays(s, desc->delays);
   brick_layout(nbr, S / 3, s->perm, s->inv, s->bank);
   DeviceScenario& d = s->d;
   d.S = S;
@@ -1096,6 +1116,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   ALLOC(d.hslot, tiles * ct::kFwdTileVoxels * kOffsets);
   ALLOC(d.near, tiles * ct::kNearTiles);
   ALLOC(d.nhalo, tiles);
+  ALLOC(d.range, 2 * tiles);
   if (d.tiles > d.wave_grid) {
     unsigned char* rec = nullptr;
     ALLOC(rec, tiles * (int64_t)ct::wave_record_bytes());
@@ -1139,12 +1160,14 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
     }
   const HaloTables wave_halo = wave_job.get();
   const HaloTables sweep_halo = sweep_job.get();
+  s->halo_fits = *std::min_element(wave_halo.count.begin(), wave_halo.count.end()) >= 0;
   d.sweep_blocks = (int)sweep_start.size() - 1;
   r = r ? r : alloc(s, &d.sstart, (int64_t)sweep_start.size());
   r = r ? r : alloc(s, &d.shalo, (int64_t)sweep_halo.halo.size());
   r = r ? r : alloc(s, &d.shpos, (int64_t)sweep_halo.pos.size());
   r = r ? r : alloc(s, &d.shslot, (int64_t)sweep_halo.slot.size());
   r = r ? r : alloc(s, &d.snhalo, (int64_t)sweep_halo.count.size());
+  r = r ? r : alloc(s, &d.srange, 2 * (int64_t)sweep_halo.count.size());
   r = r ? r : upload(s, d.gains, h_gains.data(), sizeof(float) * S * kGainCols);
   r = r ? r : upload(s, d.nbr, h_nbr.data(), sizeof(int32_t) * V * kOffsets);
   r = r ? r : upload(s, d.coefs, h_coefs.data(), sizeof(float) * V * kOffsets);
@@ -1197,8 +1220,8 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   std::vector<float> nan_v((size_t)V, std::nanf(""));
   r = r ? r : upload(s, d.avg_delays, nan_v.data(), sizeof(float) * V);
   if (!r) {
-    cudaError_t e = ct::launch_min_delay(d, st);
-    if (e != cudaSuccess) r = cuda_fail(e, "min delay kernel");
+    cudaError_t e = ct::launch_delay_ranges(d, st);
+    if (e != cudaSuccess) r = cuda_fail(e, "delay range kernels");
   }
   if (!r && d.umma) {
     cudaError_t e = ct::umma_prepare(d, st);
@@ -1385,16 +1408,11 @@ int ct_run_epoch_host(ct_scn* scn, int64_t* batch_index, const int32_t* beat_ord
   CT_DEVICE_SCOPE(scn->ctx->device);
   DeviceScenario& d = scn->d;
   cudaStream_t st = scn->ctx->stream;
-  // the delays of connected pairs must be >= 1, as ct_write_field checks; their largest sizes the
-  // exchange ring
+  // the delays of connected pairs must be >= 1, as ct_write_field checks
   const std::vector<int32_t>& nbr = scn->nbr_host;
-  int64_t dmax = 1;
-  for (size_t i = 0; i < nbr.size(); ++i) {
-    if (nbr[i] < 0) continue;
-    if (delays[i] < 1)
+  for (size_t i = 0; i < nbr.size(); ++i)
+    if (nbr[i] >= 0 && delays[i] < 1)
       return fail(CT_ERR_INVALID_ARGUMENT, "delay %zu of a connected pair is %d; delays must be >= 1", i, delays[i]);
-    if (delays[i] > dmax) dmax = delays[i];
-  }
   int rc = ensure_xfer(scn);
   if (rc) return rc;
   const int64_t ng = d.S * kGainCols, nc = d.V * kOffsets;
@@ -1415,10 +1433,9 @@ int ct_run_epoch_host(ct_scn* scn, int64_t* batch_index, const int32_t* beat_ord
   if (measurements)
     CT_CUDA(cudaMemcpyAsync(d.meas, measurements, sizeof(float) * d.B * d.T * d.M, cudaMemcpyHostToDevice, st),
             "copy measurements");
-  CT_CUDA(ct::launch_min_delay(d, st), "min delay kernel");
+  CT_CUDA(ct::launch_delay_ranges(d, st), "delay range kernels");
   scn->launches += 4;
-  scn->dmax_bound = dmax;
-  scn->updates_at_read = -1;
+  bound_delays(scn, delays);
   rc = ct_run_epoch(scn, batch_index, beat_order, grad_mode, precision);
   if (rc) {
     cudaStreamSynchronize(st);
@@ -1445,7 +1462,7 @@ int ct_simulate(ct_scn* scn, float* measurements_out, float* states_out) try {
   int rc = prepare_exchange(scn);
   if (rc) return rc;
   for (int64_t beat = 0; beat < d.B; ++beat) {
-    CT_CUDA(run_phase(scn, CT_PHASE_FORWARD, 1,
+    CT_CUDA(run_phase(scn, CT_PHASE_FORWARD, d.routes == ct::kDecide ? 2 : 1,
                       [&] { return ct::launch_forward(d, scn->algo.maximum_regularization_threshold, st); }),
             "forward kernel");
     CT_CUDA(run_phase(scn, CT_PHASE_MEASURE, 2, [&] { return ct::launch_measure(d, beat, false, st); }),
@@ -1601,8 +1618,7 @@ int ct_write_field(ct_scn* scn, int field, const void* src, size_t nbytes) try {
         if (nbr[i] >= 0 && del[i] < 1)
           return fail(CT_ERR_INVALID_ARGUMENT, "delay %zu of a connected pair is %d; delays must be >= 1", i, del[i]);
       dst = d.delays;
-      scn->dmax_bound = max_connected_delay(nbr, del);
-      scn->updates_at_read = -1;
+      bound_delays(scn, del);
       break;
     }
     case CT_FIELD_MEASUREMENTS_ACTUAL: dst = d.meas; break;
@@ -1628,7 +1644,7 @@ int ct_write_field(ct_scn* scn, int field, const void* src, size_t nbytes) try {
     CT_CUDA(cudaMemcpyAsync(dst, staged.data(), nbytes, cudaMemcpyHostToDevice, scn->ctx->stream), "write field");
     CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "write field");
   }
-  if (field == CT_FIELD_DELAYS) CT_CUDA(ct::launch_min_delay(d, scn->ctx->stream), "min delay kernel");
+  if (field == CT_FIELD_DELAYS) CT_CUDA(ct::launch_delay_ranges(d, scn->ctx->stream), "delay range kernels");
   CT_CUDA(cudaStreamSynchronize(scn->ctx->stream), "write field");
   return CT_OK;
 } CT_CATCH
@@ -1866,6 +1882,8 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     wl.nphases = (int)b->beat_phases[(size_t)beat].size() - 1;
     wl.ntiles = (int)b->beat_tiles[(size_t)beat].size();
     wl.record = b->record;
+    wl.routes = ct::kStaged;
+    for (size_t i = 0; i < n; ++i) wl.routes = std::max(wl.routes, b->scns[i]->d.routes);
     wl.status = d0.status;
     wl.heartbeat = d0.heartbeat;
     const int wave_grid = std::min(b->grid, wl.ntiles);
@@ -1900,6 +1918,8 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     if (adjoint) {
       B_CUDA(batch_mark(b, CT_PHASE_MEASURE));
       wl.scns = b->adj_dev;
+      wl.routes = ct::kStaged;
+      for (size_t i = 0; i < n; ++i) wl.routes = std::max(wl.routes, b->scns[i]->d.rroutes);
       B_CUDA(ct::launch_wave(wl, true, wave_grid, st));
       B_CUDA(fork_side(b));
       for (size_t i = 0; i < n; ++i) {
@@ -1931,7 +1951,7 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     u.bias1 = u.bias2 = 1.0f;
     u.bias_dev = b->epoch_dev[i].bias;
     B_CUDA(ct::launch_update(d, u, ss));
-    if (!a.freeze_delays) B_CUDA(ct::launch_min_delay(d, ss));
+    if (!a.freeze_delays) B_CUDA(ct::launch_delay_ranges(d, ss));
     B_CUDA(ct::launch_batch_metrics_dev(d, &b->epoch_dev[i].batch_index, ss));
   }
   B_CUDA(join_side(b));

@@ -15,9 +15,14 @@ constexpr int kOffsets = 26;   // neighbour offsets per voxel
 constexpr int kGainCols = 78;  // 26 offsets x 3 neighbour components
 constexpr int kFwdTileVoxels = 32;  // voxels per tile of the recursions (consecutive in device order)
 constexpr int kFwdHaloMax = 192;    // halo slots of a tile; the last one stands for absent neighbours
+constexpr int kFwdRingSpread = 24;  // largest difference of delays that a tile's staged history holds
 constexpr int kNearTiles = 64;      // tiles of a halo that its staging warp can follow
 constexpr int kSweepVoxels = 8;     // most voxels per block of the gradient sweep
 constexpr int kSweepHaloMax = 112;  // halo slots of such a block
+
+// Which tiles a launch of the recursions meets: only such whose history fits the staged ring (the kernel without the direct
+// way), such and others (the kernel with both), or what the delays on the device say (both, one of which leaves).
+enum WaveRoutes { kStaged, kDecide, kEvery };
 
 // Counts the progress of a launch, so that a bounded wait can tell a long wait from a lost one.
 struct Heartbeat {
@@ -90,6 +95,7 @@ struct DeviceScenario {
   // steps that each tile has finished, 128 bytes apart
   uint4* xch;
   int xrows;             // power of two; grows with the delays
+  int routes, rroutes;   // WaveRoutes of the forward and of the adjoint's direction
   float4* record;        // packed registers of tiles that share a CTA, null when every tile has its own
   // halo tables: slots of each tile's (and each sweep block's) neighbourhood
   int32_t* halo;         // [tiles, kFwdHaloMax] device voxels of the halo in order, the last one repeated
@@ -97,12 +103,14 @@ struct DeviceScenario {
   int16_t* hslot;        // [tiles, 26 * kFwdTileVoxels] slot of each item's neighbour
   int32_t* near;         // [tiles, kNearTiles] tiles of the halo, the last one repeated
   int32_t* nhalo;        // [tiles] voxels of the halo, -1 if it is too large for the slots
+  int32_t* range;        // [tiles, 2] smallest and largest delay of the tile's connected items
   int sweep_blocks;      // blocks of the gradient sweep: consecutive voxels whose halo fits
   int32_t* sstart;       // [sweep blocks + 1] their first voxels
   int32_t* shalo;        // [sweep blocks, kSweepHaloMax]
   int16_t* shpos;
   int16_t* shslot;       // [sweep blocks, 26 * kSweepVoxels]
   int32_t* snhalo;       // [sweep blocks]
+  int32_t* srange;       // [sweep blocks, 2]
   // adjoint mode, allocated on first use
   int32_t* rev;          // [V,26] voxel whose offset n points at this voxel, -1 if none
   int32_t* rhalo;        // the tiles' halo tables of that direction
@@ -110,6 +118,7 @@ struct DeviceScenario {
   int16_t* rhslot;
   int32_t* rnear;
   int32_t* rnhalo;
+  int32_t* rrange;
   float* LX;             // [T,S] gradient of the loss with respect to the states
   // plain form (ct_plain.cu), allocated on first use
   float* plain_mreg;     // [S] maximum regularisation of the current step
@@ -136,7 +145,8 @@ struct WaveScn {
   const float* coefs;
   const int32_t* delays;
   const float* gains;
-  const int32_t* dmin;
+  const int32_t* dmin;   // the scenario's smallest and largest delay
+  const int32_t* range;  // [tiles, 2] those of each tile's items
   uint4* xch;
   float* rows;         // [T,S] finished rows: states, or their gradient
   // forward
@@ -163,6 +173,7 @@ struct WaveLaunch {
   const int* phase_begin;  // [nphases + 1] first tile of each phase, or null: one phase
   int nphases;
   int ntiles;
+  int routes;              // WaveRoutes
   float4* record;          // [ntiles] packed registers, null if no CTA owns two tiles of a phase
   int32_t* status;
   Heartbeat* heartbeat;
@@ -241,7 +252,9 @@ struct UpdateScalars {
   const float* bias_dev = nullptr;  // if set: {bias1, bias2} read on the device (graph replay)
 };
 cudaError_t launch_update(DeviceScenario& d, const UpdateScalars& s, cudaStream_t stream);
-cudaError_t launch_min_delay(DeviceScenario& d, cudaStream_t stream);
+// Delay ranges of the scenario, its tiles and its sweep blocks: after every change of the delays, and once the adjoint's
+// tables exist.
+cudaError_t launch_delay_ranges(DeviceScenario& d, cudaStream_t stream);
 
 // Voxel blocks of `words` 32-bit words between reference and device voxel order (perm[u] = the
 // reference voxel of device voxel u): gather dst[u] = src[perm[u]], else scatter dst[perm[u]] = src[u].

@@ -70,19 +70,41 @@ __global__ void roll_delays_kernel(float* __restrict__ coefs, int32_t* __restric
 }
 
 // dmin[0] = smallest, dmin[1] = largest delay of a connected (voxel, offset) pair
-__global__ void min_delay_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ delays, int64_t n,
-                                 int32_t* __restrict__ dmin) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Smallest and largest delay of the connected pairs: of each tile of the recursions (of its items in the adjoint's direction,
+// too, once its table exists), of each block of the sweep, and of all. One warp per tile or block; what bounds it is its
+// launch (a block's 832 entries are 26 coalesced loads). {INT_MAX, INT_MIN} where nothing is connected.
+struct DelayRanges {
+  const int32_t* nbr;
+  const int32_t* rev;  // null before the adjoint's tables are made
+  const int32_t* delays;
+  const int32_t* sstart;
+  int V, tiles, blocks;
+  int32_t *range, *srange, *rrange, *all;
+};
+__global__ void delay_ranges_kernel(const DelayRanges p) {
+  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32), lane = threadIdx.x & 31;
+  if (w >= p.tiles + p.blocks + (p.rev ? p.tiles : 0)) return;
+  const bool sweep = w >= p.tiles && w < p.tiles + p.blocks, back = w >= p.tiles + p.blocks;
+  const int b = sweep ? w - p.tiles : back ? w - p.tiles - p.blocks : w;
+  const int v0 = sweep ? p.sstart[b] : b * kFwdTileVoxels, v1 = sweep ? p.sstart[b + 1] : min(p.V, v0 + kFwdTileVoxels);
+  const int32_t* src = back ? p.rev : p.nbr;
   int32_t lo = INT_MAX, hi = INT_MIN;
-  if (i < n && nbr[i] >= 0) lo = hi = delays[i];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    lo = min(lo, __shfl_down_sync(0xffffffffu, lo, off));
-    hi = max(hi, __shfl_down_sync(0xffffffffu, hi, off));
+  for (int i = v0 * kOffsets + lane; i < v1 * kOffsets; i += 32) {
+    const int32_t j = src[i];
+    if (j < 0) continue;
+    const int32_t d = p.delays[back ? j * kOffsets + i % kOffsets : i];
+    lo = min(lo, d);
+    hi = max(hi, d);
   }
-  if ((threadIdx.x & 31) == 0 && lo != INT_MAX) {
-    atomicMin(dmin, lo);
-    atomicMax(dmin + 1, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane != 0) return;
+  int32_t* out = (sweep ? p.srange : back ? p.rrange : p.range) + 2 * b;
+  out[0] = lo;
+  out[1] = hi;
+  if (!sweep && !back && lo <= hi) {
+    atomicMin(p.all, lo);
+    atomicMax(p.all + 1, hi);
   }
 }
 
@@ -305,10 +327,11 @@ cudaError_t launch_update(DeviceScenario& d, const UpdateScalars& s, cudaStream_
   return cudaGetLastError();
 }
 
-cudaError_t launch_min_delay(DeviceScenario& d, cudaStream_t stream) {
+cudaError_t launch_delay_ranges(DeviceScenario& d, cudaStream_t stream) {
   set_min_max_kernel<<<1, 1, 0, stream>>>(d.dmin);
-  const int64_t n = d.V * kOffsets;
-  min_delay_kernel<<<blocks(n, 256), 256, 0, stream>>>(d.nbr, d.delays, n, d.dmin);
+  const DelayRanges p = {d.nbr, d.rev, d.delays, d.sstart, (int)d.V, d.tiles, d.sweep_blocks, d.range, d.srange, d.rrange, d.dmin};
+  const int64_t warps = (int64_t)d.tiles * (d.rev ? 2 : 1) + d.sweep_blocks;
+  delay_ranges_kernel<<<blocks(32 * warps, 256), 256, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

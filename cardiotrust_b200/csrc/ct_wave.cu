@@ -40,12 +40,18 @@
 //   * History. The staging warp copies the tile's halo (at most kHaloSlots - 1 voxels) row by row into
 //     a ring of kRingRows rows in shared memory. A voxel's slot is chosen so that (slot mod 8) =
 //     (2 y + z) mod 8: the eight lanes of a quarter warp are 4 x 2 neighbouring (y, z), so their 16-byte
-//     reads fall into eight different bank groups whatever the offset. Where the spread of delays does
-//     not fit the ring, or a halo is too large, the compute warps poll the exchange ring themselves.
+//     reads fall into eight different bank groups whatever the offset. Where the spread of a tile's delays does
+//     not fit the ring, or its halo is too large, the compute warps poll the exchange ring themselves. That way has a
+//     kernel of its own (ANY), launched where such tiles may occur: the polling loops in every warp's code cost the staged
+//     tiles 15 % (instruction fetch; as a second copy of the visit behind a call, which saves 60 registers in local
+//     memory each time, the polled tiles took twice as long). The delays change on the device; where the host's bounds do not
+//     tell, both kernels are launched and the one that is not meant leaves (4 us). Shell of 47,264 voxels, T = 1,000, a
+//     slow layer of 100 to 173 steps and a fast one of 2 to 4: forward 30.3 ms with every tile polling, 22.1 so; with
+//     the slow layer alone 20.4 and 12.0.
 //   * Two steps are handed over together where no delay is shorter (one set of waits and arrivals for both: 1.33 ->
 //     1.25 ms on the 20x20x20 cuboid), each step's sums as soon as they are there (1.25 -> 1.18 ms with the
 //     smaller staging batches).
-//   * A CTA that visits several tiles in turn, min(dmin, 64) steps each, keeps their
+//   * A CTA that visits several tiles in turn, min(dmin, 64) steps each (the scenario's smallest delay), keeps their
 //     registers in packed records (60 floats per lane) between visits. All rows that a visit reads belong to
 //     earlier blocks of steps, so its staging warp waits once for the progress that the tiles around have
 //     published and starts all copies (64x64x48 shell, T = 4,000: 27.4 -> 24.3 ms). Work is ordered by (phase, block
@@ -59,6 +65,8 @@
 // 24.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 23 on the first and the last, where the
 // inbox form took 11.2 and 145 with the gradients in it.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "ct_internal.cuh"
 #include "ct_sync.cuh"
@@ -83,6 +91,8 @@ constexpr int kMaxVisit = 64;            // steps per visit of a CTA that owns s
 constexpr int kPerLane = kHaloSlots / (32 * kStageWarps);  // halo voxels per lane of a staging warp
 constexpr int kSmemPerCta = 233472 / 2 - 1024;  // two CTAs per SM
 constexpr unsigned long long kWaitNs = 2000000000ull;
+// the rows of one group of steps and of the batch that is staged beside it
+static_assert(kFwdRingSpread + 2 + kGroup + kBatch <= kRingRows, "a tile's history fits the ring");
 static_assert(kTile == 32 && kLastItems == 2 && kHaloSlots % (32 * kStageWarps) == 0, "lane = voxel");
 
 struct WaveSmem {
@@ -219,24 +229,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, WaveSm
 // Phase parity of the n-th use (0, 1, ...) of a ring entry at position pos.
 __device__ __forceinline__ uint32_t row_parity(int pos) { return (uint32_t)(pos / kRingRows) & 1u; }
 
-// Delay range of a scenario.
+// Delay range of a tile's own items: one slow or fast layer of tissue leaves the other tiles their pairs and rings.
 struct Geometry {
   int dmin, dmax;
   bool pairs; // no step reads the step before: two steps may be handed over together
-  int visit;  // steps per visit of a CTA with several tiles (never more than dmin)
   bool ring;  // the rows of one step and of two batches fit the shared ring
 };
-__device__ __forceinline__ Geometry geometry(const WaveScn& p) {
+__device__ __forceinline__ Geometry geometry(const WaveScn& p, int tile) {
   Geometry g;
-  g.dmin = p.dmin[0];
-  g.dmax = p.dmin[1];
+  g.dmin = p.range[2 * tile];
+  g.dmax = p.range[2 * tile + 1];
   if (g.dmin > g.dmax) g.dmin = g.dmax = 1;  // no connected pair: nothing is read
-  if (g.dmin < 1) g.dmin = 1;
-  if (g.dmax < g.dmin) g.dmax = g.dmin;
   g.pairs = g.dmin >= kGroup;
-  g.visit = min(g.dmin, kMaxVisit);
-  g.ring = (long long)g.dmax - g.dmin + 2 + kGroup + 4 <= kRingRows;
+  g.ring = (long long)g.dmax - g.dmin <= kFwdRingSpread;
   return g;
+}
+// Steps per visit of a CTA with several tiles: the scenario's smallest delay at most, so that every row that a visit
+// reads belongs to an earlier block of steps.
+__device__ __forceinline__ int visit_steps(const WaveScn& p) {
+  return p.dmin[0] > p.dmin[1] ? 1 : min(p.dmin[0], kMaxVisit);
 }
 
 // The CTA's visits, in the order that every warp of it follows.
@@ -271,7 +282,7 @@ __device__ __forceinline__ bool next_visit(const WaveSmem& sm, const WaveLaunch&
       v.t0 = 0;
       v.t1 = p.T;
       if (v.whole) return true;
-      const int len = geometry(p).visit;
+      const int len = visit_steps(p);
       if (w.block > (p.T - 1) / len) continue;
       w.live = true;
       v.t0 = w.block * len;
@@ -330,6 +341,7 @@ __device__ __forceinline__ int copy_rows(const uint4* const (&from)[kPerLane], c
 // the 20x20x20 cuboid; always 2: 1.20, and 7 % slower on the shell). Loads into
 // registers were slower: their round trips to L2 do not overlap (the loads of two batches share
 // scoreboards), 2,250 cycles per two rows.
+template <bool ANY>
 __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L) {
   const int lane = threadIdx.x & 31;
   Walk walk;
@@ -346,10 +358,10 @@ __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L)
   const uint32_t ring = smem_u32(&sm.ring[0][0]);
   while (next_visit(sm, L, walk, v)) {
     const WaveScn& p = scenario_of(sm, L, v.scn);
-    const Geometry geo = geometry(p);
     const int tile = v.v0 / kTile;
+    const Geometry geo = geometry(p, tile);
     const int nh = p.nhalo[tile];
-    if (!geo.ring || nh < 0) continue;
+    if (ANY && (!geo.ring || nh < 0)) continue;
     int r = v.t0 - geo.dmax - 1;
     const int end = v.t1 - geo.dmin;  // rows [r, end)
     const int after = pos + end - r;
@@ -451,13 +463,13 @@ struct Tile {
   float ctrl[3], threshold, mse, reg;
   int V, S, T, mask, ntiles, lane;
   int floor, need;  // ring positions of rows t - dmax - 1 and t - dmin, minus t
-  bool live;
+  bool live, ring;
 };
 
 // The items' delayed rows for steps [t, t + N), from the shared ring or polled from the exchange ring.
-template <int N, bool RING, int NI>
+template <int N, bool ANY, int NI>
 __device__ __forceinline__ bool fetch(WaveSmem& sm, const WaveLaunch& L, const Tile<NI>& k, int t, float (&x)[N][NI][3]) {
-  if (RING) {
+  if (!ANY || k.ring) {
     const int pos = k.need + t + N - 1;  // rows are staged in order
     if (!mbar_wait(&sm.full[pos & (kRingRows - 1)], row_parity(pos), sm, L)) return false;
 #pragma unroll
@@ -473,28 +485,33 @@ __device__ __forceinline__ bool fetch(WaveSmem& sm, const WaveLaunch& L, const T
   }
   bool good = true;
 #pragma unroll
-  for (int s = 0; s < N; ++s)
+  for (int s = 0; s < N; ++s) {
+    int spins = 0;
+    unsigned long long since = 0;
+    for (;;) {
+      uint4 e[NI];
+      bool there = true;
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int r = t + s + k.off[i];
-      x[s][i][0] = x[s][i][1] = x[s][i][2] = 0.0f;
-      if ((int)k.at[i] >= 0 && r >= 0) {
-        const uint4* q = k.src + (size_t)(r & k.mask) * k.V + k.at[i];
-        uint4 e = ld_entry(q);
-        int spins = 0;
-        unsigned long long since = 0;
-        while (e.w != (uint32_t)r + 1u) {
-          if (!go_on(sm, L, spins, since, 63)) {
-            good = false;
-            break;
-          }
-          e = ld_entry(q);
-        }
-        x[s][i][0] = __uint_as_float(e.x);
-        x[s][i][1] = __uint_as_float(e.y);
-        x[s][i][2] = __uint_as_float(e.z);
+      for (int i = 0; i < NI; ++i) {
+        const int r = t + s + k.off[i];
+        const bool reads = (int)k.at[i] >= 0 && r >= 0;
+        e[i] = ld_entry(reads ? k.src + (size_t)(r & k.mask) * k.V + k.at[i] : k.src);
+        if (!reads) e[i] = make_uint4(0, 0, 0, (uint32_t)r + 1u);
+        there = there && e[i].w == (uint32_t)r + 1u;
+      }
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        x[s][i][0] = __uint_as_float(e[i].x);
+        x[s][i][1] = __uint_as_float(e[i].y);
+        x[s][i][2] = __uint_as_float(e[i].z);
+      }
+      if (there) break;
+      if (!go_on(sm, L, spins, since, 63)) {
+        good = false;
+        break;
       }
     }
+  }
   return __all_sync(0xffffffffu, good);
 }
 
@@ -522,10 +539,10 @@ __device__ __forceinline__ void read_own(WaveSmem& sm, const Tile<NI>& k, int t,
 }
 
 // Steps [t, t + N) of one warp's items. False: a wait ran out.
-template <int N, int NI, int POS, bool ADJ, bool RING>
+template <int N, int NI, int POS, bool ADJ, bool ANY>
 __device__ __forceinline__ bool compute_group(WaveSmem& sm, const WaveLaunch& L, Tile<NI>& k, Cursor& cur, int w, int t) {
   float x[N][NI][3];
-  if (!fetch<N, RING>(sm, L, k, t, x)) return false;
+  if (!fetch<N, ANY>(sm, L, k, t, x)) return false;
   // the items' chains; x becomes the all-pass outputs (forward)
   float sum[N][3];  // adjoint: the items' contributions
 #pragma unroll
@@ -652,7 +669,7 @@ __device__ __forceinline__ bool compute_group(WaveSmem& sm, const WaveLaunch& L,
     __syncwarp();
     if (k.lane == 0) mbar_arrive(&sm.taken[w - 1][buf]);
     // every warp has read what steps before t + N need: no later step reads rows before t + N - dmax - 1
-    if (POS == kLast && RING && k.lane < N) mbar_arrive(&sm.empty[(k.floor + t + k.lane) & (kRingRows - 1)]);
+    if (POS == kLast && (!ANY || k.ring) && k.lane < N) mbar_arrive(&sm.empty[(k.floor + t + k.lane) & (kRingRows - 1)]);
   }
   ++cur.group;
   if (POS == kLast && (cur.group & 127) == 0 && k.lane == 0) atomicAdd(&L.heartbeat->count, 1u);
@@ -660,7 +677,7 @@ __device__ __forceinline__ bool compute_group(WaveSmem& sm, const WaveLaunch& L,
 }
 
 // One visit of a compute warp: NI offsets from 4 w for steps [v.t0, v.t1). False: a wait ran out.
-template <int NI, int POS, bool ADJ, bool RING>
+template <int NI, int POS, bool ADJ, bool ANY>
 __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L, const WaveScn& p, const Geometry& geo,
                                               const Visit& v, Cursor& cur, int w) {
   const int lane = threadIdx.x & 31;
@@ -674,6 +691,7 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
   k.S = 3 * p.V;
   k.T = p.T;
   k.live = lane < min(kTile, k.V - v.v0);
+  k.ring = !ANY || (geo.ring && p.nhalo[tile] >= 0);
   const int vox = v.v0 + (k.live ? lane : 0);
   k.mask = p.xrows - 1;
   k.src = p.xch;
@@ -707,7 +725,7 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
       const float* gr = p.gains + (size_t)3 * (ADJ ? (ok ? src : 0) : vox) * kGainCols + 3 * (n0 + i);
       k.c[i] = ok ? p.coefs[own] : 0.0f;
       k.off[i] = -(ok ? p.delays[own] : geo.dmin);
-      k.at[i] = RING ? (ok ? (uint32_t)p.hslot[((size_t)tile * kTile + lane) * kOffsets + n0 + i] : (uint32_t)kZeroSlot)
+      k.at[i] = k.ring ? (ok ? (uint32_t)p.hslot[((size_t)tile * kTile + lane) * kOffsets + n0 + i] : (uint32_t)kZeroSlot)
                      : (uint32_t)src;
 #pragma unroll
       for (int b = 0; b < 3; ++b) {
@@ -760,7 +778,7 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
   const int base = k.floor + geo.dmax + 1;
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
-    if (RING) {
+    if (k.ring) {
       k.at[i] = smem_u32(&sm.ring[0][k.at[i]]);
       k.off[i] += base;
     }
@@ -768,7 +786,7 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
   }
   if (!ADJ) {
     float x[1][NI][3];
-    if (!fetch<1, RING>(sm, L, k, v.t0 - 1, x)) return false;
+    if (!fetch<1, ANY>(sm, L, k, v.t0 - 1, x)) return false;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
 #pragma unroll
@@ -776,31 +794,32 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
   }
 
   int t = v.t0, said = v.t0;
+  const int step = visit_steps(p);
   // last warp: the rows before t are finished, for the staging warps that ask for the progress of tiles
   auto say = [&](bool now) {
-    if (POS != kLast || !v.shared || (!now && t - said < geo.visit)) return;
+    if (POS != kLast || !v.shared || (!now && t - said < step)) return;
     said = t;
     __syncwarp();
     if (lane == 0) st_progress(progress_of(p, tile), t);
   };
   if (geo.pairs)
     for (; t + kGroup <= v.t1;) {
-      if (!compute_group<kGroup, NI, POS, ADJ, RING>(sm, L, k, cur, w, t)) return false;
+      if (!compute_group<kGroup, NI, POS, ADJ, ANY>(sm, L, k, cur, w, t)) return false;
       t += kGroup;
       say(false);
     }
   for (; t < v.t1;) {
-    if (!compute_group<1, NI, POS, ADJ, RING>(sm, L, k, cur, w, t)) return false;
+    if (!compute_group<1, NI, POS, ADJ, ANY>(sm, L, k, cur, w, t)) return false;
     ++t;
     say(false);
   }
   say(true);
   if (POS == kLast) {
     asm volatile("cp.async.wait_all;" ::: "memory");  // the next visit reuses the buffers
-    if (RING && lane == 0)  // the visit's remaining rows
+    if (k.ring && lane == 0)  // the visit's remaining rows
       for (int q = 0; q < geo.dmax - geo.dmin + 1; ++q) mbar_arrive(&sm.empty[(k.floor + v.t1 + q) & (kRingRows - 1)]);
   }
-  if (RING) cur.pos += v.t1 - v.t0 + geo.dmax - geo.dmin + 1;
+  if (k.ring) cur.pos += v.t1 - v.t0 + geo.dmax - geo.dmin + 1;
   if (v.t1 < k.T) {
     save(0, (3 * NI + 3) / 4);
   } else if (!ADJ && k.live) {
@@ -815,30 +834,19 @@ __device__ __forceinline__ bool compute_visit(WaveSmem& sm, const WaveLaunch& L,
   }
   return true;
 }
-template <int NI, int POS, bool ADJ>
-__device__ __noinline__ bool direct_visit(WaveSmem& sm, const WaveLaunch& L, const WaveScn& p, Geometry geo,
-                                          Visit v, Cursor cur, int w) {
-  return compute_visit<NI, POS, ADJ, false>(sm, L, p, geo, v, cur, w);
-}
-
-template <int NI, int POS, bool ADJ>
+template <int NI, int POS, bool ADJ, bool ANY>
 __device__ __forceinline__ void compute(WaveSmem& sm, const WaveLaunch& L, int w) {
   Walk walk;
   Visit v;
   Cursor cur;
   while (next_visit(sm, L, walk, v)) {
     const WaveScn& p = scenario_of(sm, L, v.scn);
-    const Geometry geo = geometry(p);
-    if (geo.ring && p.nhalo[v.v0 / kTile] >= 0) {
-      if (!compute_visit<NI, POS, ADJ, true>(sm, L, p, geo, v, cur, w)) return;
-    } else {
-      if (!direct_visit<NI, POS, ADJ>(sm, L, p, geo, v, cur, w)) return;  // by value: nothing escapes to memory
-      cur.group += geo.pairs ? (v.t1 - v.t0) / kGroup + (v.t1 - v.t0) % kGroup : v.t1 - v.t0;
-    }
+    const Geometry geo = geometry(p, v.v0 / kTile);
+    if (!compute_visit<NI, POS, ADJ, ANY>(sm, L, p, geo, v, cur, w)) return;
   }
 }
 
-template <bool ADJ>
+template <bool ADJ, bool ANY>
 __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant__ WaveLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WaveSmem& sm = *reinterpret_cast<WaveSmem*>(smem_raw);
@@ -857,37 +865,42 @@ __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant
     if (!L.scns) sm.single = L.single;
   }
   __syncthreads();
-  // Every exchange ring must hold the rows that a reader may still want, or all of them: when a tile writes step t, its
-  // neighbours have finished step t - dmax at least, and from there on they read back to t - 2 dmax.
+  // Which of the two kernels is meant: where the host cannot know it is launched with both, and one leaves. And every
+  // exchange ring must hold the rows that a reader may still want, or all of them: when a tile writes step t, its neighbours
+  // have finished step t - dmax at least, and from there on they read back to t - 2 dmax.
+  bool apart = false, fits = true;
   for (int s = 0; s < L.nscn; ++s) {
     const WaveScn& p = scenario_of(sm, L, s);
-    const Geometry geo = geometry(p);
-    if (p.xrows < p.T && 2ll * geo.dmax + 2 > p.xrows) {  // every CTA leaves here
-      if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(L.status, 0, (int32_t)CT_ERR_NOT_SUPPORTED);
-      return;
-    }
+    if (p.dmin[0] > p.dmin[1]) continue;  // nothing is connected
+    apart = apart || (long long)p.dmin[1] - p.dmin[0] > kFwdRingSpread;
+    fits = fits && (p.xrows >= p.T || 2ll * p.dmin[1] + 2 <= p.xrows);
+  }
+  if (L.routes == kDecide && apart != ANY) return;
+  if (!fits || (L.routes == kStaged && apart)) {  // every CTA leaves here
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(L.status, 0, (int32_t)CT_ERR_NOT_SUPPORTED);
+    return;
   }
   const int w = threadIdx.x / 32;
   if (w >= kComputeWarps)
-    stage_history(sm, L);
+    stage_history<ANY>(sm, L);
   else if (w == 0)
-    compute<kItems, kFirst, ADJ>(sm, L, w);
+    compute<kItems, kFirst, ADJ, ANY>(sm, L, w);
   else if (w < kComputeWarps - 1)
-    compute<kItems, kMiddle, ADJ>(sm, L, w);
+    compute<kItems, kMiddle, ADJ, ANY>(sm, L, w);
   else
-    compute<kLastItems, kLast, ADJ>(sm, L, w);
+    compute<kLastItems, kLast, ADJ, ANY>(sm, L, w);
   asm volatile("cp.async.wait_all;" ::: "memory");  // no thread leaves before its copies have landed, after a lost wait either
 }
+
+const void* const kKernels[4] = {(const void*)wave_kernel<false, false>, (const void*)wave_kernel<true, false>,
+                                 (const void*)wave_kernel<false, true>, (const void*)wave_kernel<true, true>};
 
 bool configure(int device) {
   static bool done[128] = {};
   if (device < 0 || device >= 128) return false;
   if (!done[device]) {
-    if (cudaFuncSetAttribute(wave_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WaveSmem)) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(wave_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WaveSmem)) !=
-            cudaSuccess)
-      return false;
+    for (const void* f : kKernels)
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WaveSmem)) != cudaSuccess) return false;
     done[device] = true;
   }
   return true;
@@ -897,12 +910,14 @@ bool configure(int device) {
 
 int wave_capacity(int device) {
   configure(device);
-  int sms = 0, f = 0, a = 0;
+  int sms = 0, per_sm = 1 << 10;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, wave_kernel<false>, kThreads, sizeof(WaveSmem));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, wave_kernel<true>, kThreads, sizeof(WaveSmem));
-  const int per_sm = f < a ? f : a;
-  return sms * (per_sm < 1 ? 1 : per_sm);
+  for (const void* f : kKernels) {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, kThreads, sizeof(WaveSmem));
+    per_sm = std::min(per_sm, n);
+  }
+  return sms * std::max(per_sm, 1);
 }
 
 size_t wave_record_bytes() { return sizeof(float4) * kComputeWarps * 15 * 32; }
@@ -923,6 +938,7 @@ WaveScn wave_scenario(const DeviceScenario& d, bool adjoint, const WaveScalars& 
   a.delays = d.delays;
   a.gains = d.gains;
   a.dmin = d.dmin;
+  a.range = adjoint ? d.rrange : d.range;
   a.xch = d.xch;
   a.rows = adjoint ? d.LX : d.X;
   a.ctrl = d.ctrl;
@@ -945,8 +961,11 @@ cudaError_t launch_wave(const WaveLaunch& launch, bool adjoint, int grid, cudaSt
   if (!configure(device)) return cudaErrorInvalidValue;
   WaveLaunch l = launch;
   void* args[] = {&l};
-  return launch_cooperative(adjoint ? (const void*)wave_kernel<true> : (const void*)wave_kernel<false>, grid, kThreads,
-                            args, sizeof(WaveSmem), stream);
+  err = cudaSuccess;
+  for (int any = 0; any < 2 && err == cudaSuccess; ++any)
+    if (launch.routes == kDecide || (launch.routes == kEvery) == (any == 1))
+      err = launch_cooperative(kKernels[2 * any + (adjoint ? 1 : 0)], grid, kThreads, args, sizeof(WaveSmem), stream);
+  return err;
 }
 
 // Empty the exchange ring (tag 0: no step) and the tiles' progress.
@@ -967,6 +986,7 @@ cudaError_t launch_single(DeviceScenario& d, bool adjoint, const WaveScalars& s,
   l.nphases = 1;
   l.ntiles = (int)d.tiles;
   l.record = d.record;
+  l.routes = adjoint ? d.rroutes : d.routes;
   l.status = d.status;
   l.heartbeat = d.heartbeat;
   return launch_wave(l, adjoint, d.wave_grid, stream);

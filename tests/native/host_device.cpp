@@ -9,6 +9,7 @@
 #include <dlfcn.h>
 #include <pthread.h>
 
+#include <algorithm>
 #include <cerrno>
 #include <cstdlib>
 #include <cstring>
@@ -32,6 +33,7 @@ struct Recorded {
 };
 struct Graph {
   std::vector<Recorded> launches;
+  std::vector<std::pair<const ct::DeviceScenario*, const void*>> ranges;  // delay ranges, and the reverse table they covered
 };
 
 std::map<char*, size_t> g_blocks;
@@ -45,6 +47,7 @@ Graph* g_capturing = nullptr;
 std::vector<float> g_times;
 size_t g_time = 0;
 std::vector<int> g_orders;  // phases of every batched forward that ran
+int g_last_routes = 0;      // ct::WaveRoutes of the last forward
 int g_routes[2][3];         // tiles of the last forward and adjoint: followed by progress, by tags, polled directly
 
 void wrong(const std::string& what) {
@@ -61,16 +64,24 @@ void need(const void* p, size_t bytes, const char* what) {
   if (!live(p, bytes)) wrong(std::string(what) + " is not in a live block");
 }
 
-// The rows that readers may still want: every step, or twice the largest delay and two.
-void check_ring(const ct::WaveScn& p, const char* form) {
+// The rows that readers may still want: every step, or twice the largest delay and two. And a kernel that takes the delays
+// and halos that it meets.
+void check_ring(const ct::WaveScn& p, int routes, const char* form) {
   need(p.xch, sizeof(uint4) * ((size_t)p.xrows * p.V + 8 * (size_t)p.ntiles), form);
   if (!live(p.src, sizeof(int32_t) * p.V * ct::kOffsets) || !live(p.delays, sizeof(int32_t) * p.V * ct::kOffsets)) {
     wrong(std::string(form) + ": tables are not in a live block");
     return;
   }
-  int64_t dmax = 1;
+  int64_t dmin = INT32_MAX, dmax = 1;
   for (int64_t i = 0; i < (int64_t)p.V * ct::kOffsets; ++i)
-    if (p.src[i] >= 0 && p.delays[i] > dmax) dmax = p.delays[i];
+    if (p.src[i] >= 0) {
+      const int64_t delay = p.delays[p.rows ? p.src[i] * ct::kOffsets + i % ct::kOffsets : i];
+      dmin = std::min(dmin, delay);
+      dmax = std::max(dmax, delay);
+    }
+  if (routes == ct::kStaged && dmax - dmin > ct::kFwdRingSpread) wrong(std::string(form) + ": delays too far apart for the staged ring");
+  for (int t = 0; t < p.ntiles; ++t)
+    if (routes != ct::kEvery && p.nhalo[t] < 0) wrong(std::string(form) + ": a halo too large for the staged ring");
   if (p.xrows < p.T && p.xrows < 2 * dmax + 2) wrong(std::string(form) + ": the exchange ring is too short");
 }
 void check(const Recorded& r) {
@@ -88,7 +99,7 @@ void check(const Recorded& r) {
     for (int t = begin; t < end; ++t)
       if (l.tiles[t].x < 0 || l.tiles[t].x >= l.nscn) wrong("a tile of no scenario");
   }
-  for (int i = 0; i < l.nscn; ++i) check_ring(l.scns[i], r.adjoint ? "batched adjoint" : "batched forward");
+  for (int i = 0; i < l.nscn; ++i) check_ring(l.scns[i], l.routes, r.adjoint ? "batched adjoint" : "batched forward");
 }
 
 void count_routes(int (&n)[3], const ct::DeviceScenario& d, const int32_t* nhalo, const int32_t* near) {
@@ -130,6 +141,7 @@ int host_device_report(char* out, int len) {  // and forget it
   g_report.clear();
   return n;
 }
+int host_device_last_routes() { return g_last_routes; }
 void host_device_routes(int* out) { std::memcpy(out, g_routes, sizeof(g_routes)); }
 int host_device_phases(int* out, int len) {  // phases of the batched forwards since the last call
   const int n = (int)g_orders.size();
@@ -215,6 +227,8 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned lon
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
   for (const Recorded& r : ((Graph*)e)->launches) check(r);
+  for (const auto& r : ((Graph*)e)->ranges)
+    if (r.first->rev != r.second) wrong("a captured update leaves the adjoint's delay ranges behind");
   return cudaSuccess;
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) {
@@ -249,6 +263,8 @@ WaveScn wave_scenario(const DeviceScenario& d, bool adjoint, const WaveScalars&,
   a.delays = d.delays;
   a.xch = d.xch;
   a.part = part;
+  a.nhalo = adjoint ? d.rnhalo : d.nhalo;
+  a.rows = adjoint ? d.LX : nullptr;  // tells the directions apart here
   return a;
 }
 cudaError_t launch_wave(const WaveLaunch& l, bool adjoint, int grid, cudaStream_t) {
@@ -260,13 +276,14 @@ cudaError_t launch_wave(const WaveLaunch& l, bool adjoint, int grid, cudaStream_
   return cudaSuccess;
 }
 cudaError_t launch_forward(DeviceScenario& d, float, cudaStream_t) {
-  check_ring(wave_scenario(d, false, WaveScalars{}, nullptr), "forward");
+  g_last_routes = d.routes;
+  check_ring(wave_scenario(d, false, WaveScalars{}, nullptr), d.routes, "forward");
   count_routes(g_routes[0], d, d.nhalo, d.near);
   if (d.tiles > d.wave_grid) need(d.record, (size_t)d.tiles * kRecordBytes, "forward record");
   return cudaSuccess;
 }
 cudaError_t launch_adjoint_states(DeviceScenario& d, const WaveScalars&, cudaStream_t) {
-  check_ring(wave_scenario(d, true, WaveScalars{}, nullptr), "adjoint");
+  check_ring(wave_scenario(d, true, WaveScalars{}, nullptr), d.rroutes, "adjoint");
   count_routes(g_routes[1], d, d.rnhalo, d.rnear);
   return cudaSuccess;
 }
@@ -274,7 +291,8 @@ cudaError_t clear_exchange(DeviceScenario& d, cudaStream_t) {
   if (!g_capturing) need(d.xch, sizeof(uint4) * (size_t)d.xrows * d.V, "exchange ring");
   return cudaSuccess;
 }
-cudaError_t launch_min_delay(DeviceScenario& d, cudaStream_t) {
+cudaError_t launch_delay_ranges(DeviceScenario& d, cudaStream_t) {
+  if (g_capturing) g_capturing->ranges.push_back({&d, d.rev});
   d.dmin[0] = INT32_MAX;
   d.dmin[1] = INT32_MIN;
   for (int64_t i = 0; i < d.V * kOffsets; ++i)

@@ -24,8 +24,8 @@ T* device(const std::vector<T>& v) {
 }  // namespace
 
 enum Form {
-  kAll,        // every tile runs: status 0
-  kStaged,     // one tile of two, its history staged
+  kAllTiles,        // every tile runs: status 0
+  kStagedTile,  // one tile of two, its history staged
   kDirect,     // the same with delays too far apart for the staging ring
   kShared,     // two tiles of three in one CTA, which asks for the progress of the third
   kShortRing,  // every tile runs, in a ring that could lose rows before they are read
@@ -73,6 +73,9 @@ extern "C" int wave_waits(int form, int* status, float* ms) {
   p.delays = device(delays);
   p.gains = device(std::vector<float>((size_t)S * ct::kGainCols, 0.01f));
   p.dmin = device(dmin);
+  std::vector<int32_t> range;
+  for (int t = 0; t < tiles; ++t) range.insert(range.end(), dmin.begin(), dmin.end());
+  p.range = device(range);
   const size_t ring = sizeof(uint4) * ((size_t)p.xrows * V + 8 * tiles);
   p.xch = reinterpret_cast<uint4*>(device(std::vector<char>(ring, 0)));
   p.rows = device(std::vector<float>((size_t)T * S));
@@ -84,18 +87,19 @@ extern "C" int wave_waits(int form, int* status, float* ms) {
   p.threshold = 1.0f;
   std::vector<int2> list;
   for (int t = 0; t < tiles; ++t)
-    if (form == kAll || form == kShortRing || t + 1 < tiles) list.push_back(make_int2(0, t * kTile));
+    if (form == kAllTiles || form == kShortRing || t + 1 < tiles) list.push_back(make_int2(0, t * kTile));
   ct::WaveLaunch l{};
   l.scns = device(std::vector<ct::WaveScn>(1, p));
   l.nscn = 1;
   l.tiles = device(list);
   l.phase_begin = device(std::vector<int>{0, (int)list.size()});
   l.nphases = 1;
+  l.routes = wide ? ct::kDecide : ct::kStaged;
   l.ntiles = (int)list.size();
   l.record = reinterpret_cast<float4*>(device(std::vector<char>(list.size() * ct::wave_record_bytes(), 0)));
   l.status = device(std::vector<int32_t>(1, 0));
   l.heartbeat = device(std::vector<ct::Heartbeat>(1));
-  const void* all[] = {p.src, p.halo, p.hpos, p.hslot, p.near, p.nhalo, p.coefs, p.delays, p.gains, p.dmin, p.xch, p.rows, p.ctrl,
+  const void* all[] = {p.src, p.halo, p.hpos, p.hslot, p.near, p.nhalo, p.coefs, p.delays, p.gains, p.dmin, p.range, p.xch, p.rows, p.ctrl,
                        p.u, p.ap, p.ap_last, p.part, l.scns, l.tiles, l.phase_begin, l.record, l.status, l.heartbeat};
   for (const void* q : all)
     if (!q) return __LINE__;

@@ -1,6 +1,6 @@
 """Tiles on different routes of the recursion kernel in one launch: followed by the progress of the tiles around, by the
 tags of their rows, and polled directly, alone on a CTA or several in turn; pairs of steps across the visits of a
-CTA; a batch's small members in the places that a large one leaves free.
+CTA; layers of tissue with other delays; a batch's small members in the places that a large one leaves free.
 
 States are bit-identical to the f32 oracle. Gradients lie within 1e-5 of the oracle (adjoint: f64; reference: the f32 loop),
 ten times the rounding of sums of this length in f32."""
@@ -42,9 +42,13 @@ def scenario(shape, steps, lo, hi, how=None, beats=1):
                            pulse_onset=0, pulse_sigma_samples=2.0, seed=13)
     scn = sc.build(spec)
     rng = np.random.default_rng(steps)
-    osi = rewired(scn.model, rng, how) if how else scn.model.output_state_indices
+    osi = rewired(scn.model, rng, how) if how in ("exchanged", "far") else scn.model.output_state_indices
     connected = osi[::3, ::3] >= 0
     drawn = rng.integers(lo, hi + 1, size=connected.shape)
+    if how == "layers":  # a slow layer and a fast one, as tissues with other velocities make them
+        z = np.arange(connected.shape[0]) % shape[2]
+        drawn[z // 4 == 1] = rng.integers(60, 121, size=drawn.shape)[z // 4 == 1]
+        drawn[z // 4 == 3] = rng.integers(1, 4, size=drawn.shape)[z // 4 == 3]
     drawn[0, :], drawn[-1, :] = lo, hi  # both ends occur
     delays = np.where(connected, drawn, scn.model.delays).astype(np.int32)
     gain = rng.normal(0.0, 0.06, size=osi.shape)  # damped, so that 26 connections do not grow
@@ -62,6 +66,8 @@ CASES = {
     "exchanged_short": (SHAPE, 33, 1, 4, "exchanged"),
     "far": (SHAPE, 47, 6, 11, "far"),
     "far_short": (SHAPE, 33, 2, 4, "far"),
+    "layers": (SHAPE, 150, 6, 12, "layers"),
+    "layers_small": ((7, 6, 19), 260, 6, 12, "layers"),
     "smallest_3": (SHAPE, 41, 3, 9),
     "smallest_7": (SHAPE, 50, 7, 12),
 }

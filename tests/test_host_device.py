@@ -190,6 +190,45 @@ def test_batch_after_an_exchange_ring_that_could_not_grow(host, ctx):
     assert host.report() == ""
 
 
+def test_batch_updates_know_the_tables_that_came_later(host, ctx):
+    """A reference batch is captured before a member runs its first adjoint epoch by itself: the batch's updates from then on
+    cover the delay ranges of that direction."""
+    from cardiotrust_b200 import algorithm as alg
+
+    engines, batch = _batch(ctx, MEMBERS)
+    for e in engines:
+        e.set_freeze(False, False)
+        _with_delays(e, 9)  # short enough for the rings to stay as they are
+    batch.run_epoch()
+    engines[1].run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=0)
+    batch.run_epoch()
+    assert host.report() == ""
+
+
+def test_kernel_follows_the_delays(host, ctx):
+    """The recursions' kernel without the direct way runs alone while the delays surely fit the staged ring: exact after a
+    write, one step wider on both sides with every update whose read-back has not landed (here: none does). Otherwise
+    both are launched, and the device decides."""
+    from cardiotrust_b200 import algorithm as alg
+
+    eng = _engine(ctx, (4, 4, 4), 300, algorithm=alg.Algorithm(freeze_delays=False))
+    small = _engine(ctx, (4, 4, 4), 200)
+    batch = alg.EpochBatch(ctx, [eng, small], precision=alg.Precision.Fp32)
+    OPEN.append(batch)
+    STAGED, DECIDE = 0, 1
+    for largest, routes in ((8 + 24, STAGED), (8 + 25, DECIDE), (20, STAGED)):
+        _with_delays(eng, largest)
+        eng.simulate()
+        assert host.lib.host_device_last_routes() == routes, largest
+        batch.run_epoch()  # captured again where the kernel changes
+    _with_delays(eng, 20)
+    for update in range(10):  # delays 8 to 20: bounds 7 to 21, ..., 1 to 28, where the spread has passed 24
+        eng.run_epoch(0, precision=0)
+        assert host.lib.host_device_last_routes() == (DECIDE if update > 6 else STAGED), update
+    batch.run_epoch()
+    assert host.report() == ""
+
+
 def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
     """An update moves no delay past 1,000, but leaves a larger one that was written where it is: the ring that is
     sized afterwards holds the rows that it reads."""
