@@ -48,6 +48,12 @@ def lib():
         _lib.oracle_from_coef_to_samples.argtypes = [ctypes.c_float]
         _lib.oracle_set_threads.argtypes = [ctypes.c_int]
         _lib.oracle_max_threads.restype = ctypes.c_int
+        # without argument types ctypes passes an address as a 32-bit int, which holds for a low heap only
+        ptr, i64, f32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_float
+        _lib.oracle_sgd_f32.argtypes = [ptr, ptr, i64, f32, i64]
+        _lib.oracle_adam_f32.argtypes = [ptr, ptr, ptr, ptr, i64, i64, f32, i64]
+        _lib.oracle_roll_delays_f32.argtypes = [ptr, ptr, i64]
+        _lib.oracle_adam_bias_f32.argtypes = [i64, ptr]
     return _lib
 
 
