@@ -164,6 +164,17 @@ def test_autotune_keeps_the_record_of_its_choice(host, ctx):
     assert host.report() == ""
 
 
+def test_autotune_times_every_arrangement_once(host, ctx):
+    """The two epochs that warm up an adjoint batch count for no arrangement, however fast they were."""
+    from cardiotrust_b200 import algorithm as alg
+
+    engines, batch = _batch(ctx, MEMBERS, grad_mode=alg.GradMode.Adjoint)
+    host.times(1.0, 1.0, 5.0, 4.0, 4.5)
+    assert batch.autotune()["tile_order"] == 1
+    assert int(batch.batch_indices[0]) == 5
+    assert host.report() == ""
+
+
 def _with_delays(engine, largest):
     d = engine.read("delays")
     d[:] = 8
