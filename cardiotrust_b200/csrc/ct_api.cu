@@ -70,7 +70,7 @@ struct ct_scn {
   cudaEvent_t dmax_event = nullptr;
   int64_t updates = 0;          // updates that may roll delays, enqueued so far
   int64_t updates_at_read = -1; // `updates` when the pending read-back was enqueued (-1: none)
-  // bumped whenever the algorithm settings or the exchange ring change (batches re-capture their epoch graph)
+  // bumped whenever the algorithm settings, the exchange ring or the adjoint's tables change (batches re-capture their epoch graph)
   uint64_t config_gen = 0;
   // Device voxel order: device voxel u holds reference voxel perm[u]; inv is the inverse.
   std::vector<int32_t> perm, inv;
@@ -342,7 +342,6 @@ int prepare_exchange(ct_scn* s) {
   const bool wide = s->dmax_bound - s->dmin_bound > ct::kFwdRingSpread;
   const int routes = !s->halo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
   const int rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
-  if (d.routes != routes || d.rroutes != rroutes) s->config_gen += 1;
   d.routes = routes;
   d.rroutes = rroutes;
   int64_t want = 8, all = 8;
@@ -1753,6 +1752,10 @@ struct ct_batch {
   cudaGraphExec_t exec = nullptr;
   bool use_graph = true;
   std::vector<uint64_t> captured_gen;
+  // WaveRoutes of the captured epoch, which covers those of every member. It stays where a member's go down again: the
+  // bounds behind them widen with every update that the host is ahead of the device, and would have an epoch captured
+  // again, with a wait for the device, each time that they pass the staged ring's limit and come back.
+  int routes = ct::kStaged, rroutes = ct::kStaged;
   int64_t graph_kernels = 0;
   int tile_order = 0;  // tuned choice (ct_batch_autotune): how the tiles are arranged in phases
   // optional per-phase timing (eager launches, CUDA events on the context stream)
@@ -1882,8 +1885,7 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     wl.nphases = (int)b->beat_phases[(size_t)beat].size() - 1;
     wl.ntiles = (int)b->beat_tiles[(size_t)beat].size();
     wl.record = b->record;
-    wl.routes = ct::kStaged;
-    for (size_t i = 0; i < n; ++i) wl.routes = std::max(wl.routes, b->scns[i]->d.routes);
+    wl.routes = b->routes;
     wl.status = d0.status;
     wl.heartbeat = d0.heartbeat;
     const int wave_grid = std::min(b->grid, wl.ntiles);
@@ -1918,8 +1920,7 @@ cudaError_t batch_enqueue_epoch(ct_batch* b) {
     if (adjoint) {
       B_CUDA(batch_mark(b, CT_PHASE_MEASURE));
       wl.scns = b->adj_dev;
-      wl.routes = ct::kStaged;
-      for (size_t i = 0; i < n; ++i) wl.routes = std::max(wl.routes, b->scns[i]->d.rroutes);
+      wl.routes = b->rroutes;
       B_CUDA(ct::launch_wave(wl, true, wave_grid, st));
       B_CUDA(fork_side(b));
       for (size_t i = 0; i < n; ++i) {
@@ -1964,6 +1965,7 @@ int batch_prepare(ct_batch* b) {
   cudaStream_t st = b->ctx->stream;
   const size_t n = b->scns.size();
   bool stale = b->exec == nullptr && b->use_graph;
+  int routes = ct::kStaged, rroutes = ct::kStaged;
   for (size_t i = 0; i < n; ++i) {
     ct_scn* s = b->scns[i];
     if (b->grad_mode == CT_GRAD_ADJOINT) {
@@ -1973,8 +1975,13 @@ int batch_prepare(ct_batch* b) {
     int rc = prepare_exchange(s);
     if (rc) return rc;
     if (b->captured_gen.size() == n && b->captured_gen[i] != s->config_gen) stale = true;
+    routes = std::max(routes, s->d.routes);
+    rroutes = std::max(rroutes, s->d.rroutes);
   }
+  stale = stale || routes > b->routes || rroutes > b->rroutes;
   if (!stale && b->captured_gen.size() == n) return CT_OK;
+  b->routes = routes;
+  b->rroutes = rroutes;
   // descriptors
   std::vector<ct::WaveScn> fa(n), aa(n);
   const bool adjoint = b->grad_mode == CT_GRAD_ADJOINT;

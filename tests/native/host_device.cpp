@@ -17,6 +17,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../cardiotrust_b200/csrc/ct_internal.cuh"
@@ -47,6 +48,8 @@ Graph* g_capturing = nullptr;
 std::vector<float> g_times;
 size_t g_time = 0;
 std::vector<int> g_orders;  // phases of every batched forward that ran
+bool g_landed = false;  // what was recorded on a stream has happened
+int g_captures = 0;     // epochs captured since the last count
 int g_last_routes = 0;      // ct::WaveRoutes of the last forward
 int g_routes[2][3];         // tiles of the last forward and adjoint: followed by progress, by tags, polled directly
 
@@ -141,6 +144,8 @@ int host_device_report(char* out, int len) {  // and forget it
   g_report.clear();
   return n;
 }
+void host_device_landed(int on) { g_landed = on != 0; }
+int host_device_captures() { return std::exchange(g_captures, 0); }
 int host_device_last_routes() { return g_last_routes; }
 void host_device_routes(int* out) { std::memcpy(out, g_routes, sizeof(g_routes)); }
 int host_device_phases(int* out, int len) {  // phases of the batched forwards since the last call
@@ -207,13 +212,14 @@ cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = (cudaEvent_t)1, cudaSu
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventQuery(cudaEvent_t) { return cudaErrorNotReady; }
+cudaError_t cudaEventQuery(cudaEvent_t) { return g_landed ? cudaSuccess : cudaErrorNotReady; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
   *ms = g_time < g_times.size() ? g_times[g_time++] : 1.0f;
   return cudaSuccess;
 }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
   g_capturing = new Graph;
+  ++g_captures;
   return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {

@@ -240,6 +240,25 @@ def test_kernel_follows_the_delays(host, ctx):
     assert host.report() == ""
 
 
+def test_batch_keeps_its_graph_while_the_bounds_come_and_go(host, ctx):
+    """Delays 8 to 31 fit the staged ring. While an update's read-back is under way the bounds are wider and do not; the
+    batch captures once for that, not with every change."""
+    from cardiotrust_b200 import algorithm as alg
+
+    engines, batch = _batch(ctx, MEMBERS[1:])
+    for e in engines:
+        e.set_freeze(False, False)
+        _with_delays(e, 8 + 23)
+    batch.run_epoch()
+    host.lib.host_device_captures()
+    for epoch in range(14):
+        host.lib.host_device_landed(epoch // 2 % 2)
+        batch.run_epoch()
+    host.lib.host_device_landed(0)
+    assert host.lib.host_device_captures() == 1
+    assert host.report() == ""
+
+
 def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
     """An update moves no delay past 1,000, but leaves a larger one that was written where it is: the ring that is
     sized afterwards holds the rows that it reads."""
