@@ -59,6 +59,9 @@ struct ct_scn {
   std::vector<int32_t> nbr_dev;   // neighbour table in device order (adjoint reverse table)
   std::vector<uint8_t> bank;      // (2 y + z) mod 8 of each device voxel's grid coordinates
   bool symmetric = true;          // a voxel's neighbours all have it as a neighbour
+  // Which tiles see how far their readers are (prepare_exchange), in the forward's and the adjoint's direction: all of
+  // them by the rows that they read themselves, all by rows that they stage for it, or not all.
+  enum Sight { kByRows, kByStaging, kNot } sight = kByRows, rsight = kByRows;
   // Bounds of the delays of connected pairs: exact after creation and delay writes, one wider
   // per update that rolls delays (roll_delays moves a delay by at most one, and none past 1,000). They size the
   // exchange ring and choose the recursions' kernel without reading the device.
@@ -334,8 +337,8 @@ int prepare_sliced(ct_scn* s) {
 
 // The exchange ring of the recursion kernels. A tile overwrites the entry of step t - xrows when it
 // finishes step t; by then every tile that it reads has finished step t - dmax and so reads no row before
-// t - 2 dmax any more, provided that the tiles that read it are among those that it reads. Without
-// that symmetry the ring holds every step of the beat.
+// t - 2 dmax any more, provided that the tiles that read it are among those that it reads or stages a voxel
+// of. Where they are not, the ring holds every step of the beat.
 int prepare_exchange(ct_scn* s) {
   DeviceScenario& d = s->d;
   refresh_delay_bounds(s);
@@ -347,7 +350,10 @@ int prepare_exchange(ct_scn* s) {
   int64_t want = 8, all = 8;
   while (want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30)) want <<= 1;
   while (all < d.T) all <<= 1;
-  if (!s->symmetric || want > all) want = all;
+  auto bounded = [](ct_scn::Sight sight, int kernel) {
+    return sight == ct_scn::kByRows || (sight == ct_scn::kByStaging && kernel == ct::kStaged);
+  };
+  if (!bounded(s->sight, routes) || !bounded(s->rsight, rroutes) || want > all) want = all;
   if (d.xch && d.xrows >= want) return CT_OK;
   CT_CUDA(cudaStreamSynchronize(s->ctx->stream), "exchange ring");
   release(s, d.xch);
@@ -368,10 +374,13 @@ int prepare_exchange(ct_scn* s) {
 struct HaloTables {
   std::vector<int32_t> halo, count, near;  // near: the blocks (of TV voxels) that the source voxels lie in
   std::vector<int16_t> pos, slot;
+  bool all = true;  // every voxel of `more` has its place
 };
-// start: each block's first voxel and, at the end, V; empty for blocks of TV voxels.
+// start: each block's first voxel and, at the end, V; empty for blocks of TV voxels. more: voxels that a block's halo takes
+// in although no item reads them, where they fit; without entries if there are none.
+using Followed = std::vector<std::vector<int32_t>>;
 HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_t>& bank, int64_t V, int TV, int HM,
-                       const std::vector<int32_t>& start = {}) {
+                       const std::vector<int32_t>& start = {}, const Followed& more = {}) {
   HaloTables t;
   const int64_t blocks = start.empty() ? (V + TV - 1) / TV : (int64_t)start.size() - 1;
   t.halo.assign((size_t)(blocks * HM), 0);
@@ -394,7 +403,15 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
     }
     if ((int)list.size() > HM - 1) {
       t.count[(size_t)b] = -1;
+      t.all = t.all && (more.empty() || more[(size_t)b].empty());
       continue;
+    }
+    if (!more.empty()) {
+      const std::vector<int32_t>& extra = more[(size_t)b];
+      if (list.size() + extra.size() < (size_t)HM)
+        list.insert(list.end(), extra.begin(), extra.end());
+      else
+        t.all = false;
     }
     t.count[(size_t)b] = (int32_t)list.size();
     if (list.empty()) continue;
@@ -439,6 +456,34 @@ HaloTables build_halos(const std::vector<int32_t>& src, const std::vector<uint8_
       if (src[(size_t)i] >= 0) t.slot[(size_t)(b * TV * kOffsets + i - u0 * kOffsets)] = place[(size_t)src[(size_t)i]];
   }
   return t;
+}
+
+// For each tile a voxel of every tile that reads it and that it does not read itself: by following that voxel's rows it
+// knows how far its reader is. Empty where no tile needs one. (A table that lets the activation pass in one direction only
+// has such tiles. Without this its ring had to hold the whole beat, 3.1 GB for 47,264 voxels and 4,000 steps.)
+Followed unseen_readers(const std::vector<int32_t>& src, int64_t V) {
+  const int TV = ct::kFwdTileVoxels;
+  const int64_t tiles = (V + TV - 1) / TV;
+  std::vector<std::vector<int32_t>> reads((size_t)tiles);
+  std::vector<int32_t> seen((size_t)tiles, -1);
+  for (int64_t i = 0; i < V * kOffsets; ++i) {
+    const int32_t b = (int32_t)(i / kOffsets / TV), a = src[(size_t)i] < 0 ? b : src[(size_t)i] / TV;
+    if (a == b || seen[(size_t)a] == b) continue;
+    seen[(size_t)a] = b;
+    reads[(size_t)b].push_back(a);
+  }
+  Followed out((size_t)tiles);
+  bool any = false;
+  for (int64_t b = 0; b < tiles; ++b)
+    for (int32_t a : reads[(size_t)b])
+      if (std::find(reads[(size_t)a].begin(), reads[(size_t)a].end(), (int32_t)b) == reads[(size_t)a].end()) {
+        out[(size_t)a].push_back((int32_t)(b * TV));
+        any = true;
+      }
+  return any ? out : Followed{};
+}
+ct_scn::Sight sight_of(const Followed& readers, const HaloTables& t) {
+  return readers.empty() ? ct_scn::kByRows : t.all ? ct_scn::kByStaging : ct_scn::kNot;
 }
 
 // Consecutive voxels in blocks of at most TV, a block ending early where its halo would pass HM - 1 voxels. (Uncut, one block
@@ -500,7 +545,9 @@ int prepare_adjoint(ct_scn* s) {
                     "adjoint mode: two voxels reach the same neighbour along one offset (not a lattice)");
       slot = (int32_t)v;
     }
-  const HaloTables t = build_halos(rev, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax);
+  const Followed readers = s->symmetric ? Followed{} : unseen_readers(rev, V);
+  const HaloTables t = build_halos(rev, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax, {}, readers);
+  s->rsight = sight_of(readers, t);
   s->rhalo_fits = *std::min_element(t.count.begin(), t.count.end()) >= 0;
   int rc = alloc(s, &d.rhalo, (int64_t)t.halo.size());
   if (!rc) rc = alloc(s, &d.rhpos, (int64_t)t.pos.size());
@@ -1157,7 +1204,12 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
       const int32_t* row = h_nbr.data() + (size_t)w * kOffsets;
       if (std::find(row, row + kOffsets, (int32_t)u) == row + kOffsets) s->symmetric = false;
     }
-  const HaloTables wave_halo = wave_job.get();
+  HaloTables wave_halo = wave_job.get();
+  if (!s->symmetric) {
+    const Followed readers = unseen_readers(h_nbr, V);
+    if (!readers.empty()) wave_halo = build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax, {}, readers);
+    s->sight = sight_of(readers, wave_halo);
+  }
   const HaloTables sweep_halo = sweep_job.get();
   s->halo_fits = *std::min_element(wave_halo.count.begin(), wave_halo.count.end()) >= 0;
   d.sweep_blocks = (int)sweep_start.size() - 1;

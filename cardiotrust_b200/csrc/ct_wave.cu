@@ -229,6 +229,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, WaveSm
 // Phase parity of the n-th use (0, 1, ...) of a ring entry at position pos.
 __device__ __forceinline__ uint32_t row_parity(int pos) { return (uint32_t)(pos / kRingRows) & 1u; }
 
+// Steps per visit of a CTA with several tiles: the scenario's smallest delay at most, so that every row that a visit
+// reads belongs to an earlier block of steps.
+__device__ __forceinline__ int visit_steps(const WaveScn& p) {
+  return p.dmin[0] > p.dmin[1] ? 1 : min(p.dmin[0], kMaxVisit);
+}
+
 // Delay range of a tile's own items: one slow or fast layer of tissue leaves the other tiles their pairs and rings.
 struct Geometry {
   int dmin, dmax;
@@ -239,17 +245,11 @@ __device__ __forceinline__ Geometry geometry(const WaveScn& p, int tile) {
   Geometry g;
   g.dmin = p.range[2 * tile];
   g.dmax = p.range[2 * tile + 1];
-  if (g.dmin > g.dmax) g.dmin = g.dmax = 1;  // no connected pair: nothing is read
+  if (g.dmin > g.dmax) g.dmin = g.dmax = visit_steps(p);  // no connected pair: only rows of its readers are followed, if any
   g.pairs = g.dmin >= kGroup;
   g.ring = (long long)g.dmax - g.dmin <= kFwdRingSpread;
   return g;
 }
-// Steps per visit of a CTA with several tiles: the scenario's smallest delay at most, so that every row that a visit
-// reads belongs to an earlier block of steps.
-__device__ __forceinline__ int visit_steps(const WaveScn& p) {
-  return p.dmin[0] > p.dmin[1] ? 1 : min(p.dmin[0], kMaxVisit);
-}
-
 // The CTA's visits, in the order that every warp of it follows.
 struct Visit {
   int tile, scn, v0, t0, t1;

@@ -16,6 +16,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <set>
 #include <string>
 #include <utility>
 #include <vector>
@@ -85,7 +86,20 @@ void check_ring(const ct::WaveScn& p, int routes, const char* form) {
   if (routes == ct::kStaged && dmax - dmin > ct::kFwdRingSpread) wrong(std::string(form) + ": delays too far apart for the staged ring");
   for (int t = 0; t < p.ntiles; ++t)
     if (routes != ct::kEvery && p.nhalo[t] < 0) wrong(std::string(form) + ": a halo too large for the staged ring");
-  if (p.xrows < p.T && p.xrows < 2 * dmax + 2) wrong(std::string(form) + ": the exchange ring is too short");
+  if (p.xrows >= p.T) return;
+  if (p.xrows < 2 * dmax + 2) wrong(std::string(form) + ": the exchange ring is too short");
+  // rows are written again: a tile that is read knows how far its reader is, by its items (polled) or its halo (staged)
+  std::vector<std::set<int>> reads((size_t)p.ntiles), sees((size_t)p.ntiles);
+  for (int64_t i = 0; i < (int64_t)p.V * ct::kOffsets; ++i)
+    if (p.src[i] >= 0) reads[(size_t)(i / ct::kOffsets / ct::kFwdTileVoxels)].insert(p.src[i] / ct::kFwdTileVoxels);
+  for (int t = 0; t < p.ntiles; ++t) {
+    sees[(size_t)t] = reads[(size_t)t];
+    for (int i = 0; routes == ct::kStaged && i < p.nhalo[t]; ++i)
+      sees[(size_t)t].insert(p.halo[(size_t)t * ct::kFwdHaloMax + i] / ct::kFwdTileVoxels);
+  }
+  for (int t = 0; t < p.ntiles; ++t)
+    for (int a : reads[(size_t)t])
+      if (a != t && !sees[(size_t)a].count(t)) wrong(std::string(form) + ": a tile overwrites rows that are still read");
 }
 void check(const Recorded& r) {
   const ct::WaveLaunch& l = r.launch;
@@ -270,6 +284,7 @@ WaveScn wave_scenario(const DeviceScenario& d, bool adjoint, const WaveScalars&,
   a.xch = d.xch;
   a.part = part;
   a.nhalo = adjoint ? d.rnhalo : d.nhalo;
+  a.halo = adjoint ? d.rhalo : d.halo;
   a.rows = adjoint ? d.LX : nullptr;  // tells the directions apart here
   return a;
 }

@@ -1,6 +1,6 @@
 """Tiles on different routes of the recursion kernel in one launch: followed by the progress of the tiles around, by the
 tags of their rows, and polled directly, alone on a CTA or several in turn; pairs of steps across the visits of a
-CTA; layers of tissue with other delays; a batch's small members in the places that a large one leaves free.
+CTA; layers of tissue with other delays; tiles that are read by tiles that they do not read; a batch's small members in the places that a large one leaves free.
 
 States are bit-identical to the f32 oracle. Gradients lie within 1e-5 of the oracle (adjoint: f64; reference: the f32 loop),
 ten times the rounding of sums of this length in f32."""
@@ -35,6 +35,15 @@ def rewired(p, rng, how):
     return np.where(np.repeat(np.repeat(nbr, 3, axis=0), 3, axis=1) >= 0, to, -1).astype(np.int32)
 
 
+def one_way(p, shape, ends):
+    """Voxels from the third brick on read none before it, or, as ends of the activation's way, none at all."""
+    osi = p.output_state_indices.copy()
+    x = np.unravel_index(np.arange(osi.shape[0] // 3), shape)[0]
+    behind = np.repeat(x >= 8, 3)
+    osi[behind[:, None] & ((np.repeat(x, 3)[np.maximum(osi, 0)] < 8) | ends)] = -1
+    return osi
+
+
 def scenario(shape, steps, lo, hi, how=None, beats=1):
     from cardiotrust_b200 import scenario as sc
 
@@ -43,6 +52,8 @@ def scenario(shape, steps, lo, hi, how=None, beats=1):
     scn = sc.build(spec)
     rng = np.random.default_rng(steps)
     osi = rewired(scn.model, rng, how) if how in ("exchanged", "far") else scn.model.output_state_indices
+    if how in ("one_way", "ends"):
+        osi = one_way(scn.model, shape, how == "ends")
     connected = osi[::3, ::3] >= 0
     drawn = rng.integers(lo, hi + 1, size=connected.shape)
     if how == "layers":  # a slow layer and a fast one, as tissues with other velocities make them
@@ -68,6 +79,10 @@ CASES = {
     "far_short": (SHAPE, 33, 2, 4, "far"),
     "layers": (SHAPE, 150, 6, 12, "layers"),
     "layers_small": ((7, 6, 19), 260, 6, 12, "layers"),
+    "one_way": (SHAPE, 150, 4, 9, "one_way"),
+    "one_way_small": ((13, 6, 7), 300, 4, 9, "one_way"),
+    "one_way_ends": (SHAPE, 150, 4, 9, "ends"),
+    "one_way_ends_small": ((13, 6, 7), 300, 4, 9, "ends"),
     "smallest_3": (SHAPE, 41, 3, 9),
     "smallest_7": (SHAPE, 50, 7, 12),
 }

@@ -97,6 +97,32 @@ def test_rewired_cases_meet_every_route(host, ctx, case):
     assert sum(n[:3]) == 318 and host.report() == ""
 
 
+@pytest.mark.parametrize("case", ["one_way", "one_way_small", "one_way_ends", "one_way_ends_small"])
+def test_one_way_tables_keep_a_short_exchange_ring(host, ctx, case):
+    """Tiles that do not read their readers follow a voxel of theirs, so that the ring need not hold the whole beat, in either
+    direction; it does once the delays may not fit the staged ring."""
+    import test_gpu_routes as routes
+
+    from cardiotrust_b200 import algorithm as alg
+
+    shape, steps, lo, hi, how = routes.CASES[case]
+    live = []
+    for how in (None, how):
+        scn = routes.scenario(shape, steps, lo, hi, how)
+        scn.measurements = np.zeros((1, steps, scn.num_sensors), np.float32)
+        before = host.live()
+        OPEN.append(alg.EpochEngine.from_scenario(ctx, scn, algorithm=alg.Algorithm(freeze_delays=False)))
+        OPEN[-1].run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=0)
+        live.append(host.live() - before)
+    rows = 16 * int(np.prod(shape))
+    assert live[1] - live[0] < 8 * rows
+    assert host.report() == ""
+    _with_delays(OPEN[-1], 8 + 25)
+    OPEN[-1].run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=0)
+    assert host.live() - before - live[1] > (steps - 64) * rows
+    assert host.report() == ""
+
+
 def _engine(ctx, shape, steps, **kw):
     from cardiotrust_b200 import algorithm as alg
     from cardiotrust_b200 import scenario as sc
