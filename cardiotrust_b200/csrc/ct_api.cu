@@ -335,7 +335,7 @@ int prepare_sliced(ct_scn* s) {
   return CT_OK;
 }
 
-// The exchange ring of the recursion kernels. A tile overwrites the entry of step t - xrows when it
+// The kernels that the delays and halos call for, and the exchange ring of the recursions. A tile overwrites the entry of step t - xrows when it
 // finishes step t; by then every tile that it reads has finished step t - dmax and so reads no row before
 // t - 2 dmax any more, provided that the tiles that read it are among those that it reads or stages a voxel
 // of. Where they are not, the ring holds every step of the beat.
@@ -347,6 +347,7 @@ int prepare_exchange(ct_scn* s) {
   const int rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
   d.routes = routes;
   d.rroutes = rroutes;
+  d.sweep_any = s->dmax_bound - s->dmin_bound > ct::kSweepRingSpread;
   int64_t want = 8, all = 8;
   while (want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30)) want <<= 1;
   while (all < d.T) all <<= 1;
@@ -1808,6 +1809,7 @@ struct ct_batch {
   // bounds behind them widen with every update that the host is ahead of the device, and would have an epoch captured
   // again, with a wait for the device, each time that they pass the staged ring's limit and come back.
   int routes = ct::kStaged, rroutes = ct::kStaged;
+  std::vector<char> sweep_any;  // the same of each member's gradient sweep
   int64_t graph_kernels = 0;
   int tile_order = 0;  // tuned choice (ct_batch_autotune): how the tiles are arranged in phases
   // optional per-phase timing (eager launches, CUDA events on the context stream)
@@ -2029,11 +2031,14 @@ int batch_prepare(ct_batch* b) {
     if (b->captured_gen.size() == n && b->captured_gen[i] != s->config_gen) stale = true;
     routes = std::max(routes, s->d.routes);
     rroutes = std::max(rroutes, s->d.rroutes);
+    if (b->sweep_any.size() == n && !b->sweep_any[i] && s->d.sweep_any) stale = true;
   }
   stale = stale || routes > b->routes || rroutes > b->rroutes;
   if (!stale && b->captured_gen.size() == n) return CT_OK;
   b->routes = routes;
   b->rroutes = rroutes;
+  b->sweep_any.assign(n, 0);
+  for (size_t i = 0; i < n; ++i) b->sweep_any[i] = b->scns[i]->d.sweep_any;
   // descriptors
   std::vector<ct::WaveScn> fa(n), aa(n);
   const bool adjoint = b->grad_mode == CT_GRAD_ADJOINT;

@@ -32,8 +32,13 @@
 // e / 8, and a voxel's slot has (slot mod 8) = (2 y + z) mod 8, so a quarter warp's eight entries lie in
 // eight different bank groups. The factor fma(mr, mse/M, maxreg * reg) is the same for a voxel's 26
 // offsets and is formed once per (voxel, step). Blocks end early where their halo would not fit. Where a block's delays
-// spread too far for the ring its items read the rows from global memory (a slow layer of tissue in a shell of 47,264
-// voxels, T = 1,000: 8.24 ms with every block doing so, 4.82 with that layer's blocks only).
+// spread too far for the ring (a tissue of less than 0.25 m/s at 2.5 mm and 2 kHz) its items read the rows from global
+// memory, two steps ahead; that way has a kernel of its own (ANY), launched where the host's bounds do not rule it out, and a
+// loop with registers of its own. 20x20x20 cuboid, T = 1,000, 0.2 m/s everywhere: 1.42 ms with each read waiting for its
+// answer, 1.35 one step ahead, 1.14 so, 1.05 four ahead, which is slower where the rows are scattered (shell of 47,264 voxels, T =
+// 500, each pair's delay drawn from 8 to 60: 4.23, 4.01, 3.66 and 3.89; by cp.async into the ring's place, eight ahead,
+// 1.21 and 4.76); one thread per item took 1.19 and 3.07 there. A slow layer in that shell: 2.42, now 2.34. Without
+// that way the other blocks' kernel is smaller: 0.787 -> 0.777 on the cuboid at 0.6 m/s.
 // Three CTAs per SM with 80 registers and 112 slots beat four with 72 and 96, which keep some values in local
 // memory and cut more blocks. 20x20x20 cuboid, T = 2,000, textbook: 2.28 ms with one thread per item gathering single
 // floats through L1, 1.83 with four CTAs and blocks of exactly 8 voxels, 1.66 with addresses that do not
@@ -41,6 +46,8 @@
 // per thread in paired multiply-adds, 16 voxels per block: 1.77 and 7.6; a pair of FP32 operations with three
 // operands takes 2.4 cycles. Two mbarriers instead of the CTA barrier, so that warps may be steps apart: 1.70.)
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "ct_internal.cuh"
 
@@ -53,6 +60,8 @@ constexpr int kSlots = kSweepHaloMax;      // per ring row; the last one stays z
 constexpr int kRows = 32;   // power of two
 constexpr int kRowBytes = kSlots * 16;
 constexpr int kChunk = 8;   // steps staged together
+constexpr int kAhead = 2;   // steps that a block without a ring reads ahead, divides kChunk
+static_assert(kSweepRingSpread + 2 * kChunk <= kRows && kChunk % kAhead == 0, "a block's history fits the ring");
 constexpr int kCols = (3 * (kSlots - 1) + kThreads - 1) / kThreads;  // halo words per thread and row
 
 enum { kTextbook = 0, kSimple = 1, kAdjoint = 2 };
@@ -70,6 +79,7 @@ struct SweepArgs {
   float* dC;
   float* fir;
   float* iir;
+  int32_t* status;
   int blocks;
   const int32_t* start;  // [blocks + 1] first voxel of each block
   const int32_t* halo;   // [blocks, kSlots] voxels of the halo
@@ -79,6 +89,7 @@ struct SweepArgs {
   const int32_t* range;  // [blocks, 2] smallest and largest delay of the block's connected items
   DeriveScalars s;
   int simple;
+  bool any;
 };
 
 struct SweepSmem {
@@ -163,8 +174,8 @@ __device__ __forceinline__ void sweep_step(Item& k, const float (&in)[3], const 
   }
 }
 
-// MODE, and which of the two gradients are wanted.
-template <int MODE, bool GAINS, bool COEFS>
+// MODE, which of the two gradients are wanted, and whether blocks may come whose delays do not fit the ring.
+template <int MODE, bool GAINS, bool COEFS, bool ANY>
 __global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_constant__ SweepArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
@@ -192,7 +203,12 @@ __global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_co
   if (dmin > dmax) dmin = dmax = 1;  // no connected pair
   if (dmin < 1) dmin = 1;
   const int nh = p.nhalo[blockIdx.x];
-  const bool ring = (int64_t)dmax - dmin + 2 * kChunk <= kRows;
+  const bool fits = (int64_t)dmax - dmin <= kSweepRingSpread;
+  if (!ANY && !fits) {
+    if (tid == 0) atomicCAS(p.status, 0, (int32_t)CT_ERR_NOT_SUPPORTED);
+    return;
+  }
+  const bool ring = !ANY || fits;
   const int late = k.valid ? d - dmin : 0;  // how far behind the newest row the item reads
   // from here on t >= d holds (for absent items too: their stored delay gates nothing but zeros)
   const int settled = MODE == kTextbook ? max(dmax, d) : dmax;
@@ -305,77 +321,99 @@ __global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_co
   factors(0, 0);
   // address of the neighbour in ring row 0; without a ring its column of X
   const uint32_t slot = ring ? ring0 + 16u * (uint32_t)p.hslot[(size_t)blockIdx.x * kThreads + vl * kOffsets + n] : 3u * (uint32_t)max(nb, 0);
-  int buf = 0;  // t0 / kChunk mod 3
-  for (int t0 = 0; t0 < T; t0 += kChunk) {
-    cp_async_wait<0>();
-    // this chunk's history, factors and the next chunk's own rows are there for all; the previous chunk's
-    // buffers and the ring rows older than t0 - dmax are free (kRows >= spread + 2 chunks)
-    __syncthreads();
-    const int next = buf == 2 ? 0 : buf + 1, after = next == 2 ? 0 : next + 1;
-    stage_history(t0 + kChunk);
-    stage_own(t0 + 2 * kChunk, after);
-    cp_async_commit();
-    if (t0 + kChunk < T) factors(next, ((t0 / kChunk) + 1) & 1);
-    const float4* rows = &sm.row[buf][0][vl];
-    const float4* facs = &sm.q[(t0 / kChunk) & 1][0][vl];
-    const int tn = min(kChunk, T - t0);
-    auto one = [&](int s, const float (&in)[3], bool on) {
-      const float4 r4 = rows[s * kVox];
-      const float r[3] = {r4.x, r4.y, r4.z};
-      float q[3] = {r[0], r[1], r[2]};
-      if (kNeedQ) {
-        const float4 q4 = facs[s * kVox];
-        q[0] = q4.x;
-        q[1] = q4.y;
-        q[2] = q4.z;
-      }
-      sweep_step<MODE, GAINS, COEFS>(k, in, r, q, on);
-    };
-    if (ring && tn == kChunk && t0 >= settled) {
-      // the chunk's rows are consecutive but for one wrap: an immediate offset from one of two addresses
-      const int first = (t0 - late) & (kRows - 1);
-      const uint32_t low = slot + (uint32_t)first * kRowBytes, high = low - kRows * kRowBytes;
+  auto gather = [&](int t, float (&x)[3]) {
+    const bool on = k.valid && t >= d && t < T;
+    const float* from = p.X + (int64_t)(t - d) * S + slot;
 #pragma unroll
-      for (int s = 0; s < kChunk; ++s) {
-        const uint32_t at = (first + s >= kRows ? high : low) + s * kRowBytes;
-        float in[3];
-        float pad;
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(in[0]), "=f"(in[1]), "=f"(in[2]), "=f"(pad) : "r"(at));
-        one(s, in, true);
-      }
-    } else {
-      for (int s = 0; s < tn; ++s) {
-        const int t = t0 + s;
-        float in[3];
-        if (ring) {
-          const uint32_t at = slot - ring0 + (uint32_t)((t - late) & (kRows - 1)) * kRowBytes;
-          const float4 h = *reinterpret_cast<const float4*>(smem_raw + at);
-          in[0] = h.x;
-          in[1] = h.y;
-          in[2] = h.z;
-        } else {
+    for (int b = 0; b < 3; ++b) x[b] = on ? __ldg(from + b) : 0.0f;
+  };
+  // with and without a ring, each with registers of its own
+  auto steps = [&](auto with_ring) {
+    constexpr bool kRing = decltype(with_ring)::value;
+    int buf = 0;  // t0 / kChunk mod 3
+    for (int t0 = 0; t0 < T; t0 += kChunk) {
+      float ahead[kAhead][3];  // without a ring: the next steps' inputs, under way over the barrier and the steps before
+      if (!kRing) {
 #pragma unroll
-          for (int b = 0; b < 3; ++b) in[b] = (k.valid && t >= d) ? __ldg(p.X + (int64_t)(t - d) * S + slot + b) : 0.0f;
+        for (int s = 0; s < kAhead; ++s) gather(t0 + s, ahead[s]);
+      }
+      cp_async_wait<0>();
+      // this chunk's history, factors and the next chunk's own rows are there for all; the previous chunk's
+      // buffers and the ring rows older than t0 - dmax are free (kRows >= spread + 2 chunks)
+      __syncthreads();
+      const int next = buf == 2 ? 0 : buf + 1, after = next == 2 ? 0 : next + 1;
+      if (kRing) stage_history(t0 + kChunk);
+      stage_own(t0 + 2 * kChunk, after);
+      cp_async_commit();
+      if (t0 + kChunk < T) factors(next, ((t0 / kChunk) + 1) & 1);
+      const float4* rows = &sm.row[buf][0][vl];
+      const float4* facs = &sm.q[(t0 / kChunk) & 1][0][vl];
+      const int tn = min(kChunk, T - t0);
+      auto one = [&](int s, const float (&in)[3], bool on) {
+        const float4 r4 = rows[s * kVox];
+        const float r[3] = {r4.x, r4.y, r4.z};
+        float q[3] = {r[0], r[1], r[2]};
+        if (kNeedQ) {
+          const float4 q4 = facs[s * kVox];
+          q[0] = q4.x;
+          q[1] = q4.y;
+          q[2] = q4.z;
         }
-        one(s, in, t >= d);
-      }
-    }
-    if (kAdj) {
-      // chunk sums into the totals: the error of a long sum stays that of its T / 8 partial sums
-      if (GAINS) {
+        sweep_step<MODE, GAINS, COEFS>(k, in, r, q, on);
+      };
+      if (kRing && tn == kChunk && t0 >= settled) {
+        // the chunk's rows are consecutive but for one wrap: an immediate offset from one of two addresses
+        const int first = (t0 - late) & (kRows - 1);
+        const uint32_t low = slot + (uint32_t)first * kRowBytes, high = low - kRows * kRowBytes;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int s = 0; s < kChunk; ++s) {
+          const uint32_t at = (first + s >= kRows ? high : low) + s * kRowBytes;
+          float in[3];
+          float pad;
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(in[0]), "=f"(in[1]), "=f"(in[2]), "=f"(pad) : "r"(at));
+          one(s, in, true);
+        }
+      } else if (kRing) {
+        for (int s = 0; s < tn; ++s) {
+          const int t = t0 + s;
+          const float4 h = *reinterpret_cast<const float4*>(smem_raw + (slot - ring0) + (uint32_t)((t - late) & (kRows - 1)) * kRowBytes);
+          const float in[3] = {h.x, h.y, h.z};
+          one(s, in, t >= d);
+        }
+      } else {
+#pragma unroll 1
+        for (int s0 = 0; s0 < tn; s0 += kAhead) {
 #pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            k.dG[a][b] = k.dG[a][b] + k.sG[a][b];
-            k.sG[a][b] = 0.0f;
+          for (int i = 0; i < kAhead; ++i) {
+            const int t = t0 + s0 + i;
+            if (t >= T) break;
+            const float in[3] = {ahead[i][0], ahead[i][1], ahead[i][2]};
+            if (s0 + kAhead < kChunk) gather(t + kAhead, ahead[i]);
+            one(s0 + i, in, t >= d);
           }
+        }
       }
-      k.dC = k.dC + k.sC;
-      k.sC = 0.0f;
+      if (kAdj) {
+        // chunk sums into the totals: the error of a long sum stays that of its T / 8 partial sums
+        if (GAINS) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+              k.dG[a][b] = k.dG[a][b] + k.sG[a][b];
+              k.sG[a][b] = 0.0f;
+            }
+        }
+        k.dC = k.dC + k.sC;
+        k.sC = 0.0f;
+      }
+      buf = next;
     }
-    buf = next;
-  }
+  };
+  if (ring)
+    steps(std::true_type{});
+  else
+    steps(std::false_type{});
   const int w = p.start[blockIdx.x] + vl;  // the voxel, read again rather than kept in a register
   if (w >= p.start[blockIdx.x + 1]) return;
   if (GAINS) {
@@ -407,21 +445,25 @@ __global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_co
   }
 }
 
-template <int MODE, bool GAINS, bool COEFS>
-cudaError_t launch(const SweepArgs& a, cudaStream_t stream) {
+template <int MODE, bool GAINS, bool COEFS, bool ANY>
+cudaError_t launch_form(const SweepArgs& a, cudaStream_t stream) {
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;
   static bool done[128] = {};
   if (device < 0 || device >= 128) return cudaErrorInvalidValue;
   if (!done[device]) {
-    err = cudaFuncSetAttribute(sweep_kernel<MODE, GAINS, COEFS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    err = cudaFuncSetAttribute(sweep_kernel<MODE, GAINS, COEFS, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(SweepSmem));
     if (err != cudaSuccess) return err;
     done[device] = true;
   }
-  sweep_kernel<MODE, GAINS, COEFS><<<(unsigned)a.blocks, kThreads, sizeof(SweepSmem), stream>>>(a);
+  sweep_kernel<MODE, GAINS, COEFS, ANY><<<(unsigned)a.blocks, kThreads, sizeof(SweepSmem), stream>>>(a);
   return cudaGetLastError();
+}
+template <int MODE, bool GAINS, bool COEFS>
+cudaError_t launch(const SweepArgs& a, cudaStream_t stream) {
+  return a.any ? launch_form<MODE, GAINS, COEFS, true>(a, stream) : launch_form<MODE, GAINS, COEFS, false>(a, stream);
 }
 
 template <int MODE>
@@ -447,6 +489,8 @@ SweepArgs sweep_args(DeviceScenario& d, const DeriveScalars& s) {
   a.dC = d.dC;
   a.fir = d.fir;
   a.iir = d.iir;
+  a.status = d.status;
+  a.any = d.sweep_any;
   a.blocks = d.sweep_blocks;
   a.start = d.sstart;
   a.halo = d.shalo;

@@ -33,7 +33,13 @@ struct Recorded {
   bool adjoint;
   int grid;
 };
+// A gradient sweep, and whether its kernel takes blocks without a ring.
+struct Sweep {
+  const ct::DeviceScenario* d;
+  bool any;
+};
 struct Graph {
+  std::vector<Sweep> sweeps;
   std::vector<Recorded> launches;
   std::vector<std::pair<const ct::DeviceScenario*, const void*>> ranges;  // delay ranges, and the reverse table they covered
 };
@@ -51,6 +57,7 @@ size_t g_time = 0;
 std::vector<int> g_orders;  // phases of every batched forward that ran
 bool g_landed = false;  // what was recorded on a stream has happened
 int g_captures = 0;     // epochs captured since the last count
+bool g_last_sweep = false;  // whether the last sweep takes blocks without a ring
 int g_last_routes = 0;      // ct::WaveRoutes of the last forward
 int g_routes[2][3];         // tiles of the last forward and adjoint: followed by progress, by tags, polled directly
 
@@ -119,6 +126,25 @@ void check(const Recorded& r) {
   for (int i = 0; i < l.nscn; ++i) check_ring(l.scns[i], l.routes, r.adjoint ? "batched adjoint" : "batched forward");
 }
 
+void check_sweep(const Sweep& w) {
+  int64_t dmin = INT32_MAX, dmax = 1;
+  for (int64_t i = 0; i < w.d->V * ct::kOffsets; ++i)
+    if (w.d->nbr[i] >= 0) {
+      dmin = std::min<int64_t>(dmin, w.d->delays[i]);
+      dmax = std::max<int64_t>(dmax, w.d->delays[i]);
+    }
+  if (!w.any && dmax - dmin > ct::kSweepRingSpread) wrong("delays too far apart for the sweep's ring");
+}
+cudaError_t sweep(const ct::DeviceScenario& d) {
+  g_last_sweep = d.sweep_any;
+  const Sweep w{&d, d.sweep_any};
+  if (g_capturing)
+    g_capturing->sweeps.push_back(w);
+  else
+    check_sweep(w);
+  return cudaSuccess;
+}
+
 void count_routes(int (&n)[3], const ct::DeviceScenario& d, const int32_t* nhalo, const int32_t* near) {
   n[0] = n[1] = n[2] = 0;
   for (int t = 0; t < d.tiles; ++t) ++n[nhalo[t] < 0 ? 2 : nhalo[t] > 0 && near[t * ct::kNearTiles] < 0 ? 1 : 0];
@@ -160,6 +186,7 @@ int host_device_report(char* out, int len) {  // and forget it
 }
 void host_device_landed(int on) { g_landed = on != 0; }
 int host_device_captures() { return std::exchange(g_captures, 0); }
+int host_device_last_sweep() { return g_last_sweep; }
 int host_device_last_routes() { return g_last_routes; }
 void host_device_routes(int* out) { std::memcpy(out, g_routes, sizeof(g_routes)); }
 int host_device_phases(int* out, int len) {  // phases of the batched forwards since the last call
@@ -247,6 +274,7 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned lon
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
   for (const Recorded& r : ((Graph*)e)->launches) check(r);
+  for (const Sweep& w : ((Graph*)e)->sweeps) check_sweep(w);
   for (const auto& r : ((Graph*)e)->ranges)
     if (r.first->rev != r.second) wrong("a captured update leaves the adjoint's delay ranges behind");
   return cudaSuccess;
@@ -347,8 +375,8 @@ void output_state_indices_host(const int32_t*, const int32_t*, int64_t, int64_t,
                                int32_t*) {}
 cudaError_t umma_prepare(DeviceScenario&, cudaStream_t) { return cudaSuccess; }
 cudaError_t slice_prepare(DeviceScenario&, cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_derive(DeviceScenario&, const DeriveScalars&, cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_adjoint_gradients(DeviceScenario&, const DeriveScalars&, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_derive(DeviceScenario& d, const DeriveScalars&, cudaStream_t) { return sweep(d); }
+cudaError_t launch_adjoint_gradients(DeviceScenario& d, const DeriveScalars&, cudaStream_t) { return sweep(d); }
 cudaError_t launch_update(DeviceScenario&, const UpdateScalars&, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_measure(DeviceScenario&, int64_t, bool, cudaStream_t) { return cudaGetLastError(); }
 cudaError_t launch_map_residuals(DeviceScenario&, int64_t, cudaStream_t) { return cudaSuccess; }

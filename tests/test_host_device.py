@@ -266,6 +266,29 @@ def test_kernel_follows_the_delays(host, ctx):
     assert host.report() == ""
 
 
+def test_sweep_follows_the_delays(host, ctx):
+    """The gradient sweep's kernel without the way for blocks whose delays do not fit its ring runs while they surely do."""
+    from cardiotrust_b200 import algorithm as alg
+
+    eng = _engine(ctx, (4, 4, 4), 100, algorithm=alg.Algorithm(freeze_delays=False))
+    small = _engine(ctx, (4, 4, 4), 80, algorithm=alg.Algorithm(freeze_delays=False))
+    batch = alg.EpochBatch(ctx, [eng, small], precision=alg.Precision.Fp32)
+    OPEN.append(batch)
+    for largest, wide in ((8 + 16, 0), (8 + 17, 1), (12, 0), (90, 1)):
+        _with_delays(eng, largest)
+        for mode in (alg.GradMode.Reference, alg.GradMode.Adjoint):
+            _with_delays(eng, largest)
+            eng.run_epoch(0, grad_mode=mode, precision=0)
+            assert host.lib.host_device_last_sweep() == wide, largest
+        batch.run_epoch()
+    _with_delays(eng, 20)
+    for update in range(6):  # delays 8 to 20: bounds 7 to 21, ..., whose spread passes 16 after three updates
+        eng.run_epoch(0, precision=0)
+        assert host.lib.host_device_last_sweep() == (update > 2), update
+    batch.run_epoch()
+    assert host.report() == ""
+
+
 def test_batch_keeps_its_graph_while_the_bounds_come_and_go(host, ctx):
     """Delays 8 to 31 fit the staged ring. While an update's read-back is under way the bounds are wider and do not; the
     batch captures once for that, not with every change."""
