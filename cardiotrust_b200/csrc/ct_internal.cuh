@@ -115,7 +115,7 @@ struct DeviceScenario {
   int32_t* srange;       // [sweep blocks, 2]
   // adjoint mode, allocated on first use
   int32_t* rev;          // [V,26] voxel whose offset n points at this voxel, -1 if none
-  int32_t* rhalo;        // the tiles' halo tables of that direction
+  int32_t* rhalo;        // the tiles' halo tables of that direction (on a lattice the forward's but for rhslot)
   int16_t* rhpos;
   int16_t* rhslot;
   int32_t* rnear;
@@ -257,6 +257,8 @@ cudaError_t launch_update(DeviceScenario& d, const UpdateScalars& s, cudaStream_
 // Delay ranges of the scenario, its tiles and its sweep blocks: after every change of the delays, and once the adjoint's
 // tables exist.
 cudaError_t launch_delay_ranges(DeviceScenario& d, cudaStream_t stream);
+// rev and rhslot of a lattice: nbr and hslot with the offsets in opposite order.
+cudaError_t launch_mirror_tables(DeviceScenario& d, cudaStream_t stream);
 
 // Voxel blocks of `words` 32-bit words between reference and device voxel order (perm[u] = the
 // reference voxel of device voxel u): gather dst[u] = src[perm[u]], else scatter dst[perm[u]] = src[u].

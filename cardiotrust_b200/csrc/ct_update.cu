@@ -69,6 +69,16 @@ __global__ void roll_delays_kernel(float* __restrict__ coefs, int32_t* __restric
   delays[i] = d;
 }
 
+// One thread per item of a tile, `pairs` of which are items of voxels.
+__global__ void mirror_tables_kernel(const int32_t* __restrict__ nbr, const int16_t* __restrict__ hslot, int64_t pairs, int64_t n,
+                                     int32_t* __restrict__ rev, int16_t* __restrict__ rhslot) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t from = i / kOffsets * kOffsets + (kOffsets - 1 - i % kOffsets);
+  rhslot[i] = hslot[from];
+  if (i < pairs) rev[i] = nbr[from];
+}
+
 // dmin[0] = smallest, dmin[1] = largest delay of a connected (voxel, offset) pair
 // Smallest and largest delay of the connected pairs: of each tile of the recursions (of its items in the adjoint's direction,
 // too, once its table exists), of each block of the sweep, and of all. One warp per tile or block; what bounds it is its
@@ -324,6 +334,12 @@ cudaError_t launch_update(DeviceScenario& d, const UpdateScalars& s, cudaStream_
                                                        s.bias2, s.bias_dev);
     roll_delays_kernel<<<blocks(nc, 256), 256, 0, stream>>>(d.coefs, d.delays, nc);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mirror_tables(DeviceScenario& d, cudaStream_t stream) {
+  const int64_t n = (int64_t)d.tiles * kFwdTileVoxels * kOffsets;
+  mirror_tables_kernel<<<blocks(n, 256), 256, 0, stream>>>(d.nbr, d.hslot, d.V * kOffsets, n, d.rev, d.rhslot);
   return cudaGetLastError();
 }
 

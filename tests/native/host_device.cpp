@@ -351,6 +351,13 @@ cudaError_t launch_delay_ranges(DeviceScenario& d, cudaStream_t) {
     }
   return cudaSuccess;
 }
+cudaError_t launch_mirror_tables(DeviceScenario& d, cudaStream_t) {
+  const int64_t n = (int64_t)d.tiles * kFwdTileVoxels * kOffsets;
+  need(d.rev, sizeof(int32_t) * d.V * kOffsets, "reverse table");
+  need(d.rhslot, sizeof(int16_t) * n, "reverse slots");
+  for (int64_t i = 0; i < d.V * kOffsets; ++i) d.rev[i] = d.nbr[i / kOffsets * kOffsets + (kOffsets - 1 - i % kOffsets)];
+  return cudaSuccess;
+}
 cudaError_t launch_permute_blocks(const void* src, void* dst, const int32_t* perm, int64_t V, int64_t words, bool gather,
                                   cudaStream_t) {
   for (int64_t u = 0; u < V; ++u)

@@ -320,6 +320,28 @@ def test_delays_above_the_roll_limit_keep_their_ring(host, ctx):
     assert host.report() == ""
 
 
+def test_adjoint_tables_of_a_lattice(host, ctx):
+    """The adjoint's direction shares the forward's halo tables on a lattice: less memory than tables of its own, and a
+    refused allocation leaves nothing behind."""
+    from cardiotrust_b200 import algorithm as alg
+    from cardiotrust_b200._lib import CtError
+
+    eng = _engine(ctx, (8, 6, 6), 10)
+    before = host.live()
+    host.fail_from(4 * 10 * 3 * 288)  # the gradient of the states
+    with pytest.raises(CtError, match="made to fail"):
+        eng.run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=0)
+    host.fail_from(NEVER)
+    assert host.live() == before
+    eng.run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=0)
+    own = 9 * 192 * (4 + 2)  # halos and their slots
+    assert host.live() - before - 4 * 10 * 3 * 288 < 288 * 26 * (4 + 2) + own
+    eng.run_epoch(0, grad_mode=alg.GradMode.Reference, precision=0)
+    OPEN.pop().close()
+    assert host.live() == 0
+    assert host.report() == ""
+
+
 #: no thread can be started, then each size of host allocation fails: a status each time, never an abort
 CHILD = """
 import sys
