@@ -489,8 +489,8 @@ ct_scn::Sight sight_of(const Followed& readers, const HaloTables& t) {
 }
 
 // Consecutive voxels in blocks of at most TV, a block ending early where its halo would pass HM - 1 voxels. (Uncut, one block
-// of 809 with 96 halo voxels, which gathered its history from global memory, took as long as all the others: 1.42 ms
-// instead of 0.95 per beat on 6,468 voxels, T = 1,500.)
+// of 809, whose 96 halo voxels did not fit the 95 slots that a block had then, gathered its history from global memory and
+// took as long as all the others: 1.42 ms instead of 0.95 per beat on 6,468 voxels, T = 1,500.)
 std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int TV, int HM) {
   std::vector<int32_t> start{0}, seen((size_t)V, -1);
   int halo = 0;

@@ -28,7 +28,6 @@ enum WaveRoutes { kStaged, kDecide, kEvery };
 // Counts the progress of a launch, so that a bounded wait can tell a long wait from a lost one.
 struct Heartbeat {
   unsigned int count;
-  unsigned int unused;
 };
 
 // Everything of one scenario that lives on the device.

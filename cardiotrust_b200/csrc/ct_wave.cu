@@ -60,7 +60,7 @@
 //   * Every wait is bounded: a wait that sees neither its data nor any progress of the launch (a
 //     heartbeat counter) for 2 s records CT_ERR_TIMEOUT and the CTA leaves.
 // What bounds it: the cycle of a row through the chain of warps, the exchange and the halo's staging, once
-// per dmin steps (20x20x20 cuboid, dmin = 8: 4,300 + 6,000 clock cycles; issue slots 51 % used, DRAM 1.7 %).
+// per dmin steps (20x20x20 cuboid, dmin = 8: 1.18 ms are 9,300 clock cycles for each; issue slots 51 % used, DRAM 1.7 %).
 // Measured, ms before -> now: forward 2.87 -> 1.18 (20x20x20, T = 2,000), 0.56 -> 0.23 (8x8x8, T = 500), 54.6 ->
 // 24.5 (64x64x48 shell, T = 4,000); adjoint recursion 1.05 and 23 on the first and the last, where the
 // inbox form took 11.2 and 145 with the gradients in it.
@@ -78,8 +78,7 @@ constexpr int kTile = kFwdTileVoxels;
 constexpr int kItems = 4;        // offsets per compute warp (the last one: 2)
 constexpr int kComputeWarps = 7;
 constexpr int kLastItems = kOffsets - kItems * (kComputeWarps - 1);
-constexpr int kStageWarps = 1;
-constexpr int kThreads = 32 * (kComputeWarps + kStageWarps);
+constexpr int kThreads = 32 * (kComputeWarps + 1);  // and the staging warp
 constexpr int kHaloSlots = kFwdHaloMax;  // slots per ring row; the last one stays zero (absent neighbours)
 constexpr int kZeroSlot = kHaloSlots - 1;
 constexpr int kRingRows = 32;            // power of two
@@ -88,18 +87,18 @@ constexpr int kGroup = 2;                // steps per hand-over, where no delay 
 constexpr int kBatch = 4;                // rows that the staging warp copies together (two at first)
 constexpr int kOwn = 4;                  // steps of the last warp's global reads in flight, power of two
 constexpr int kMaxVisit = 64;            // steps per visit of a CTA that owns several tiles
-constexpr int kPerLane = kHaloSlots / (32 * kStageWarps);  // halo voxels per lane of a staging warp
+constexpr int kPerLane = kHaloSlots / 32;  // halo voxels per lane of the staging warp
 constexpr int kSmemPerCta = 233472 / 2 - 1024;  // two CTAs per SM
 constexpr unsigned long long kWaitNs = 2000000000ull;
 // the rows of one group of steps and of the batch that is staged beside it
 static_assert(kFwdRingSpread + 2 + kGroup + kBatch <= kRingRows, "a tile's history fits the ring");
-static_assert(kTile == 32 && kLastItems == 2 && kHaloSlots % (32 * kStageWarps) == 0, "lane = voxel");
+static_assert(kTile == 32 && kLastItems == 2 && kHaloSlots % 32 == 0, "lane = voxel");
 
 struct WaveSmem {
   uint4 ring[kRingRows][kHaloSlots];          // {x0, x1, x2, -}
   uint4 hand[kComputeWarps - 1][kHand][kGroup][32];  // {sum0, sum1, sum2, group number + 1} from warp w to w + 1
   float own[kOwn][6][32];                     // the last warp's global reads per step
-  uint64_t full[kRingRows];                   // the slot's row is staged (every staging warp)
+  uint64_t full[kRingRows];                   // the slot's row is staged (every lane of the staging warp)
   uint64_t empty[kRingRows];                  // no later step reads the slot's row
   uint64_t taken[kComputeWarps - 1][kHand];   // warp w + 1 has taken the entry
   int abort;
@@ -339,8 +338,7 @@ __device__ __forceinline__ int copy_rows(const uint4* const (&from)[kPerLane], c
 // the halo in device order (runs of neighbouring entries). Two rows at a time while it waits for rows to
 // be finished, a few more while it finds them ready (3 against 4 with one tile per CTA: 1.18 against 1.23 ms on
 // the 20x20x20 cuboid; always 2: 1.20, and 7 % slower on the shell). Loads into
-// registers were slower: their round trips to L2 do not overlap (the loads of two batches share
-// scoreboards), 2,250 cycles per two rows.
+// registers were slower.
 template <bool ANY>
 __device__ __forceinline__ void stage_history(WaveSmem& sm, const WaveLaunch& L) {
   const int lane = threadIdx.x & 31;
@@ -855,7 +853,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_kernel(const __grid_constant
     (&sm.hand[0][0][0][0])[i] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x == 0) {
     for (int i = 0; i < kRingRows; ++i) {
-      mbar_init(&sm.full[i], 32 * kStageWarps);
+      mbar_init(&sm.full[i], 32);
       mbar_init(&sm.empty[i], 1);
     }
     for (int w = 0; w < kComputeWarps - 1; ++w)
