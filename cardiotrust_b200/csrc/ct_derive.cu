@@ -24,8 +24,8 @@
 // The tangent z runs forward in time like ap itself, so neither the adjoint chain nor the
 // all-pass history has to be stored or recomputed for the coefficients.
 //
-// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of 91 and
-// 51 instructions), and the waits of a block's warps for each other at each chunk.
+// What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of 89 and
+// 48 instructions), and the waits of a block's warps for each other at each chunk.
 // Layout: a CTA owns up to 8 consecutive voxels (4 x 2 neighbours in y and z inside a grid), 208 items. The history that
 // the items gather comes from a ring of rows in shared memory, one 16-byte entry {x0, x1, x2, -}
 // per halo voxel, staged by cp.async one chunk of 8 steps ahead; thread e works on voxel e mod 8, offset

@@ -248,7 +248,9 @@ int ct_batch_run_epoch(ct_batch* batch, int64_t* batch_indices);
  * ct_batch_run_epoch) under candidate schedules and keeps the fastest: the arrangement of the
  * members' tiles in phases (0: small members fill the places that a large member's phase leaves
  * free; 1: every large member by itself; 2: one phase), which sets how the
- * tiles of members of different sizes spread over the CTAs. Up to five epochs; synchronous.
+ * tiles of members of different sizes spread over the CTAs. Up to five epochs (each arrangement once, in
+ * adjoint mode after two that do not count); an arrangement that needs more memory than there is
+ * is left out; synchronous.
  * Writes the choice and its epoch time (ms) to the non-NULL outputs; ckpt_k, once the adjoint's
  * checkpoint interval, receives 64 (no checkpoints are stored). */
 int ct_batch_autotune(ct_batch* batch, int64_t* batch_indices, int* ckpt_k, int* tile_order, double* best_ms);
