@@ -336,26 +336,32 @@ int prepare_sliced(ct_scn* s) {
   return CT_OK;
 }
 
-// The kernels that the delays and halos call for, and the exchange ring of the recursions. A tile overwrites the entry of step t - xrows when it
-// finishes step t; by then every tile that it reads has finished step t - dmax and so reads no row before
-// t - 2 dmax any more, provided that the tiles that read it are among those that it reads or stages a voxel
+// The kernels that the delays and halos call for, and the exchange ring of the recursions. A tile overwrites the entry
+// of step t - xrows when it finishes step t; by then every tile that it reads has finished step t - dmax and so reads no
+// row before t - 2 dmax any more, provided that the tiles that read it are among those that it reads or stages a voxel
 // of. Where they are not, the ring holds every step of the beat.
 int prepare_exchange(ct_scn* s) {
   DeviceScenario& d = s->d;
-  refresh_delay_bounds(s);
-  const bool wide = s->dmax_bound - s->dmin_bound > ct::kFwdRingSpread;
-  const int routes = !s->halo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
-  const int rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
-  d.routes = routes;
-  d.rroutes = rroutes;
-  d.sweep_any = s->dmax_bound - s->dmin_bound > ct::kSweepRingSpread;
   int64_t want = 8, all = 8;
-  while (want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30)) want <<= 1;
   while (all < d.T) all <<= 1;
-  auto bounded = [](ct_scn::Sight sight, int kernel) {
-    return sight == ct_scn::kByRows || (sight == ct_scn::kByStaging && kernel == ct::kStaged);
+  auto look = [&] {  // false: the ring cannot be shorter than the beat
+    refresh_delay_bounds(s);
+    const bool wide = s->dmax_bound - s->dmin_bound > ct::kFwdRingSpread;
+    d.routes = !s->halo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
+    d.rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
+    d.sweep_any = s->dmax_bound - s->dmin_bound > ct::kSweepRingSpread;
+    for (want = 8; want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30);) want <<= 1;
+    auto bounded = [](ct_scn::Sight sight, int kernel) {
+      return sight == ct_scn::kByRows || (sight == ct_scn::kByStaging && kernel == ct::kStaged);
+    };
+    const bool shorter = bounded(s->sight, d.routes) && bounded(s->rsight, d.rroutes);
+    if (!shorter || want > all) want = all;
+    return shorter;
   };
-  if (!bounded(s->sight, routes) || !bounded(s->rsight, rroutes) || want > all) want = all;
+  if (!look() && d.xrows < all && s->updates_at_read >= 0) {  // the bounds may be wider than the delays
+    CT_CUDA(cudaStreamSynchronize(s->ctx->stream), "exchange ring");
+    look();
+  }
   if (d.xch && d.xrows >= want) return CT_OK;
   CT_CUDA(cudaStreamSynchronize(s->ctx->stream), "exchange ring");
   release(s, d.xch);

@@ -55,7 +55,8 @@ Graph* g_capturing = nullptr;
 std::vector<float> g_times;
 size_t g_time = 0;
 std::vector<int> g_orders;  // phases of every batched forward that ran
-bool g_landed = false;  // what was recorded on a stream has happened
+int g_landed = 0;  // what was recorded on a stream has happened: never, always, or once the stream was waited for
+bool g_waited = false;
 int g_captures = 0;     // epochs captured since the last count
 bool g_last_sweep = false;  // whether the last sweep takes blocks without a ring
 int g_last_routes = 0;      // ct::WaveRoutes of the last forward
@@ -184,7 +185,7 @@ int host_device_report(char* out, int len) {  // and forget it
   g_report.clear();
   return n;
 }
-void host_device_landed(int on) { g_landed = on != 0; }
+void host_device_landed(int when) { g_landed = when; }
 int host_device_captures() { return std::exchange(g_captures, 0); }
 int host_device_last_sweep() { return g_last_sweep; }
 int host_device_last_routes() { return g_last_routes; }
@@ -247,13 +248,19 @@ cudaError_t cudaGetLastError() {
 const char* cudaGetErrorString(cudaError_t) { return "made to fail"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return *s = (cudaStream_t)1, cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+  g_waited = true;
+  return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = (cudaEvent_t)1, cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventQuery(cudaEvent_t) { return g_landed ? cudaSuccess : cudaErrorNotReady; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) {
+  g_waited = false;
+  return cudaSuccess;
+}
+cudaError_t cudaEventQuery(cudaEvent_t) { return g_landed == 1 || (g_landed == 2 && g_waited) ? cudaSuccess : cudaErrorNotReady; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
   *ms = g_time < g_times.size() ? g_times[g_time++] : 1.0f;
   return cudaSuccess;

@@ -123,6 +123,26 @@ def test_one_way_tables_keep_a_short_exchange_ring(host, ctx, case):
     assert host.report() == ""
 
 
+def test_one_way_ring_stays_short_while_the_bounds_are_wide(host, ctx):
+    """Delays 8 to 31 fit the staged ring. Epochs that are enqueued ahead widen the host's bounds past it; the device is asked
+    before the ring grows to the whole beat."""
+    import test_gpu_routes as routes
+
+    from cardiotrust_b200 import algorithm as alg
+
+    shape, steps, _, _, how = routes.CASES["one_way_small"]
+    scn = routes.scenario(shape, steps, 8, 31, how)
+    scn.measurements = np.zeros((1, steps, scn.num_sensors), np.float32)
+    OPEN.append(alg.EpochEngine.from_scenario(ctx, scn, algorithm=alg.Algorithm(freeze_delays=False), num_batch_slots=16))
+    before = host.live()
+    host.lib.host_device_landed(2)
+    for epoch in range(6):
+        OPEN[-1].run_epoch(epoch, precision=0, sync=False)
+    host.lib.host_device_landed(0)
+    assert host.live() == before
+    assert host.report() == ""
+
+
 def _engine(ctx, shape, steps, **kw):
     from cardiotrust_b200 import algorithm as alg
     from cardiotrust_b200 import scenario as sc
