@@ -233,7 +233,7 @@ __device__ __forceinline__ uint32_t row_parity(int pos) { return (uint32_t)(pos 
 // Steps per visit of a CTA with several tiles: the scenario's smallest delay at most, so that every row that a visit
 // reads belongs to an earlier block of steps.
 __device__ __forceinline__ int visit_steps(const WaveScn& p) {
-  return p.dmin[0] > p.dmin[1] ? 1 : min(p.dmin[0], kMaxVisit);
+  return p.dmin[0] > p.dmin[1] ? kMaxVisit : min(p.dmin[0], kMaxVisit);  // nothing connected: nothing is read
 }
 
 // Delay range of a tile's own items: one slow or fast layer of tissue leaves the other tiles their pairs and rings.
