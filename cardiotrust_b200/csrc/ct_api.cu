@@ -68,6 +68,7 @@ struct ct_scn {
   // exchange ring and choose the recursions' kernel without reading the device.
   int64_t dmin_bound = 1, dmax_bound = 1;
   bool halo_fits = true, rhalo_fits = true;  // every tile's halo (in the adjoint's direction) fits the staging slots
+  bool sweep_fits = true;                    // every sweep block's halo does
   // Asynchronous read-back of the device's delay range after an update (pinned words + event):
   // once it has landed, the bounds become that range, wider by the updates enqueued since.
   int32_t* dmax_host = nullptr;
@@ -349,7 +350,7 @@ int prepare_exchange(ct_scn* s) {
     const bool wide = s->dmax_bound - s->dmin_bound > ct::kFwdRingSpread;
     d.routes = !s->halo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
     d.rroutes = !s->rhalo_fits ? ct::kEvery : wide ? ct::kDecide : ct::kStaged;
-    d.sweep_any = s->dmax_bound - s->dmin_bound > ct::kSweepRingSpread;
+    d.sweep_any = !s->sweep_fits || s->dmax_bound - s->dmin_bound > ct::kSweepRingSpread;
     for (want = 8; want < 2 * s->dmax_bound + 2 && want < (int64_t(1) << 30);) want <<= 1;
     auto bounded = [](ct_scn::Sight sight, int kernel) {
       return sight == ct_scn::kByRows || (sight == ct_scn::kByStaging && kernel == ct::kStaged);
@@ -494,10 +495,14 @@ ct_scn::Sight sight_of(const Followed& readers, const HaloTables& t) {
   return readers.empty() ? ct_scn::kByRows : t.all ? ct_scn::kByStaging : ct_scn::kNot;
 }
 
-// Consecutive voxels in blocks of at most TV, a block ending early where its halo would pass HM - 1 voxels. (Uncut, one block
-// of 809, whose 96 halo voxels did not fit the 95 slots that a block had then, gathered its history from global memory and
-// took as long as all the others: 1.42 ms instead of 0.95 per beat on 6,468 voxels, T = 1,500.)
-std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int TV, int HM) {
+// Consecutive voxels in blocks of at most TV, a block ending early where its halo would pass HM - 1 voxels. (Uncut, one
+// block of 809, whose 96 halo voxels did not fit the 95 slots that a block had then, gathered its history from global
+// memory and took as long as all the others: 1.42 ms instead of 0.95 per beat on 6,468 voxels, T = 1,500.) Where that makes
+// a quarter more blocks than TV voxels each, and more than the `at_once` that run side by side, as with neighbours
+// anywhere, none is cut: blocks of four voxels leave half of their threads idle, which costs more than gathering does
+// (neighbours drawn at random, 47,264 voxels, T = 500: sweep 7.76 ms cut, 5.64 uncut; 8,000 voxels, T = 1,000: 2.06 and 1.66; 512
+// voxels, T = 500, 128 blocks: 0.081 and 0.144).
+std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int TV, int HM, int64_t at_once) {
   std::vector<int32_t> start{0}, seen((size_t)V, -1);
   int halo = 0;
   for (int64_t u = 0; u < V; ++u) {
@@ -523,6 +528,12 @@ std::vector<int32_t> cut_blocks(const std::vector<int32_t>& src, int64_t V, int 
     }
   }
   start.push_back((int32_t)V);
+  const int64_t blocks = (int64_t)start.size() - 1;
+  if (blocks > at_once && 4 * blocks > 5 * ((V + TV - 1) / TV)) {
+    start.clear();
+    for (int64_t u = 0; u < V; u += TV) start.push_back((int32_t)u);
+    start.push_back((int32_t)V);
+  }
   return start;
 }
 
@@ -1225,7 +1236,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   std::vector<int32_t> sweep_start;
   auto wave_job = beside([&] { return build_halos(h_nbr, s->bank, V, ct::kFwdTileVoxels, ct::kFwdHaloMax); });
   auto sweep_job = beside([&] {
-    sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax);
+    sweep_start = cut_blocks(h_nbr, V, ct::kSweepVoxels, ct::kSweepHaloMax, ct::kSweepPerSm * ctx->num_sms);
     return build_halos(h_nbr, s->bank, V, ct::kSweepVoxels, ct::kSweepHaloMax, sweep_start);
   });
   gather_rows(h_gains.data(), desc->gains, s->perm, 3, kGainCols);
@@ -1251,6 +1262,7 @@ int ct_scenario_create(ct_ctx* ctx, const ct_scenario_desc* desc, const ct_algor
   }
   const HaloTables sweep_halo = sweep_job.get();
   s->halo_fits = *std::min_element(wave_halo.count.begin(), wave_halo.count.end()) >= 0;
+  s->sweep_fits = *std::min_element(sweep_halo.count.begin(), sweep_halo.count.end()) >= 0;
   d.sweep_blocks = (int)sweep_start.size() - 1;
   r = r ? r : alloc(s, &d.sstart, (int64_t)sweep_start.size());
   r = r ? r : alloc(s, &d.shalo, (int64_t)sweep_halo.halo.size());

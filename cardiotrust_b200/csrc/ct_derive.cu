@@ -85,7 +85,7 @@ struct SweepArgs {
   const int32_t* halo;   // [blocks, kSlots] voxels of the halo
   const int16_t* hpos;   // [blocks, kSlots] their slots
   const int16_t* hslot;  // [blocks, kVox * 26], slot of the item's neighbour, kZero if absent
-  const int32_t* nhalo;  // [blocks] voxels of the halo
+  const int32_t* nhalo;  // [blocks] voxels of the halo, -1 if it is too large
   const int32_t* range;  // [blocks, 2] smallest and largest delay of the block's connected items
   DeriveScalars s;
   int simple;
@@ -98,8 +98,7 @@ struct SweepSmem {
   float4 row[3][kChunk][kVox];  // mapped residuals or lx
   float4 q[2][kChunk][kVox];    // reference mode: fma(mr, mse/M, maxreg * reg)
 };
-constexpr int kPerSm = 3;
-static_assert(sizeof(SweepSmem) <= 233472 / kPerSm - 1024, "blocks per SM");
+static_assert(sizeof(SweepSmem) <= 233472 / kSweepPerSm - 1024, "blocks per SM");
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -176,7 +175,7 @@ __device__ __forceinline__ void sweep_step(Item& k, const float (&in)[3], const 
 
 // MODE, which of the two gradients are wanted, and whether blocks may come whose delays do not fit the ring.
 template <int MODE, bool GAINS, bool COEFS, bool ANY>
-__global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_constant__ SweepArgs p) {
+__global__ void __launch_bounds__(kThreads, kSweepPerSm) sweep_kernel(const __grid_constant__ SweepArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
   constexpr bool kAdj = MODE == kAdjoint;
@@ -203,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, kPerSm) sweep_kernel(const __grid_co
   if (dmin > dmax) dmin = dmax = 1;  // no connected pair
   if (dmin < 1) dmin = 1;
   const int nh = p.nhalo[blockIdx.x];
-  const bool fits = (int64_t)dmax - dmin <= kSweepRingSpread;
+  const bool fits = (int64_t)dmax - dmin <= kSweepRingSpread && nh >= 0;
   if (!ANY && !fits) {
     if (tid == 0) atomicCAS(p.status, 0, (int32_t)CT_ERR_NOT_SUPPORTED);
     return;

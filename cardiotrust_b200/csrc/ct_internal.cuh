@@ -19,6 +19,7 @@ constexpr int kFwdRingSpread = 24;  // largest difference of delays that a tile'
 constexpr int kNearTiles = 64;      // tiles of a halo that its staging warp can follow
 constexpr int kSweepVoxels = 8;     // most voxels per block of the gradient sweep
 constexpr int kSweepHaloMax = 112;  // halo slots of such a block
+constexpr int kSweepPerSm = 3;        // blocks per SM
 constexpr int kSweepRingSpread = 16;  // largest difference of delays that its staged history holds
 
 // Which tiles a launch of the recursions meets: only such whose history fits the staged ring (the kernel without the direct
@@ -104,13 +105,13 @@ struct DeviceScenario {
   int32_t* near;         // [tiles, kNearTiles] tiles of the halo, the last one repeated
   int32_t* nhalo;        // [tiles] voxels of the halo, -1 if it is too large for the slots
   int32_t* range;        // [tiles, 2] smallest and largest delay of the tile's connected items
-  bool sweep_any;        // blocks of the gradient sweep may come whose delays are further apart than their ring holds
-  int sweep_blocks;      // blocks of the gradient sweep: consecutive voxels whose halo fits
+  bool sweep_any;        // blocks of the gradient sweep may come whose delays or halo their ring does not hold
+  int sweep_blocks;      // blocks of the gradient sweep: consecutive voxels
   int32_t* sstart;       // [sweep blocks + 1] their first voxels
   int32_t* shalo;        // [sweep blocks, kSweepHaloMax]
   int16_t* shpos;
   int16_t* shslot;       // [sweep blocks, 26 * kSweepVoxels]
-  int32_t* snhalo;       // [sweep blocks]
+  int32_t* snhalo;       // [sweep blocks] -1 if it does not fit
   int32_t* srange;       // [sweep blocks, 2]
   // adjoint mode, allocated on first use
   int32_t* rev;          // [V,26] voxel whose offset n points at this voxel, -1 if none

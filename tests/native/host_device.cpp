@@ -58,6 +58,7 @@ std::vector<int> g_orders;  // phases of every batched forward that ran
 int g_landed = 0;  // what was recorded on a stream has happened: never, always, or once the stream was waited for
 bool g_waited = false;
 int g_captures = 0;     // epochs captured since the last count
+int g_sweep_blocks = 0;     // of the last sweep
 bool g_last_sweep = false;  // whether the last sweep takes blocks without a ring
 int g_last_routes = 0;      // ct::WaveRoutes of the last forward
 int g_routes[2][3];         // tiles of the last forward and adjoint: followed by progress, by tags, polled directly
@@ -135,8 +136,11 @@ void check_sweep(const Sweep& w) {
       dmax = std::max<int64_t>(dmax, w.d->delays[i]);
     }
   if (!w.any && dmax - dmin > ct::kSweepRingSpread) wrong("delays too far apart for the sweep's ring");
+  for (int b = 0; b < w.d->sweep_blocks; ++b)
+    if (!w.any && w.d->snhalo[b] < 0) wrong("a halo too large for the sweep's ring");
 }
 cudaError_t sweep(const ct::DeviceScenario& d) {
+  g_sweep_blocks = d.sweep_blocks;
   g_last_sweep = d.sweep_any;
   const Sweep w{&d, d.sweep_any};
   if (g_capturing)
@@ -187,6 +191,7 @@ int host_device_report(char* out, int len) {  // and forget it
 }
 void host_device_landed(int when) { g_landed = when; }
 int host_device_captures() { return std::exchange(g_captures, 0); }
+int host_device_sweep_blocks() { return g_sweep_blocks; }
 int host_device_last_sweep() { return g_last_sweep; }
 int host_device_last_routes() { return g_last_routes; }
 void host_device_routes(int* out) { std::memcpy(out, g_routes, sizeof(g_routes)); }

@@ -16,17 +16,19 @@ TOL = 1e-5
 SHAPE = (22, 21, 22)  # 318 tiles, more than the CTAs of a device of 148 SMs
 
 
-def rewired(p, rng, how):
+def rewired(p, rng, how, shape=SHAPE):
     """Voxels of the last layer that a walk from voxel 0 reaches get other neighbours, most of a tile's voxels in some places, a
     few in others. "exchanged": each other's, so that along each offset still no two voxels reach the same one.
-    "far": anywhere in the grid."""
+    "far": anywhere in the grid ("far_everywhere": those of every voxel)."""
     V = p.coefs.shape[0]
     nbr = np.where(p.output_state_indices[::3, ::3] >= 0, p.output_state_indices[::3, ::3] // 3, -1)
-    x, y, z = np.unravel_index(np.arange(V), SHAPE)
-    last = (x == SHAPE[0] - 1) | (z == SHAPE[2] - 1)
+    x, y, z = np.unravel_index(np.arange(V), shape)
+    last = (x == shape[0] - 1) | (z == shape[2] - 1)
     place = (y // 4 + z // 4 + x // 4) % 3
     w = np.nonzero(last & (rng.random(V) < np.array([0.9, 0.2, 0.0])[place]))[0]
-    if how == "far":
+    if how == "far_everywhere":
+        w = np.arange(V)
+    if how.startswith("far"):
         nbr[w] = np.argsort(rng.random((w.size, V)), axis=1)[:, :26]
     else:
         for n in range(26):
@@ -51,9 +53,11 @@ def scenario(shape, steps, lo, hi, how=None, beats=1):
                            pulse_onset=0, pulse_sigma_samples=2.0, seed=13)
     scn = sc.build(spec)
     rng = np.random.default_rng(steps)
-    osi = rewired(scn.model, rng, how) if how in ("exchanged", "far") else scn.model.output_state_indices
+    osi = rewired(scn.model, rng, how, shape) if how in ("exchanged", "far", "far_everywhere") else scn.model.output_state_indices
     if how in ("one_way", "ends"):
         osi = one_way(scn.model, shape, how == "ends")
+    if how == "alone":
+        osi = np.full_like(scn.model.output_state_indices, -1)
     connected = osi[::3, ::3] >= 0
     drawn = rng.integers(lo, hi + 1, size=connected.shape)
     if how == "layers":  # a slow layer and a fast one, as tissues with other velocities make them
@@ -77,8 +81,11 @@ CASES = {
     "exchanged_short": (SHAPE, 33, 1, 4, "exchanged"),
     "far": (SHAPE, 47, 6, 11, "far"),
     "far_short": (SHAPE, 33, 2, 4, "far"),
+    "far_everywhere": ((13, 16, 14), 60, 4, 9, "far_everywhere"),
+    "far_everywhere_small": ((7, 6, 5), 90, 4, 9, "far_everywhere"),
     "layers": (SHAPE, 150, 6, 12, "layers"),
     "layers_small": ((7, 6, 19), 260, 6, 12, "layers"),
+    "alone": (SHAPE, 150, 4, 9, "alone"),
     "one_way": (SHAPE, 150, 4, 9, "one_way"),
     "one_way_small": ((13, 6, 7), 300, 4, 9, "one_way"),
     "one_way_ends": (SHAPE, 150, 4, 9, "ends"),
@@ -120,7 +127,7 @@ def test_routes(alg, ctx, oracle_mod, case):
     np.testing.assert_array_equal(eng.read("grad_gains").view(np.uint32), o32.d_gains.view(np.uint32))
     np.testing.assert_array_equal(eng.read("grad_coefs").view(np.uint32), o32.d_coefs.view(np.uint32))
 
-    if "far" in CASES[case]:  # two voxels reach the same one: refused
+    if "far" in case:  # two voxels reach the same one: refused
         with pytest.raises(alg.CtError, match="not a lattice"):
             eng.run_epoch(0, grad_mode=alg.GradMode.Adjoint, precision=alg.Precision.Fp32)
         eng.close()

@@ -309,6 +309,25 @@ def test_sweep_follows_the_delays(host, ctx):
     assert host.report() == ""
 
 
+@pytest.mark.parametrize("case, cut", [("far", True), ("far_everywhere", False)])
+def test_sweep_blocks_of_scattered_neighbours(host, ctx, case, cut):
+    """Blocks end where their halo would not fit, unless that left many of them small: then every block has its eight voxels,
+    and the kernel that takes halos of any size runs."""
+    import test_gpu_routes as routes
+
+    from cardiotrust_b200 import algorithm as alg
+
+    scn = routes.scenario(*routes.CASES[case])
+    scn.measurements = np.zeros((1, scn.control_function.shape[0], scn.num_sensors), np.float32)
+    OPEN.append(alg.EpochEngine.from_scenario(ctx, scn, algorithm=alg.Algorithm(freeze_delays=False)))
+    OPEN[-1].run_epoch(0, precision=0)
+    full = -(-int(np.prod(routes.CASES[case][0])) // 8)
+    blocks = host.lib.host_device_sweep_blocks()
+    assert full < blocks <= 1.25 * full if cut else blocks == full
+    assert host.lib.host_device_last_sweep() == (0 if cut else 1)
+    assert host.report() == ""
+
+
 def test_batch_keeps_its_graph_while_the_bounds_come_and_go(host, ctx):
     """Delays 8 to 31 fit the staged ring. While an update's read-back is under way the bounds are wider and do not; the
     batch captures once for that, not with every change."""
