@@ -26,25 +26,25 @@
 //
 // What bounds it: FP32 issue (69 operations per item-step in textbook mode, 33 in adjoint mode, of 89 and
 // 48 instructions), and the waits of a block's warps for each other at each chunk.
-// Layout: a CTA owns up to 8 consecutive voxels (4 x 2 neighbours in y and z inside a grid), 208 items. The history that
-// the items gather comes from a ring of rows in shared memory, one 16-byte entry {x0, x1, x2, -}
-// per halo voxel, staged by cp.async one chunk of 8 steps ahead; thread e works on voxel e mod 8, offset
-// e / 8, and a voxel's slot has (slot mod 8) = (2 y + z) mod 8, so a quarter warp's eight entries lie in
-// eight different bank groups. The factor fma(mr, mse/M, maxreg * reg) is the same for a voxel's 26
-// offsets and is formed once per (voxel, step). Blocks end early where their halo would not fit. Where a block's delays
-// spread too far for the ring (a tissue of less than 0.25 m/s at 2.5 mm and 2 kHz) its items read the rows from global
-// memory, two steps ahead; that way has a kernel of its own (ANY), launched where the host's bounds do not rule it out, and a
-// loop with registers of its own. 20x20x20 cuboid, T = 1,000, 0.2 m/s everywhere: 1.42 ms with each read waiting for its
-// answer, 1.35 one step ahead, 1.14 so, 1.05 four ahead, which is slower where the rows are scattered (shell of 47,264 voxels, T =
-// 500, each pair's delay drawn from 8 to 60: 4.23, 4.01, 3.66 and 3.89; by cp.async into the ring's place, eight ahead,
-// 1.21 and 4.76); one thread per item took 1.19 and 3.07 there. A slow layer in that shell: 2.42, now 2.34. Without
-// that way the other blocks' kernel is smaller: 0.787 -> 0.777 on the cuboid at 0.6 m/s.
-// Three CTAs per SM with 80 registers and 112 slots beat four with 72 and 96, which keep some values in local
-// memory and cut more blocks. 20x20x20 cuboid, T = 2,000, textbook: 2.28 ms with one thread per item gathering single
-// floats through L1, 1.83 with four CTAs and blocks of exactly 8 voxels, 1.66 with addresses that do not
-// wrap inside a chunk, 1.56 so. Ellipsoidal shell of 47,264 voxels, T = 4,000, adjoint sweep: 15, then 7.3. (Two items
-// per thread in paired multiply-adds, 16 voxels per block: 1.77 and 7.6; a pair of FP32 operations with three
-// operands takes 2.4 cycles. Two mbarriers instead of the CTA barrier, so that warps may be steps apart: 1.70.)
+// Layout: a CTA owns up to 8 consecutive voxels (4 x 2 neighbours in y and z inside a grid), 208 items. The history
+// that the items gather comes from a ring of rows in shared memory, one 16-byte entry {x0, x1, x2, -} per halo voxel,
+// staged by cp.async one chunk of 8 steps ahead; thread e works on voxel e mod 8, offset e / 8, and a voxel's slot has
+// (slot mod 8) = (2 y + z) mod 8, so a quarter warp's eight entries lie in eight different bank groups. The factor
+// fma(mr, mse/M, maxreg * reg) is the same for a voxel's 26 offsets and is formed once per (voxel, step). Blocks end
+// early where their halo would not fit. Where a block's delays spread too far for the ring (a tissue of less than 0.25
+// m/s at 2.5 mm and 2 kHz) its items read the rows from global memory, two steps ahead; that way has a kernel of its
+// own (ANY), launched where the host's bounds do not rule it out, and a loop with registers of its own. 20x20x20
+// cuboid, T = 1,000, 0.2 m/s everywhere: 1.42 ms with each read waiting for its answer, 1.35 one step ahead, 1.14 so,
+// 1.05 four ahead, which is slower where the rows are scattered (shell of 47,264 voxels, T = 500, each pair's delay
+// drawn from 8 to 60: 4.23, 4.01, 3.66 and 3.89; by cp.async into the ring's place, eight ahead, 1.21 and 4.76); one
+// thread per item took 1.19 and 3.07 there. A slow layer in that shell: 2.42, now 2.34. Without that way the other
+// blocks' kernel is smaller: 0.787 -> 0.777 on the cuboid at 0.6 m/s. Three CTAs per SM with 80 registers and 112 slots
+// beat four with 72 and 96, which keep some values in local memory and cut more blocks. 20x20x20 cuboid, T = 2,000,
+// textbook: 2.28 ms with one thread per item gathering single floats through L1, 1.83 with four CTAs and blocks of
+// exactly 8 voxels, 1.66 with addresses that do not wrap inside a chunk, 1.56 so. Ellipsoidal shell of 47,264 voxels, T
+// = 4,000, adjoint sweep: 15, then 7.3. (Two items per thread in paired multiply-adds, 16 voxels per block: 1.77 and
+// 7.6; a pair of FP32 operations with three operands takes 2.4 cycles. Two mbarriers instead of the CTA barrier, so
+// that warps may be steps apart: 1.70.)
 #include <cuda_runtime.h>
 
 #include <type_traits>

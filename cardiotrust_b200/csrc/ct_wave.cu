@@ -29,14 +29,15 @@
 //     gains, coefficients and chain states in registers, and passes the voxel's three partial sums
 //     to warp w+1 through shared memory (a systolic chain: the column order of the sums is kept, and
 //     no all-pass output leaves its warp). The last warp finishes the rows; warp 7 stages history.
-//   * No grid barrier: a finished row goes to an exchange ring in global memory (L2) as one
-//     16-byte entry {x0, x1, x2, step + 1} per voxel, and the readers look at the entry itself until its
-//     tag is the step they need: a 128-bit relaxed access is one access, so no fence separates data and
-//     flag. That is the programming model's word for the polls (ld.relaxed.b128); the staging warp's cp.async of 16
-//     aligned bytes relies on the hardware, which moves such a piece of one 32-byte sector as a whole. Every read is of a row at least dmin steps back, so tiles run up to dmin steps apart, and the
-//     latency of the exchange overlaps the work on the steps between. (The former kernels met at a
-//     grid barrier every 8 steps, staged a block's rows after it and ran their producer and consumer
-//     phases one after the other.)
+//   * No grid barrier: a finished row goes to an exchange ring in global memory (L2) as one 16-byte entry
+//     {x0, x1, x2, step + 1} per voxel, and the readers look at the entry itself until its tag is the step
+//     they need: a 128-bit relaxed access is one access, so no fence separates data and flag. That is the
+//     programming model's word for the polls (ld.relaxed.b128); the staging warp's cp.async of 16 aligned
+//     bytes relies on the hardware, which moves such a piece of one 32-byte sector as a whole. Every read
+//     is of a row at least dmin steps back, so tiles run up to dmin steps apart, and the latency of the
+//     exchange overlaps the work on the steps between. (The former kernels met at a grid barrier every 8
+//     steps, staged a block's rows after it and ran their producer and consumer phases one after the
+//     other.)
 //   * History. The staging warp copies the tile's halo (at most kHaloSlots - 1 voxels) row by row into
 //     a ring of kRingRows rows in shared memory. A voxel's slot is chosen so that (slot mod 8) =
 //     (2 y + z) mod 8: the eight lanes of a quarter warp are 4 x 2 neighbouring (y, z), so their 16-byte
